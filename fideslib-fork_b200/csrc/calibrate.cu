@@ -37,10 +37,10 @@ __global__ void __launch_bounds__(CAL_THREADS) bf_peak_kernel(uint64_t* out, uin
   out[blockIdx.x * blockDim.x + threadIdx.x] = s;
 }
 
-// The FP64 forward butterfly of the NTT passes for primes below 2^50 (reduce x, FP64
-// modular product of y, x +- r), on register-resident doubles.
-__global__ void __launch_bounds__(CAL_THREADS) bf_peak_f64_kernel(uint64_t* out, double q, double qinv, double2 w0,
-                                                                 double2 w1, double2 w2, double2 w3, int rounds) {
+// The FP64 forward butterfly of the NTT passes for primes below 2^50 (FP64 modular product of
+// y, x +- r, x reduced first on one stage of four), on register-resident doubles.
+__global__ void __launch_bounds__(CAL_THREADS) bf_peak_f64_kernel(uint64_t* out, double q, double qinv, double w0,
+                                                                 double w1, double w2, double w3, int rounds) {
   double x[CAL_E];
   const uint64_t seed = (uint64_t)(blockIdx.x * blockDim.x + threadIdx.x) * 0x9E3779B97F4A7C15ull;
 #pragma unroll
@@ -48,13 +48,13 @@ __global__ void __launch_bounds__(CAL_THREADS) bf_peak_f64_kernel(uint64_t* out,
   for (int it = 0; it < rounds; ++it) {
 #pragma unroll
     for (int b = 3; b >= 0; --b) {
-      const double2 w = b == 3 ? w0 : b == 2 ? w1 : b == 1 ? w2 : w3;
+      const double w = b == 3 ? w0 : b == 2 ? w1 : b == 1 ? w2 : w3;
 #pragma unroll
       for (int r = 0; r < CAL_E; ++r)
         if (!(r & (1 << b))) {
           const int s = r | (1 << b);
-          const double a = nttk::f_reduce(x[r], q, qinv);
-          const double t = nttk::f_mulmod(x[s], w.x, w.y, q);
+          const double a = b == 3 ? nttk::f_reduce(x[r], q, qinv) : x[r];
+          const double t = nttk::f_mulmod(x[s], w, q, qinv);
           x[r] = __dadd_rn(a, t);
           x[s] = __dsub_rn(a, t);
         }
@@ -75,7 +75,7 @@ double measure_bf_peak_f64(int device) {
   const int blocks = sms * 8;
   const uint64_t q = (1ull << 50) - (1ull << 17) + 1;  // any odd modulus below 2^50
   const double qd = (double)q;
-  auto tw = [&](uint64_t w) { return make_double2((double)(w % q), (double)(w % q) / qd); };
+  auto tw = [&](uint64_t w) { return (double)(w % (q / 2)); };
   uint64_t* out = nullptr;
   cudaStream_t st = nullptr;
   cudaEvent_t e0 = nullptr, e1 = nullptr;

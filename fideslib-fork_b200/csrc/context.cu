@@ -15,6 +15,7 @@
 
 #include "context.hpp"
 #include "conv_tc.hpp"
+#include "ntt.cuh"
 
 namespace fides {
 
@@ -215,10 +216,14 @@ Context* create_context(int logN, int n_q, int K, int dnum, const uint64_t* prim
     FIDES_CUDA(cudaSetDevice(device));
     // ---- per-prime constants and twiddles
     std::vector<DevPrime> hp(np);
-    std::vector<ShoupConst> tf((size_t)np * N), ti((size_t)np * N), il(np);
-    std::vector<double2> tff((size_t)np * N), tfi((size_t)np * N);
-    std::vector<double> twf_w((size_t)np * N), twi_w((size_t)np * N);
+    std::vector<ShoupConst> il(np);
     std::vector<F64Prime> f64(np);
+    // NTT twiddles (the transforms start at N = 2^10): 8-byte entries where the FP64 butterflies
+    // run, 16-byte ones elsewhere
+    std::vector<size_t> tw_at(np + 1, 0);
+    for (int i = 0; i < np; ++i)
+      tw_at[i + 1] = tw_at[i] + (logN < 10 ? 0 : tw_block(logN) * (primes[i] < NTT_F64_MAX ? 8 : 16));
+    std::vector<uint64_t> twid(tw_at[np] / sizeof(uint64_t));
     auto work = [&](int i) {
       uint64_t q = primes[i];
       DevPrime& d = hp[i];
@@ -229,7 +234,7 @@ Context* create_context(int logN, int n_q, int K, int dnum, const uint64_t* prim
       d.r64_s = h_shoup(d.r64, q).ws;
       d.ninv = h_invmod(N % q, q);
       d.ninv_s = h_shoup(d.ninv, q).ws;
-      d.pad = 0;
+      d.tw = tw_at[i];
       std::vector<uint64_t> pw(N), ipw(N);
       uint64_t ip = h_invmod(c->psi[i], q);
       pw[0] = ipw[0] = 1;
@@ -237,20 +242,44 @@ Context* create_context(int logN, int n_q, int K, int dnum, const uint64_t* prim
         pw[j] = h_mulmod(pw[j - 1], c->psi[i], q);
         ipw[j] = h_mulmod(ipw[j - 1], ip, q);
       }
-      for (uint64_t j = 0; j < N; ++j) {
-        uint32_t r = h_brev((uint32_t)j, logN);
-        tf[i * N + j] = h_shoup(pw[r], q);
-        ti[i * N + j] = h_shoup(ipw[r], q);
-      }
       il[i] = h_shoup(h_mulmod(ipw[h_brev(1, logN)], d.ninv, q), q);
       const double qd = (double)q;  // exact for q < 2^53; used only for q < 2^50
-      for (size_t j = 0; j < (size_t)N; ++j) {
-        tff[i * N + j] = make_double2((double)tf[i * N + j].w, (double)tf[i * N + j].w / qd);
-        tfi[i * N + j] = make_double2((double)ti[i * N + j].w, (double)ti[i * N + j].w / qd);
-        twf_w[i * N + j] = (double)tf[i * N + j].w / qd;  // correctly rounded w / q
-        twi_w[i * N + j] = (double)ti[i * N + j].w / qd;
-      }
-      f64[i] = F64Prime{qd, 1.0 / qd, (double)d.ninv, (double)d.ninv / qd, (double)il[i].w, (double)il[i].w / qd};
+      auto centred = [&](uint64_t w) { return w > q / 2 ? -(double)(q - w) : (double)w; };
+      f64[i] = F64Prime{qd, 1.0 / qd, centred(d.ninv), centred(il[i].w)};
+      if (logN < 10) return;
+      // the twiddle tables (layout in ntt.cuh); the twiddle of global stage s, block m is the
+      // (2^s + m)-th power in bit-reversed order
+      for (int le = 4; le >= (ntt_has_le3(logN) ? 3 : 4); --le)
+        for (bool fwd : {true, false}) {
+          const std::vector<uint64_t>& w = fwd ? pw : ipw;
+          const size_t start = tw_start(logN, fwd, le);
+          double* fd = reinterpret_cast<double*>(reinterpret_cast<char*>(twid.data()) + tw_at[i]) + start;
+          ShoupConst* sh = reinterpret_cast<ShoupConst*>(reinterpret_cast<char*>(twid.data()) + tw_at[i]) + start;
+          const int log1 = (logN + 1) / 2;
+          size_t base = 0;  // of this sub-transform
+          for (int pass = 0; pass < 2; ++pass) {
+            const int logp = pass ? logN / 2 : log1, sbase = pass ? log1 : 0, subs = pass ? 1 << log1 : 1;
+            for (int sub = 0; sub < subs; ++sub, base += tw_sub(logp, fwd, le))
+              for (int ch = 0; ch < tw_chunks(logp, le); ++ch) {
+                const int lo = tw_lo(logp, fwd, le, ch), slots = tw_slots(logp, fwd, le, ch);
+                const size_t off = base + tw_off(logp, fwd, le, ch);
+                for (int b = tw_blo(logp, fwd, le, ch); b <= tw_bhi(logp, fwd, le, ch); ++b) {
+                  const int sig = logp - 1 - b, H = (1 << le) >> (b - lo + 1);
+                  for (int th = 0; th < slots; ++th)
+                    for (int hi = 0; hi < H; ++hi) {
+                      const uint32_t m = (1u << (sbase + sig)) + ((uint32_t)sub << sig) +
+                                         ((uint32_t)th << (lo + le - b - 1)) + (uint32_t)hi;
+                      const uint64_t v = w[h_brev(m, logN)];
+                      const int e = H + hi;
+                      if (q < NTT_F64_MAX)
+                        fd[off + (size_t)((e >> 1) * slots + th) * 2 + (e & 1)] = centred(v);
+                      else
+                        sh[off + (size_t)e * slots + th] = h_shoup(v, q);
+                    }
+                }
+              }
+          }
+        }
     };
     {
       unsigned nt = std::max(1u, std::min(16u, std::thread::hardware_concurrency()));
@@ -352,19 +381,14 @@ Context* create_context(int logN, int n_q, int K, int dnum, const uint64_t* prim
       }
     // ---- pack everything into one device blob
     std::vector<char> blob;
-    size_t o_prime, o_tf, o_ti, o_il, o_pinv, o_pmod, o_rs, o_pq, o_tff, o_tfi, o_f64, o_tww, o_twwi;
+    size_t o_prime, o_tw, o_il, o_pinv, o_pmod, o_rs, o_pq, o_f64;
     append(blob, hp, o_prime);
-    append(blob, tf, o_tf);
-    append(blob, ti, o_ti);
+    append(blob, twid, o_tw);
     append(blob, il, o_il);
     append(blob, pinv, o_pinv);
     append(blob, pmod, o_pmod);
     append(blob, rs, o_rs);
     append(blob, pqinv, o_pq);
-    append(blob, tff, o_tff);
-    append(blob, tfi, o_tfi);
-    append(blob, twf_w, o_tww);
-    append(blob, twi_w, o_twwi);
     append(blob, f64, o_f64);
     struct Off {
       size_t sp, spr, pre, dp, dpr, mat, tcb, tcd;
@@ -399,17 +423,12 @@ Context* create_context(int logN, int n_q, int K, int dnum, const uint64_t* prim
     FIDES_CUDA(cudaMemcpy(c->d_tables, blob.data(), blob.size(), cudaMemcpyHostToDevice));
     char* base = static_cast<char*>(c->d_tables);
     c->d_prime = reinterpret_cast<DevPrime*>(base + o_prime);
-    c->d_tw_fwd = reinterpret_cast<ShoupConst*>(base + o_tf);
-    c->d_tw_inv = reinterpret_cast<ShoupConst*>(base + o_ti);
+    c->d_tw = base + o_tw;
     c->d_inv_last = reinterpret_cast<ShoupConst*>(base + o_il);
     c->d_pinv = reinterpret_cast<ShoupConst*>(base + o_pinv);
     c->d_pmod = reinterpret_cast<ShoupConst*>(base + o_pmod);
     c->d_rescale = reinterpret_cast<RescaleConst*>(base + o_rs);
     c->d_pqinv = reinterpret_cast<ShoupConst*>(base + o_pq);
-    c->d_twf_fwd = reinterpret_cast<double2*>(base + o_tff);
-    c->d_twf_inv = reinterpret_cast<double2*>(base + o_tfi);
-    c->d_tww_fwd = reinterpret_cast<double*>(base + o_tww);
-    c->d_tww_inv = reinterpret_cast<double*>(base + o_twwi);
     c->d_f64 = reinterpret_cast<F64Prime*>(base + o_f64);
     auto mk = [&](const Off& o) {
       ConvTable t;

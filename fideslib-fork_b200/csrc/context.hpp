@@ -71,10 +71,9 @@ struct ConvTable {
 enum ConvEngine { CONV_AUTO = 0, CONV_SIMT = 1, CONV_TENSOR = 2 };
 
 // FP64 constants of a prime below 2^50 for the floating-point NTT butterflies: q, 1/q, and
-// the inverse transform's last-stage factors N^-1 and psi_rev^-1[1] N^-1 with their
-// quotients by q.
+// the inverse transform's last-stage factors N^-1 and psi_rev^-1[1] N^-1, centred.
 struct F64Prime {
-  double q, qinv, ninv, ninv_q, last, last_q;
+  double q, qinv, ninv, last;
 };
 
 struct RescaleConst {
@@ -98,13 +97,8 @@ struct Context {
 
   // device tables
   DevPrime* d_prime = nullptr;       // [n_q + K]
-  ShoupConst* d_tw_fwd = nullptr;    // [n_q + K][N]: psi_rev (bit-reversed powers of psi)
-  ShoupConst* d_tw_inv = nullptr;    // [n_q + K][N]: psi^-1 bit-reversed
+  char* d_tw = nullptr;              // NTT twiddle tables, one block per prime at DevPrime::tw (ntt.cuh)
   ShoupConst* d_inv_last = nullptr;  // [n_q + K]: psi_rev^-1[1] * N^-1 (last GS stage)
-  double2* d_twf_fwd = nullptr;      // [n_q + K][N]: (w, w / q) of d_tw_fwd as doubles (q < 2^50)
-  double2* d_twf_inv = nullptr;      // [n_q + K][N]: the same for d_tw_inv
-  double* d_tww_fwd = nullptr;       // [n_q + K][N]: w / q alone, correctly rounded (row passes derive w)
-  double* d_tww_inv = nullptr;
   F64Prime* d_f64 = nullptr;         // [n_q + K]
   ShoupConst* d_pinv = nullptr;      // [n_q]: P^-1 mod q_j
   ShoupConst* d_pmod = nullptr;      // [n_q]: P mod q_j

@@ -20,7 +20,7 @@ struct __align__(16) DevPrime {
   uint64_t r64_s; // Shoup companion of r64
   uint64_t ninv;  // N^-1 mod q
   uint64_t ninv_s;
-  uint64_t pad;
+  uint64_t tw;    // byte offset of the prime's NTT twiddle tables (ntt.cuh)
 };
 
 __host__ __device__ __forceinline__ uint64_t mulhi64(uint64_t a, uint64_t b) {

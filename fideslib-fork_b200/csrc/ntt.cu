@@ -17,9 +17,7 @@ void ntt_limbs(Context* c, const LimbRef* limbs, int n, bool inverse, cudaStream
   if (!ok) throw Error(-1, "NTT prologue/epilogue not available in this direction");
   nttk::PassArgs a;
   a.primes = c->d_prime;
-  a.tw = inverse ? c->d_tw_inv : c->d_tw_fwd;
-  a.twf = inverse ? c->d_twf_inv : c->d_twf_fwd;
-  a.tww = inverse ? c->d_tww_inv : c->d_tww_fwd;
+  a.tw = c->d_tw;
   a.f64 = c->d_f64;
   a.inv_last = c->d_inv_last;
   a.pinv = c->d_pinv;
@@ -31,7 +29,7 @@ void ntt_limbs(Context* c, const LimbRef* limbs, int n, bool inverse, cudaStream
   a.n_q = c->n_q;
   {
     uint64_t nf = 0;
-    for (int i = 0; i < n; ++i) nf += c->primes[limbs[i].prime] < (1ull << 50);
+    for (int i = 0; i < n; ++i) nf += c->primes[limbs[i].prime] < NTT_F64_MAX;
     c->ntt_limbs_by_form[0] += nf;
     c->ntt_limbs_by_form[1] += (uint64_t)n - nf;
   }

@@ -46,6 +46,58 @@ enum NttOut {
   OUT_SUB_PINV = 4,  // inverse only: out = (v - ep0[i]) P^-1
 };
 
+// ---- Twiddle tables.  A pass runs the stages of one register chunk (2^le residues per thread) after
+// another; in each chunk a thread needs 2^le - 1 twiddles, one heap of them: entry (number of twiddles
+// of the stage) + hi is twiddle hi of that stage, so a full chunk's stages use entries 1, 2-3, 4-7, ...
+// Threads that share the register span's upper bits (th = t >> lo) share the heap.  A chunk's heaps are
+// stored interleaved by th, so the lanes of a warp read consecutive addresses:
+//   integer twiddles (16 bytes, w and its Shoup companion): entry i of th at i * slots + th;
+//   FP64 twiddles (8 bytes): entries in pairs, i of th at ((i >> 1) * slots + th) * 2 + (i & 1).
+// Stored by natural index, the twiddles of a chunk's last stage lay 64 bytes apart from lane to lane,
+// and their loads alone were 40-55 % of the passes' L1 wavefronts (the L1 data pipe was 80 % busy).
+// With this layout and the FP64 butterflies' single 8-byte twiddle (ntt_impl.cuh) 300 limbs of 50-bit
+// primes at N = 2^16 take 124.5 us forward and 128.3 us inverse, against 140.3 and 150.7 (copying them
+// twice, as two passes must, takes 100).
+// A table (one prime, direction and le): the column pass's chunks, then those of each row of the row
+// pass.
+constexpr int tw_chunks(int logp, int le) { return (logp + le - 1) / le; }
+// lowest bit of the register span of chunk c
+constexpr int tw_lo(int logp, bool fwd, int le, int c) {
+  return fwd ? (logp - (c + 1) * le > 0 ? logp - (c + 1) * le : 0) : (c * le + le <= logp ? c * le : logp - le);
+}
+// the pair bits [blo, bhi] of chunk c
+constexpr int tw_bhi(int logp, bool fwd, int le, int c) {
+  return fwd ? logp - 1 - c * le : (c * le + le - 1 < logp - 1 ? c * le + le - 1 : logp - 1);
+}
+constexpr int tw_blo(int logp, bool fwd, int le, int c) {
+  return fwd ? (logp - (c + 1) * le > 0 ? logp - (c + 1) * le : 0) : c * le;
+}
+constexpr int tw_slots(int logp, bool fwd, int le, int c) { return 1 << (logp - le - tw_lo(logp, fwd, le, c)); }
+constexpr int tw_off(int logp, bool fwd, int le, int c) {
+  int o = 0;
+  for (int k = 0; k < c; ++k) o += tw_slots(logp, fwd, le, k) << le;
+  return o;
+}
+constexpr int tw_sub(int logp, bool fwd, int le) { return tw_off(logp, fwd, le, tw_chunks(logp, le)); }
+constexpr size_t tw_table(int logN, bool fwd, int le) {
+  return (size_t)tw_sub((logN + 1) / 2, fwd, le) + ((size_t)tw_sub(logN / 2, fwd, le) << ((logN + 1) / 2));
+}
+// Passes with 8 residues per thread exist for these rings (measured faster for small launches at
+// N >= 2^15; smaller rings keep 16 only).
+constexpr bool ntt_has_le3(int logN) { return logN >= 15; }
+// Start of the table of (direction, le) in a prime's block, and the block's size, in entries.
+constexpr size_t tw_start(int logN, bool fwd, int le) {
+  size_t o = 0;
+  if (le == 3) o += tw_table(logN, true, 4) + tw_table(logN, false, 4);
+  return o + (fwd ? 0 : tw_table(logN, true, le));
+}
+constexpr size_t tw_block(int logN) {
+  return tw_table(logN, true, 4) + tw_table(logN, false, 4) +
+         (ntt_has_le3(logN) ? tw_table(logN, true, 3) + tw_table(logN, false, 3) : 0);
+}
+// primes with the FP64 butterflies
+constexpr uint64_t NTT_F64_MAX = 1ull << 50;
+
 struct LimbRef {
   uint64_t* ptr;          // output (and input of the first pass when src is null)
   const uint64_t* src;    // optional input of the first pass

@@ -47,12 +47,12 @@ __device__ __forceinline__ ShoupConst ld_tw(const ShoupConst* p, uint64_t pol) {
   asm("ld.global.nc.L2::cache_hint.v2.u64 {%0, %1}, [%2], %3;" : "=l"(w), "=l"(ws) : "l"(p), "l"(pol));
   return ShoupConst{w, ws};
 }
-__device__ __forceinline__ double ld_tww(const double* p, uint64_t pol) {
+__device__ __forceinline__ double ld_twf(const double* p, uint64_t pol) {
   double v;
   asm("ld.global.nc.L2::cache_hint.f64 %0, [%1], %2;" : "=d"(v) : "l"(p), "l"(pol));
   return v;
 }
-__device__ __forceinline__ double2 ld_twf(const double2* p, uint64_t pol) {
+__device__ __forceinline__ double2 ld_twf2(const double* p, uint64_t pol) {
   double2 v;
   asm("ld.global.nc.L2::cache_hint.v2.f64 {%0, %1}, [%2], %3;" : "=d"(v.x), "=d"(v.y) : "l"(p), "l"(pol));
   return v;
@@ -87,27 +87,32 @@ __device__ __forceinline__ void gs_bf(uint64_t& x, uint64_t& y, ShoupConst w, ui
   x = s;
 }
 
-// ---- FP64 butterflies for primes q < 2^50.  The residues are integers held in doubles
-// (signed, |x| < 2^51), and every operation below is exact:
+// ---- FP64 butterflies for primes q < 2^50.  The residues are integers held in doubles and the
+// twiddles w centred, |w| < q / 2.  Every operation below is exact while |y| <= 4q:
 //   * y w = p + e exactly (p = fl(y w), e = fma(y, w, -p));
-//   * k = rint(y (w/q)) from one fma with the rounding constant 1.5 2^52 (|y w/q| < 2^51);
-//     |k - y w / q| <= 1/2 + |y| 2^-53 because w/q is correctly rounded;
-//   * p - k q is an integer below 2^52 in magnitude, so fma(-k, q, p) is exact, and so is
-//     adding e: r = y w - k q with |r| <= q (1/2 + |y| 2^-53).
-// A forward butterfly reduces x the same way (x - rint(x / q) q) before x +- r on every other
-// stage of a pass (stages 0, 2, 4, ...): after a reducing stage values are within
-// (1 + A/8) q, after the next within (13/8 + 9A/64) q, so with A the bound entering a reducing
-// stage, A <= 1.9 and every operand of a product stays below 2q <= 2^51 for q < 2^50.  The
-// inverse reduces the sum and multiplies the difference on every stage (values within q).
+//   * k = rint(p (1/q)) from one fma with the rounding constant 1.5 2^52 (|y w / q| <= 2q < 2^51);
+//     p and 1/q carry one rounding each, so |k - y w / q| <= 1/2 + |y w / q| 2^-52
+//     <= 1/2 + |y| / (8q);
+//   * p - k q is an integer below 2^53 in magnitude, so fma(-k, q, p) is exact, and so is
+//     adding e: r = y w - k q with |r| <= q / 2 + |y| / 8.
+// In units of q, a forward stage on values within B leaves B + 1/2 + B/8, or, if it reduces x to
+// x - rint(x / q) q first, 1 + B/8.  One reducing stage a chunk of at most four stages (its first)
+// keeps every value within 3.8; the last chunk of the transform reduces once more, so that its
+// results are within 2, which f_to_canon needs.  An inverse stage on values within B leaves sums
+// within 2B and products within 1/2 + B/4; every other stage reduces its sums, so B alternates
+// between 1 and 2 (the last stage of an odd row pass reduces too).
 // Between the two passes of a transform the doubles are stored as they are (their bits);
-// only the last pass writes canonical residues.  On B200 the FP64 pipe runs this
-// product at ~1.7x the rate of the 64-bit integer Shoup product, which is the NTT's bound.
+// only the last pass writes canonical residues.  The quotient from p needs no second table value
+// (w / q), and the centred twiddles' margin saves most reductions: 8.75 (forward) and 9.5 (inverse)
+// FP64 operations a butterfly and 8 bytes a twiddle, against 9.5 and 11 with w / q, plus two a
+// twiddle where w was recovered from it.  On B200 the FP64 pipe runs this product at ~1.7x the rate
+// of the 64-bit integer Shoup product.
 constexpr double F64_RND = 6755399441055744.0;  // 1.5 * 2^52
 constexpr double F64_TWO52 = 4503599627370496.0;
-__device__ __forceinline__ double f_mulmod(double y, double w, double wq, double q) {
+__device__ __forceinline__ double f_mulmod(double y, double w, double q, double qinv) {
   const double p = __dmul_rn(y, w);
   const double e = __fma_rn(y, w, -p);
-  const double k = __dadd_rn(__fma_rn(y, wq, F64_RND), -F64_RND);
+  const double k = __dadd_rn(__fma_rn(p, qinv, F64_RND), -F64_RND);
   return __dadd_rn(__fma_rn(-k, q, p), e);
 }
 __device__ __forceinline__ double f_reduce(double x, double q, double qinv) {
@@ -127,10 +132,7 @@ __device__ __forceinline__ uint64_t f_to_canon(double v, double q2_two52, uint64
 
 struct PassArgs {
   const DevPrime* primes;
-  const ShoupConst* tw;        // forward or inverse twiddles, [prime][N]
-  const double2* twf;          // the same twiddles as (w, w / q) doubles (q < 2^50)
-  const double* tww;           // w / q alone: the row passes (one twiddle per row and stage each)
-                               // read half the bytes and derive w
+  const char* tw;              // twiddle tables of all primes (DevPrime::tw)
   const F64Prime* f64;         // [prime]
   const ShoupConst* inv_last;  // [prime]: psi_rev^-1[1] * N^-1
   const ShoupConst* pinv;      // [Q prime]: P^-1 mod q (OUT_MODDOWN)
@@ -156,22 +158,20 @@ __device__ __forceinline__ int padu(int u) {
 }
 
 // Butterflies of pair bits [BLO, BHI] (in u) for a thread whose registers span bits
-// [LO, LO + LE).  FWD walks bits high -> low, inverse low -> high.
-template <int LE, int LOGP, int LO, int BHI, int BLO, bool FWD, int PASS, bool SMALL>
-__device__ __forceinline__ void run_chunk(uint64_t (&x)[1 << LE], int t, int sub, int sbase, const ShoupConst* tw,
-                                          const DevPrime& pr, ShoupConst last, uint64_t& B, uint64_t pol) {
+// [LO, LO + LE).  FWD walks bits high -> low, inverse low -> high.  tw: the chunk's twiddles of
+// this thread (SLOTS heaps interleaved, see ntt.cuh).
+template <int LE, int LOGP, int LO, int BHI, int BLO, int SLOTS, bool FWD, int PASS, bool SMALL>
+__device__ __forceinline__ void run_chunk(uint64_t (&x)[1 << LE], const ShoupConst* tw, const DevPrime& pr,
+                                          ShoupConst last, uint64_t& B, uint64_t pol) {
   constexpr int E = 1 << LE;
-  const int th = t >> LO;
 #pragma unroll
   for (int k = 0; k <= BHI - BLO; ++k) {
     const int b = FWD ? (BHI - k) : (BLO + k);
     const int rb = b - LO;
-    const int sig = LOGP - 1 - b;  // stage within this pass
-    const int s = sbase + sig;     // global stage
-    const uint32_t base = (1u << s) + ((uint32_t)sub << sig) + ((uint32_t)th << (LO + LE - b - 1));
+    const int H = E >> (rb + 1);  // twiddles of this stage
     const bool red = !FWD && B > (1ull << 62);
 #pragma unroll
-    for (int hi = 0; hi < (E >> (rb + 1)); ++hi) {
+    for (int hi = 0; hi < H; ++hi) {
       if (!FWD && PASS == COL && b == LOGP - 1) {
         // last inverse stage (global stage 0): fold N^-1 into both outputs
 #pragma unroll
@@ -182,7 +182,7 @@ __device__ __forceinline__ void run_chunk(uint64_t (&x)[1 << LE], int t, int sub
           x[r1] = shoup(a - c + B, last.w, last.ws, pr.q);
         }
       } else {
-        const ShoupConst w = ld_tw(tw + base + hi, pol);
+        const ShoupConst w = ld_tw(tw + (H + hi) * SLOTS, pol);
 #pragma unroll
         for (int lr = 0; lr < (1 << rb); ++lr) {
           const int r0 = (hi << (rb + 1)) | lr, r1 = r0 | (1 << rb);
@@ -200,50 +200,49 @@ __device__ __forceinline__ void run_chunk(uint64_t (&x)[1 << LE], int t, int sub
 }
 
 // run_chunk on FP64 residues (q < 2^50): the same stages, pairs and twiddles.
-template <int LE, int LOGP, int LO, int BHI, int BLO, bool FWD, int PASS>
-__device__ __forceinline__ void run_chunk_f64(double (&x)[1 << LE], int t, int sub, int sbase, const double2* tw,
-                                              const double* tww, const F64Prime& fp, uint64_t pol) {
-  constexpr int E = 1 << LE;
-  const int th = t >> LO;
+template <int LE, int LOGP, int LO, int BHI, int BLO, int SLOTS, bool FWD, int PASS>
+__device__ __forceinline__ void run_chunk_f64(double (&x)[1 << LE], const double* tw, const F64Prime& fp,
+                                              uint64_t pol) {
+  constexpr int E = 1 << LE, NS = BHI - BLO + 1;
 #pragma unroll
-  for (int k = 0; k <= BHI - BLO; ++k) {
+  for (int k = 0; k < NS; ++k) {
     const int b = FWD ? (BHI - k) : (BLO + k);
     const int rb = b - LO;
-    const int sig = LOGP - 1 - b;
-    const int s = sbase + sig;
-    const uint32_t base = (1u << s) + ((uint32_t)sub << sig) + ((uint32_t)th << (LO + LE - b - 1));
+    const int H = E >> (rb + 1);
+    // forward: the chunk's first stage, and the last but one of the transform's last chunk (the
+    // second where that is the first); inverse: every second stage of the pass, and a row pass's last
+    const bool red = FWD ? (k == 0 || (PASS == ROW && BLO == 0 && NS >= 2 && k == (NS > 2 ? NS - 2 : 1)))
+                         : ((b & 1) || (PASS == ROW && b == LOGP - 1));
+    double2 w{};
 #pragma unroll
-    for (int hi = 0; hi < (E >> (rb + 1)); ++hi) {
+    for (int hi = 0; hi < H; ++hi) {
       if (!FWD && PASS == COL && b == LOGP - 1) {
 #pragma unroll
         for (int lr = 0; lr < (1 << rb); ++lr) {
           const int r0 = (hi << (rb + 1)) | lr, r1 = r0 | (1 << rb);
           const double a = x[r0], c = x[r1];
-          x[r0] = f_mulmod(__dadd_rn(a, c), fp.ninv, fp.ninv_q, fp.q);
-          x[r1] = f_mulmod(__dsub_rn(a, c), fp.last, fp.last_q, fp.q);
+          x[r0] = f_mulmod(__dadd_rn(a, c), fp.ninv, fp.q, fp.qinv);
+          x[r1] = f_mulmod(__dsub_rn(a, c), fp.last, fp.q, fp.qinv);
         }
       } else {
-        double2 w;
-        if constexpr (PASS == ROW) {
-          // w from the stored, correctly rounded w / q: (w / q) q lies within q 2^-54 < 1/2
-          // of the integer w, so one fma with the rounding constant recovers w exactly
-          w.y = ld_tww(tww + base + hi, pol);
-          w.x = __dadd_rn(__fma_rn(w.y, fp.q, F64_RND), -F64_RND);
-        } else {
-          w = ld_twf(tw + base + hi, pol);
-        }
+        if (H == 1)
+          w.x = ld_twf(tw + 1, pol);
+        else if (hi & 1)
+          w.x = w.y;
+        else
+          w = ld_twf2(tw + (H + hi) * SLOTS, pol);
 #pragma unroll
         for (int lr = 0; lr < (1 << rb); ++lr) {
           const int r0 = (hi << (rb + 1)) | lr, r1 = r0 | (1 << rb);
           if (FWD) {
-            const double a = (sig & 1) ? x[r0] : f_reduce(x[r0], fp.q, fp.qinv);
-            const double r = f_mulmod(x[r1], w.x, w.y, fp.q);
+            const double a = red ? f_reduce(x[r0], fp.q, fp.qinv) : x[r0];
+            const double r = f_mulmod(x[r1], w.x, fp.q, fp.qinv);
             x[r0] = __dadd_rn(a, r);
             x[r1] = __dsub_rn(a, r);
           } else {
-            const double a = x[r0], c = x[r1];
-            x[r0] = f_reduce(__dadd_rn(a, c), fp.q, fp.qinv);
-            x[r1] = f_mulmod(__dsub_rn(a, c), w.x, w.y, fp.q);
+            const double a = x[r0], c = x[r1], sum = __dadd_rn(a, c);
+            x[r0] = red ? f_reduce(sum, fp.q, fp.qinv) : sum;
+            x[r1] = f_mulmod(__dsub_rn(a, c), w.x, fp.q, fp.qinv);
           }
         }
       }
@@ -261,24 +260,35 @@ __device__ __forceinline__ uint64_t inv_bound(uint64_t q, int stages) {
 
 
 
-// Register span of chunk c.
+// Register span and twiddles of chunk c.
 template <int LE, int LOGP, bool FWD, int C>
 struct Chunk {
-  // forward: bits from the top; inverse: bits from the bottom
-  static constexpr int BHI = FWD ? (LOGP - 1 - C * LE) : (C * LE + LE - 1 < LOGP - 1 ? C * LE + LE - 1 : LOGP - 1);
-  static constexpr int BLO = FWD ? (LOGP - (C + 1) * LE > 0 ? LOGP - (C + 1) * LE : 0) : C * LE;
-  static constexpr int LO = FWD ? BLO : (BLO + LE <= LOGP ? BLO : LOGP - LE);
+  static constexpr int BHI = tw_bhi(LOGP, FWD, LE, C), BLO = tw_blo(LOGP, FWD, LE, C);
+  static constexpr int LO = tw_lo(LOGP, FWD, LE, C);
+  static constexpr int SLOTS = tw_slots(LOGP, FWD, LE, C), OFF = tw_off(LOGP, FWD, LE, C);
 };
+
+template <int LE, int LOGP, int PASS, bool FWD, bool SMALL, typename CH>
+__device__ __forceinline__ void one_chunk(uint64_t (&x)[1 << LE], CH, int t, const ShoupConst* tw, const DevPrime& pr,
+                                          ShoupConst last, uint64_t& B, uint64_t pol) {
+  run_chunk<LE, LOGP, CH::LO, CH::BHI, CH::BLO, CH::SLOTS, FWD, PASS, SMALL>(x, tw + CH::OFF + (t >> CH::LO), pr, last,
+                                                                             B, pol);
+}
+template <int LE, int LOGP, int PASS, bool FWD, typename CH>
+__device__ __forceinline__ void one_chunk_f64(double (&x)[1 << LE], CH, int t, const double* tw, const F64Prime& fp,
+                                              uint64_t pol) {
+  run_chunk_f64<LE, LOGP, CH::LO, CH::BHI, CH::BLO, CH::SLOTS, FWD, PASS>(x, tw + CH::OFF + 2 * (t >> CH::LO), fp, pol);
+}
 
 // The register chunks of one pass, separated by shared-memory exchanges.
 template <int LE, int LOGP, int PASS, bool FWD, bool SMALL, typename SIDX>
-__device__ __forceinline__ void chunks(uint64_t (&x)[1 << LE], uint64_t* sm, SIDX sidx, int g, int t, int subtw,
-                                       int sbase, const ShoupConst* tw, const DevPrime& pr, ShoupConst last,
-                                       uint64_t& B, bool direct_load, uint64_t pol) {
+__device__ __forceinline__ void chunks(uint64_t (&x)[1 << LE], uint64_t* sm, SIDX sidx, int g, int t,
+                                       const ShoupConst* tw, const DevPrime& pr, ShoupConst last, uint64_t& B,
+                                       bool direct_load, uint64_t pol) {
   constexpr int E = 1 << LE;
   constexpr int NCH = (LOGP + LE - 1) / LE;
   using C0 = Chunk<LE, LOGP, FWD, 0>;
-  run_chunk<LE, LOGP, C0::LO, C0::BHI, C0::BLO, FWD, PASS, SMALL>(x, t, subtw, sbase, tw, pr, last, B, pol);
+  one_chunk<LE, LOGP, PASS, FWD, SMALL>(x, C0{}, t, tw, pr, last, B, pol);
   if constexpr (NCH > 1) {
     using C1 = Chunk<LE, LOGP, FWD, 1>;
     if (!direct_load) __syncthreads();
@@ -287,7 +297,7 @@ __device__ __forceinline__ void chunks(uint64_t (&x)[1 << LE], uint64_t* sm, SID
     __syncthreads();
 #pragma unroll
     for (int r = 0; r < E; ++r) x[r] = sm[sidx(g, u_of<C1::LO, LE>(t, r))];
-    run_chunk<LE, LOGP, C1::LO, C1::BHI, C1::BLO, FWD, PASS, SMALL>(x, t, subtw, sbase, tw, pr, last, B, pol);
+    one_chunk<LE, LOGP, PASS, FWD, SMALL>(x, C1{}, t, tw, pr, last, B, pol);
   }
   if constexpr (NCH > 2) {
     using C1 = Chunk<LE, LOGP, FWD, 1>;
@@ -298,21 +308,20 @@ __device__ __forceinline__ void chunks(uint64_t (&x)[1 << LE], uint64_t* sm, SID
     __syncthreads();
 #pragma unroll
     for (int r = 0; r < E; ++r) x[r] = sm[sidx(g, u_of<C2::LO, LE>(t, r))];
-    run_chunk<LE, LOGP, C2::LO, C2::BHI, C2::BLO, FWD, PASS, SMALL>(x, t, subtw, sbase, tw, pr, last, B, pol);
+    one_chunk<LE, LOGP, PASS, FWD, SMALL>(x, C2{}, t, tw, pr, last, B, pol);
   }
   static_assert(NCH <= 3, "sub-transform too large");
 }
 
 // chunks() on FP64 residues; the shared-memory exchanges move the doubles' bits.
 template <int LE, int LOGP, int PASS, bool FWD, typename SIDX>
-__device__ __forceinline__ void chunks_f64(double (&x)[1 << LE], uint64_t* smu, SIDX sidx, int g, int t, int subtw,
-                                           int sbase, const double2* tw, const double* tww, const F64Prime& fp,
-                                           bool direct_load, uint64_t pol) {
+__device__ __forceinline__ void chunks_f64(double (&x)[1 << LE], uint64_t* smu, SIDX sidx, int g, int t,
+                                           const double* tw, const F64Prime& fp, bool direct_load, uint64_t pol) {
   constexpr int E = 1 << LE;
   constexpr int NCH = (LOGP + LE - 1) / LE;
   double* sm = reinterpret_cast<double*>(smu);
   using C0 = Chunk<LE, LOGP, FWD, 0>;
-  run_chunk_f64<LE, LOGP, C0::LO, C0::BHI, C0::BLO, FWD, PASS>(x, t, subtw, sbase, tw, tww, fp, pol);
+  one_chunk_f64<LE, LOGP, PASS, FWD>(x, C0{}, t, tw, fp, pol);
   if constexpr (NCH > 1) {
     using C1 = Chunk<LE, LOGP, FWD, 1>;
     if (!direct_load) __syncthreads();
@@ -321,7 +330,7 @@ __device__ __forceinline__ void chunks_f64(double (&x)[1 << LE], uint64_t* smu, 
     __syncthreads();
 #pragma unroll
     for (int r = 0; r < E; ++r) x[r] = sm[sidx(g, u_of<C1::LO, LE>(t, r))];
-    run_chunk_f64<LE, LOGP, C1::LO, C1::BHI, C1::BLO, FWD, PASS>(x, t, subtw, sbase, tw, tww, fp, pol);
+    one_chunk_f64<LE, LOGP, PASS, FWD>(x, C1{}, t, tw, fp, pol);
   }
   if constexpr (NCH > 2) {
     using C1 = Chunk<LE, LOGP, FWD, 1>;
@@ -332,7 +341,7 @@ __device__ __forceinline__ void chunks_f64(double (&x)[1 << LE], uint64_t* smu, 
     __syncthreads();
 #pragma unroll
     for (int r = 0; r < E; ++r) x[r] = sm[sidx(g, u_of<C2::LO, LE>(t, r))];
-    run_chunk_f64<LE, LOGP, C2::LO, C2::BHI, C2::BLO, FWD, PASS>(x, t, subtw, sbase, tw, tww, fp, pol);
+    one_chunk_f64<LE, LOGP, PASS, FWD>(x, C2{}, t, tw, fp, pol);
   }
 }
 
@@ -357,13 +366,6 @@ struct PassThreads {
   static constexpr int MINB = NT >= TPS ? 1 : (TPS / NT > 32 ? 32 : TPS / NT);
 };
 
-// Ring dimensions whose passes are also built with 8 residues per thread (measured faster for
-// small launches at N >= 2^15; smaller rings keep 16 only).
-template <int LOGN>
-struct HasLe3 {
-  static constexpr bool value = LOGN >= 15;
-};
-
 template <int LOGN, int PASS, bool FWD, int IN, int OUT, int G, int LE>
 __global__ void __launch_bounds__(PassThreads<LOGN, PASS, G, LE>::NT, PassThreads<LOGN, PASS, G, LE>::MINB)
     ntt_pass(const PassArgs a, const __grid_constant__ NttLimbList L) {
@@ -376,7 +378,7 @@ __global__ void __launch_bounds__(PassThreads<LOGN, PASS, G, LE>::NT, PassThread
   const LimbRef lr = L.limbs[blockIdx.y];
   const DevPrime pr = a.primes[lr.prime];
   constexpr int N = 1 << LOGN;
-  const ShoupConst* tw = a.tw + (size_t)lr.prime * N;
+  const char* tw_prime = a.tw + pr.tw;  // this prime's twiddle tables
   const ShoupConst last = FWD ? ShoupConst{0, 0} : a.inv_last[lr.prime];
   uint64_t* data = lr.ptr;
   const int tid = threadIdx.x;
@@ -391,8 +393,10 @@ __global__ void __launch_bounds__(PassThreads<LOGN, PASS, G, LE>::NT, PassThread
   constexpr int S = N >> LOGP;  // stride of a column (COL) / number of rows (ROW)
   const int sub0 = blockIdx.x * G;
   const int sub = sub0 + g;
-  constexpr int sbase = PASS == COL ? 0 : PassShape<LOGN, COL>::LOGP;
-  const int subtw = PASS == COL ? 0 : sub;
+  // entry of the pass's (column) or the row's first twiddle
+  const size_t tw0 = tw_start(LOGN, FWD, LE) +
+                     (PASS == COL ? 0 : tw_sub(PassShape<LOGN, COL>::LOGP, FWD, LE) +
+                                            (size_t)sub * tw_sub(LOGP, FWD, LE));
 
   auto gidx = [&](int s_, int u) -> int { return PASS == COL ? s_ + u * S : s_ * P + u; };
   auto sidx = [&](int gg, int u) -> int { return PASS == COL ? u * G + gg : gg * PADP + padu<LE>(u); };
@@ -466,22 +470,21 @@ __global__ void __launch_bounds__(PassThreads<LOGN, PASS, G, LE>::NT, PassThread
 
   // ---- chunks
   const uint64_t pol = l2_evict_last_policy();
-  const bool f64 = pr.q < (1ull << 50);  // uniform per CTA: one limb per CTA
+  const bool f64 = pr.q < NTT_F64_MAX;  // uniform per CTA: one limb per CTA
   if (f64) {
     // FP64 butterflies; every pass of such a limb stores canonical residues
     const F64Prime fp = a.f64[lr.prime];
     double xf[E];
     if (first_pass) {
-      // canonical inputs in [0, q): the first stage reduces (forward: the x operand, as on every
-      // even stage; inverse: every sum) and takes operands below q into its products
+      // canonical inputs in [0, q): within the bounds of a pass's first stage as they are
 #pragma unroll
       for (int r = 0; r < E; ++r) xf[r] = f_from_u64(x[r]);
     } else {
 #pragma unroll
       for (int r = 0; r < E; ++r) xf[r] = __longlong_as_double((long long)x[r]);  // the first pass's doubles
     }
-    chunks_f64<LE, LOGP, PASS, FWD>(xf, sm, sidx, g, t, subtw, sbase, a.twf + (size_t)lr.prime * N,
-                                a.tww + (size_t)lr.prime * N, fp, direct_load && !STAGE_PRO, pol);
+    chunks_f64<LE, LOGP, PASS, FWD>(xf, sm, sidx, g, t, reinterpret_cast<const double*>(tw_prime) + tw0, fp,
+                                    direct_load && !STAGE_PRO, pol);
     if (first_pass) {
 #pragma unroll
       for (int r = 0; r < E; ++r) x[r] = (uint64_t)__double_as_longlong(xf[r]);
@@ -491,12 +494,13 @@ __global__ void __launch_bounds__(PassThreads<LOGN, PASS, G, LE>::NT, PassThread
       for (int r = 0; r < E; ++r) x[r] = f_to_canon(xf[r], q2t, pr.q);
     }
   } else {
+  const ShoupConst* tw = reinterpret_cast<const ShoupConst*>(tw_prime) + tw0;
   uint64_t B = pr.q;  // inverse: bound of the values (a multiple of q)
   if (!FWD && PASS == COL) B = inv_bound(pr.q, PassShape<LOGN, ROW>::LOGP);
   if (FWD && pr.q < (1ull << 58))
-    chunks<LE, LOGP, PASS, FWD, true>(x, sm, sidx, g, t, subtw, sbase, tw, pr, last, B, direct_load && !STAGE_PRO, pol);
+    chunks<LE, LOGP, PASS, FWD, true>(x, sm, sidx, g, t, tw, pr, last, B, direct_load && !STAGE_PRO, pol);
   else
-    chunks<LE, LOGP, PASS, FWD, false>(x, sm, sidx, g, t, subtw, sbase, tw, pr, last, B, direct_load && !STAGE_PRO, pol);
+    chunks<LE, LOGP, PASS, FWD, false>(x, sm, sidx, g, t, tw, pr, last, B, direct_load && !STAGE_PRO, pol);
 
   // ---- final reduction of the completed transform
   if (FWD && PASS == ROW) {
@@ -589,7 +593,7 @@ void launch_pass_le(Context* c, const PassArgs& a, const NttLimbList& L, cudaStr
 }
 template <int LOGN, int PASS, bool FWD, int IN, int OUT>
 void launch_pass(Context* c, const PassArgs& a, const NttLimbList& L, cudaStream_t s) {
-  if constexpr (HasLe3<LOGN>::value) {
+  if constexpr (ntt_has_le3(LOGN)) {
     if (c->ntt_residues(!FWD, PASS, L.n) == 8) {
       launch_pass_le<LOGN, PASS, FWD, IN, OUT, 3>(c, a, L, s);
       return;

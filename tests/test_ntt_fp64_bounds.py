@@ -1,0 +1,77 @@
+"""Exactness and bounds of the NTT's FP64 butterflies (primes below 2^50, csrc/ntt_impl.cuh).
+
+The quotient of a product is taken from the rounded product itself (`f_mulmod`) and most stages
+leave their sums unreduced; these tests replay the product on operands at the largest magnitudes a
+stage meets, and the bound recurrence of every chunk of every ring dimension, on the CPU.
+"""
+import random
+from fractions import Fraction
+
+import pytest
+
+RND = 6755399441055744.0  # 1.5 * 2^52
+
+
+def fma(a, b, c):
+    return float(Fraction(a) * Fraction(b) + Fraction(c))
+
+
+def f_mulmod(y, w, q, qinv):
+    p = y * w
+    e = fma(y, w, -p)
+    k = fma(p, qinv, RND) - RND
+    return fma(-k, q, p) + e
+
+
+def primes():
+    from fides_b200 import params
+    return params.gen_primes(16, 50, 4) + params.gen_primes(10, 50, 2) + params.gen_primes(12, 30, 1) + [12289]
+
+
+def test_product_is_exact_up_to_four_q():
+    rng = random.Random(5)
+    for q in primes():
+        qd, qinv = float(q), 1.0 / q
+        for it in range(500):
+            w = rng.randrange(-(q // 2), q // 2 + 1) if it % 5 else rng.choice([-1, 1]) * (q // 2)
+            y = rng.randrange(-4 * q, 4 * q + 1) if it % 3 else rng.choice([-1, 1]) * (4 * q - rng.randrange(3))
+            if w and it % 7 == 0:  # next to a half-integer quotient, where k could fall either way
+                y = (rng.randrange(-2 * q, 2 * q) * q + q // 2) // w
+                if abs(y) > 4 * q:
+                    continue
+            r = f_mulmod(float(y), float(w), qd, qinv)
+            assert r == int(r) and (int(r) - y * w) % q == 0
+            assert abs(r) <= q / 2 + abs(y) / 8 + 1
+
+
+@pytest.mark.parametrize("logp", [5, 6, 7, 8, 9])
+@pytest.mark.parametrize("le", [3, 4])
+def test_stage_bounds(logp, le):
+    """Bounds in units of q: every product operand within 4, every value within 8 (2^53), every
+    transform result within 2 (f_to_canon)."""
+    chunks = -(-logp // le)
+    # forward: the column pass from canonical input, then the row pass; a row pass follows any column
+    bound = 1.0
+    for row in (False, True):
+        for c in range(chunks):
+            n = min(le, logp - c * le)
+            last = row and c == chunks - 1
+            for k in range(n):
+                red = k == 0 or (last and n >= 2 and k == (n - 2 if n > 2 else 1))
+                assert bound <= 4
+                product = 0.5 + bound / 8
+                bound = (0.5 if red else bound) + product
+                assert bound < 4
+    assert bound < 2
+    # inverse: the row pass from canonical input, then the column pass and its last multiplications
+    bound = 1.0
+    for row in (True, False):
+        for b in range(logp):
+            assert 2 * bound <= 4
+            if not row and b == logp - 1:
+                bound = 0.5 + 2 * bound / 8
+                continue
+            red = bool(b & 1) or (row and b == logp - 1)
+            bound = max(0.5 if red else 2 * bound, 0.5 + 2 * bound / 8)
+    assert bound < 2
+
