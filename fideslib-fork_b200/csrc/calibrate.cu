@@ -53,8 +53,8 @@ __global__ void __launch_bounds__(CAL_THREADS) bf_peak_f64_kernel(uint64_t* out,
       for (int r = 0; r < CAL_E; ++r)
         if (!(r & (1 << b))) {
           const int s = r | (1 << b);
-          const double a = b == 3 ? nttk::f_reduce(x[r], q, qinv) : x[r];
-          const double t = nttk::f_mulmod(x[s], w, q, qinv);
+          const double a = b == 3 ? f_reduce(x[r], q, qinv) : x[r];
+          const double t = f_mulmod(x[s], w, q, qinv);
           x[r] = __dadd_rn(a, t);
           x[s] = __dsub_rn(a, t);
         }

@@ -1,0 +1,36 @@
+// Exact modular arithmetic on integers held in doubles, for primes q < 2^50.  On B200 the FP64 pipe
+// carries these products at a higher rate than the FMA-heavy pipe carries 64-bit integer ones.
+#pragma once
+#include <cstdint>
+
+namespace fides {
+
+constexpr double F64_RND = 6755399441055744.0;  // 1.5 * 2^52
+constexpr double F64_TWO52 = 4503599627370496.0;
+
+// y w mod q within q / 2 + |y w / q| 2^-52 q, exact for |y w / q| < 2^51 and products below 2^102:
+// y w = p + e exactly; k = rint(p (1/q)) from one fma with the rounding constant; p - k q is an
+// integer below 2^53 in magnitude, so the last fma is exact, and so is adding e.
+__device__ __forceinline__ double f_mulmod(double y, double w, double q, double qinv) {
+  const double p = __dmul_rn(y, w);
+  const double e = __fma_rn(y, w, -p);
+  const double k = __dadd_rn(__fma_rn(p, qinv, F64_RND), -F64_RND);
+  return __dadd_rn(__fma_rn(-k, q, p), e);
+}
+// x - rint(x / q) q
+__device__ __forceinline__ double f_reduce(double x, double q, double qinv) {
+  const double k = __dadd_rn(__fma_rn(x, qinv, F64_RND), -F64_RND);
+  return __fma_rn(-k, q, x);
+}
+// u64 < 2^52 -> double (exact)
+__device__ __forceinline__ double f_from_u64(uint64_t v) {
+  return __dadd_rn(__longlong_as_double((long long)(0x4330000000000000ull | v)), -F64_TWO52);
+}
+// the canonical residue of an integer |s| < 2^53
+__device__ __forceinline__ uint64_t f_canon(double s, double q, double qinv) {
+  double r = f_reduce(s, q, qinv);  // |r| <= q / 2 + 1
+  if (r < 0) r = __dadd_rn(r, q);
+  return (uint64_t)__double_as_longlong(__dadd_rn(r, F64_TWO52)) & ((1ull << 52) - 1);
+}
+
+}  // namespace fides

@@ -3,6 +3,7 @@
 #pragma once
 #include <algorithm>
 
+#include "f64arith.cuh"
 #include "ntt.cuh"
 
 namespace fides {
@@ -107,23 +108,8 @@ __device__ __forceinline__ void gs_bf(uint64_t& x, uint64_t& y, ShoupConst w, ui
 // FP64 operations a butterfly and 8 bytes a twiddle, against 9.5 and 11 with w / q, plus two a
 // twiddle where w was recovered from it.  On B200 the FP64 pipe runs this product at ~1.7x the rate
 // of the 64-bit integer Shoup product.
-constexpr double F64_RND = 6755399441055744.0;  // 1.5 * 2^52
-constexpr double F64_TWO52 = 4503599627370496.0;
-__device__ __forceinline__ double f_mulmod(double y, double w, double q, double qinv) {
-  const double p = __dmul_rn(y, w);
-  const double e = __fma_rn(y, w, -p);
-  const double k = __dadd_rn(__fma_rn(p, qinv, F64_RND), -F64_RND);
-  return __dadd_rn(__fma_rn(-k, q, p), e);
-}
-__device__ __forceinline__ double f_reduce(double x, double q, double qinv) {
-  const double k = __dadd_rn(__fma_rn(x, qinv, F64_RND), -F64_RND);
-  return __fma_rn(-k, q, x);
-}
-// u64 < 2^52 -> double (exact), and a value |v| < 2q -> its canonical residue in [0, q):
-// v + 2q + 2^52 lies in [2^52, 2^53), where the double's low 52 bits are the integer v + 2q.
-__device__ __forceinline__ double f_from_u64(uint64_t v) {
-  return __dadd_rn(__longlong_as_double((long long)(0x4330000000000000ull | v)), -F64_TWO52);
-}
+// A value |v| < 2q -> its canonical residue in [0, q): v + 2q + 2^52 lies in [2^52, 2^53), where the
+// double's low 52 bits are the integer v + 2q.
 __device__ __forceinline__ uint64_t f_to_canon(double v, double q2_two52, uint64_t qi) {
   uint64_t u = (uint64_t)__double_as_longlong(__dadd_rn(v, q2_two52)) & ((1ull << 52) - 1);  // v + 2q
   u = u >= 2 * qi ? u - 2 * qi : u;
@@ -280,8 +266,18 @@ __device__ __forceinline__ void one_chunk_f64(double (&x)[1 << LE], CH, int t, c
   run_chunk_f64<LE, LOGP, CH::LO, CH::BHI, CH::BLO, CH::SLOTS, FWD, PASS>(x, tw + CH::OFF + 2 * (t >> CH::LO), fp, pol);
 }
 
+// Barrier between a pass's shared-memory exchanges: of the CTA, or of the warp where every
+// sub-transform lies within one (WARP).
+template <bool WARP>
+__device__ __forceinline__ void pass_sync() {
+  if constexpr (WARP)
+    __syncwarp();
+  else
+    __syncthreads();
+}
+
 // The register chunks of one pass, separated by shared-memory exchanges.
-template <int LE, int LOGP, int PASS, bool FWD, bool SMALL, typename SIDX>
+template <int LE, int LOGP, int PASS, bool FWD, bool SMALL, bool WARP, typename SIDX>
 __device__ __forceinline__ void chunks(uint64_t (&x)[1 << LE], uint64_t* sm, SIDX sidx, int g, int t,
                                        const ShoupConst* tw, const DevPrime& pr, ShoupConst last, uint64_t& B,
                                        bool direct_load, uint64_t pol) {
@@ -291,10 +287,10 @@ __device__ __forceinline__ void chunks(uint64_t (&x)[1 << LE], uint64_t* sm, SID
   one_chunk<LE, LOGP, PASS, FWD, SMALL>(x, C0{}, t, tw, pr, last, B, pol);
   if constexpr (NCH > 1) {
     using C1 = Chunk<LE, LOGP, FWD, 1>;
-    if (!direct_load) __syncthreads();
+    if (!direct_load) pass_sync<WARP>();
 #pragma unroll
     for (int r = 0; r < E; ++r) sm[sidx(g, u_of<C0::LO, LE>(t, r))] = x[r];
-    __syncthreads();
+    pass_sync<WARP>();
 #pragma unroll
     for (int r = 0; r < E; ++r) x[r] = sm[sidx(g, u_of<C1::LO, LE>(t, r))];
     one_chunk<LE, LOGP, PASS, FWD, SMALL>(x, C1{}, t, tw, pr, last, B, pol);
@@ -302,10 +298,10 @@ __device__ __forceinline__ void chunks(uint64_t (&x)[1 << LE], uint64_t* sm, SID
   if constexpr (NCH > 2) {
     using C1 = Chunk<LE, LOGP, FWD, 1>;
     using C2 = Chunk<LE, LOGP, FWD, 2>;
-    __syncthreads();
+    pass_sync<WARP>();
 #pragma unroll
     for (int r = 0; r < E; ++r) sm[sidx(g, u_of<C1::LO, LE>(t, r))] = x[r];
-    __syncthreads();
+    pass_sync<WARP>();
 #pragma unroll
     for (int r = 0; r < E; ++r) x[r] = sm[sidx(g, u_of<C2::LO, LE>(t, r))];
     one_chunk<LE, LOGP, PASS, FWD, SMALL>(x, C2{}, t, tw, pr, last, B, pol);
@@ -314,7 +310,7 @@ __device__ __forceinline__ void chunks(uint64_t (&x)[1 << LE], uint64_t* sm, SID
 }
 
 // chunks() on FP64 residues; the shared-memory exchanges move the doubles' bits.
-template <int LE, int LOGP, int PASS, bool FWD, typename SIDX>
+template <int LE, int LOGP, int PASS, bool FWD, bool WARP, typename SIDX>
 __device__ __forceinline__ void chunks_f64(double (&x)[1 << LE], uint64_t* smu, SIDX sidx, int g, int t,
                                            const double* tw, const F64Prime& fp, bool direct_load, uint64_t pol) {
   constexpr int E = 1 << LE;
@@ -324,10 +320,10 @@ __device__ __forceinline__ void chunks_f64(double (&x)[1 << LE], uint64_t* smu, 
   one_chunk_f64<LE, LOGP, PASS, FWD>(x, C0{}, t, tw, fp, pol);
   if constexpr (NCH > 1) {
     using C1 = Chunk<LE, LOGP, FWD, 1>;
-    if (!direct_load) __syncthreads();
+    if (!direct_load) pass_sync<WARP>();
 #pragma unroll
     for (int r = 0; r < E; ++r) sm[sidx(g, u_of<C0::LO, LE>(t, r))] = x[r];
-    __syncthreads();
+    pass_sync<WARP>();
 #pragma unroll
     for (int r = 0; r < E; ++r) x[r] = sm[sidx(g, u_of<C1::LO, LE>(t, r))];
     one_chunk_f64<LE, LOGP, PASS, FWD>(x, C1{}, t, tw, fp, pol);
@@ -335,10 +331,10 @@ __device__ __forceinline__ void chunks_f64(double (&x)[1 << LE], uint64_t* smu, 
   if constexpr (NCH > 2) {
     using C1 = Chunk<LE, LOGP, FWD, 1>;
     using C2 = Chunk<LE, LOGP, FWD, 2>;
-    __syncthreads();
+    pass_sync<WARP>();
 #pragma unroll
     for (int r = 0; r < E; ++r) sm[sidx(g, u_of<C1::LO, LE>(t, r))] = x[r];
-    __syncthreads();
+    pass_sync<WARP>();
 #pragma unroll
     for (int r = 0; r < E; ++r) x[r] = sm[sidx(g, u_of<C2::LO, LE>(t, r))];
     one_chunk_f64<LE, LOGP, PASS, FWD>(x, C2{}, t, tw, fp, pol);
@@ -375,9 +371,9 @@ __global__ void __launch_bounds__(PassThreads<LOGN, PASS, G, LE>::NT, PassThread
   constexpr int PADP = P + P / E;
   extern __shared__ uint64_t sm[];
 
+  constexpr int N = 1 << LOGN;
   const LimbRef lr = L.limbs[blockIdx.y];
   const DevPrime pr = a.primes[lr.prime];
-  constexpr int N = 1 << LOGN;
   const char* tw_prime = a.tw + pr.tw;  // this prime's twiddle tables
   const ShoupConst last = FWD ? ShoupConst{0, 0} : a.inv_last[lr.prime];
   uint64_t* data = lr.ptr;
@@ -399,7 +395,17 @@ __global__ void __launch_bounds__(PassThreads<LOGN, PASS, G, LE>::NT, PassThread
                                             (size_t)sub * tw_sub(LOGP, FWD, LE));
 
   auto gidx = [&](int s_, int u) -> int { return PASS == COL ? s_ + u * S : s_ * P + u; };
-  auto sidx = [&](int gg, int u) -> int { return PASS == COL ? u * G + gg : gg * PADP + padu<LE>(u); };
+  // shared-memory index of element u of sub-transform gg.  One element (a row of G in a column
+  // pass) of padding after every E: the threads of a half-warp read elements E apart in the next
+  // chunk, which without it fall on the same banks (1.25 M conflicts in a column pass on 300 limbs)
+  auto sidx = [&](int gg, int u) -> int { return PASS == COL ? padu<LE>(u) * G + gg : gg * PADP + padu<LE>(u); };
+  // A row pass whose rows lie within a warp (T <= 32) exchanges, stages its loads and stores and
+  // fetches its epilogue operand warp by warp: element k of thread tid is e = k WT + lane of the
+  // warp's WT E elements.  Its warps then never wait for one another, so that one loads while
+  // others compute.
+  constexpr bool WARP = PASS == ROW && T <= 32;
+  constexpr int WT = WARP && NT > 32 ? 32 : NT;  // threads that share a staged block
+  const int blk = WARP ? tid / WT : 0, lane = tid % WT;
 
   uint64_t x[E];
 
@@ -432,7 +438,7 @@ __global__ void __launch_bounds__(PassThreads<LOGN, PASS, G, LE>::NT, PassThread
 #pragma unroll
     for (int k = 0; k < G * P / 2 / NT; ++k) {
       const int c = k * NT + tid, u = c / (G / 2), h = c % (G / 2);
-      cp_async16(sm + u * G + 2 * h, lr.pro + (size_t)u * S + sub0 + 2 * h);
+      cp_async16(sm + padu<LE>(u) * G + 2 * h, lr.pro + (size_t)u * S + sub0 + 2 * h);
     }
     cp_async_commit();
   }
@@ -444,16 +450,16 @@ __global__ void __launch_bounds__(PassThreads<LOGN, PASS, G, LE>::NT, PassThread
       __syncthreads();
 #pragma unroll
       for (int r = 0; r < E; ++r)
-        x[r] = addmod(x[r], shoup(switch_modulus(sm[u_of<LO0, LE>(t, r) * G + g], opr, pr), pm.w, pm.ws, pr.q), pr.q);
+        x[r] = addmod(x[r], shoup(switch_modulus(sm[sidx(g, u_of<LO0, LE>(t, r))], opr, pr), pm.w, pm.ws, pr.q), pr.q);
     }
   } else {
 #pragma unroll
     for (int k = 0; k < E; ++k) {
-      int e = k * NT + tid;
-      int gg = e / P, u = e % P;
+      const int e = k * WT + lane;
+      const int gg = blk * (WT / T) + e / P, u = e % P;
       sm[sidx(gg, u)] = load(gidx(sub0 + gg, u));
     }
-    __syncthreads();
+    pass_sync<WARP>();
 #pragma unroll
     for (int r = 0; r < E; ++r) x[r] = sm[sidx(g, u_of<LO0, LE>(t, r))];
   }
@@ -464,7 +470,10 @@ __global__ void __launch_bounds__(PassThreads<LOGN, PASS, G, LE>::NT, PassThread
   if constexpr (EPS) {
     const uint64_t* e0 = lr.ep0 + (size_t)sub0 * P;
 #pragma unroll
-    for (int k = 0; k < G * P / 2 / NT; ++k) cp_async16(sep + 2 * (k * NT + tid), e0 + 2 * (k * NT + tid));
+    for (int k = 0; k < E / 2; ++k) {
+      const int at = blk * (WT * E) + 2 * (k * WT + lane);
+      cp_async16(sep + at, e0 + at);
+    }
     cp_async_commit();
   }
 
@@ -483,7 +492,7 @@ __global__ void __launch_bounds__(PassThreads<LOGN, PASS, G, LE>::NT, PassThread
 #pragma unroll
       for (int r = 0; r < E; ++r) xf[r] = __longlong_as_double((long long)x[r]);  // the first pass's doubles
     }
-    chunks_f64<LE, LOGP, PASS, FWD>(xf, sm, sidx, g, t, reinterpret_cast<const double*>(tw_prime) + tw0, fp,
+    chunks_f64<LE, LOGP, PASS, FWD, WARP>(xf, sm, sidx, g, t, reinterpret_cast<const double*>(tw_prime) + tw0, fp,
                                     direct_load && !STAGE_PRO, pol);
     if (first_pass) {
 #pragma unroll
@@ -498,9 +507,9 @@ __global__ void __launch_bounds__(PassThreads<LOGN, PASS, G, LE>::NT, PassThread
   uint64_t B = pr.q;  // inverse: bound of the values (a multiple of q)
   if (!FWD && PASS == COL) B = inv_bound(pr.q, PassShape<LOGN, ROW>::LOGP);
   if (FWD && pr.q < (1ull << 58))
-    chunks<LE, LOGP, PASS, FWD, true>(x, sm, sidx, g, t, tw, pr, last, B, direct_load && !STAGE_PRO, pol);
+    chunks<LE, LOGP, PASS, FWD, true, WARP>(x, sm, sidx, g, t, tw, pr, last, B, direct_load && !STAGE_PRO, pol);
   else
-    chunks<LE, LOGP, PASS, FWD, false>(x, sm, sidx, g, t, tw, pr, last, B, direct_load && !STAGE_PRO, pol);
+    chunks<LE, LOGP, PASS, FWD, false, WARP>(x, sm, sidx, g, t, tw, pr, last, B, direct_load && !STAGE_PRO, pol);
 
   // ---- final reduction of the completed transform
   if (FWD && PASS == ROW) {
@@ -542,20 +551,20 @@ __global__ void __launch_bounds__(PassThreads<LOGN, PASS, G, LE>::NT, PassThread
   constexpr bool direct_store = (PASS == COL) || (LOL == LOGP - LE);
   if constexpr (EPS) {
     cp_async_wait_all();
-    if (direct_store) __syncthreads();  // the staged store below synchronises anyway
+    if (direct_store) pass_sync<WARP>();  // the staged store below synchronises anyway
   }
   if (direct_store) {
 #pragma unroll
     for (int r = 0; r < E; ++r) store(gidx(sub, u_of<LOL, LE>(t, r)), x[r]);
   } else {
-    __syncthreads();
+    pass_sync<WARP>();
 #pragma unroll
     for (int r = 0; r < E; ++r) sm[sidx(g, u_of<LOL, LE>(t, r))] = x[r];
-    __syncthreads();
+    pass_sync<WARP>();
 #pragma unroll
     for (int k = 0; k < E; ++k) {
-      int e = k * NT + tid;
-      int gg = e / P, u = e % P;
+      const int e = k * WT + lane;
+      const int gg = blk * (WT / T) + e / P, u = e % P;
       store(gidx(sub0 + gg, u), sm[sidx(gg, u)]);
     }
   }
@@ -566,7 +575,7 @@ template <int LOGN, int PASS, bool FWD, int IN, int OUT, int G, int LE>
 void launch_pass_g(Context* c, const PassArgs& a, const NttLimbList& L, cudaStream_t s) {
   constexpr int LOGP = PassShape<LOGN, PASS>::LOGP;
   constexpr int P = 1 << LOGP, T = P / (1 << LE);
-  constexpr int smem = (PASS == COL ? P * G : G * (P + P / (1 << LE))) * (int)sizeof(uint64_t) +
+  constexpr int smem = G * (P + P / (1 << LE)) * (int)sizeof(uint64_t) +
                        (EpStage<PASS, FWD, OUT>::on ? G * P * (int)sizeof(uint64_t) : 0);
   static bool attr_set = false;  // per instantiation; set before first launch
   if (!attr_set) {
