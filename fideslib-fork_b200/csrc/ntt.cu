@@ -7,6 +7,35 @@
 
 namespace fides {
 
+namespace {
+// The longest prefix of limbs[0, n) that fits L's runs.
+void fill_runs(NttLimbList& L, const LimbRef* limbs, int n, size_t N) {
+  auto next = [N](const uint64_t* a, const uint64_t* b) { return a ? b == a + N : !b; };
+  L.n = L.runs = 0;
+  for (int i = 0; i < n; ++i) {
+    const LimbRef& x = limbs[i];
+    bool joins = false;
+    if (i) {
+      const LimbRef& y = limbs[i - 1];
+      LimbRun& r = L.run[L.runs - 1];
+      joins = next(y.ptr, x.ptr) && next(y.src, x.src) && next(y.ep0, x.ep0) && next(y.ep1, x.ep1) &&
+              x.prime == y.prime + 1 && x.aux == y.aux;
+      if (joins) {
+        const bool same = x.pro == y.pro, step = next(y.pro, x.pro);
+        if (i - r.first == 1) r.pro_step = !same && step;
+        joins = r.pro_step ? step : same;
+      }
+    }
+    if (!joins) {
+      if (L.runs == MAX_NTT_RUNS) break;
+      L.run[L.runs++] = LimbRun{x.ptr, x.src, x.pro, x.ep0, x.ep1, (int16_t)x.prime, (int16_t)x.aux, (int16_t)i, 0};
+    }
+    L.run_of[i] = (uint8_t)(L.runs - 1);
+    L.n = i + 1;
+  }
+}
+}  // namespace
+
 void ntt_limbs(Context* c, const LimbRef* limbs, int n, bool inverse, cudaStream_t s, NttIn in, NttOut out) {
   if (n <= 0) return;
   if (c->logN < 10) throw Error(-1, "GPU NTT needs logN >= 10");
@@ -33,13 +62,13 @@ void ntt_limbs(Context* c, const LimbRef* limbs, int n, bool inverse, cudaStream
     c->ntt_limbs_by_form[0] += nf;
     c->ntt_limbs_by_form[1] += (uint64_t)n - nf;
   }
-  static thread_local NttLimbList L;  // ~25 KB: keep off the stack
-  // balanced chunks of at most the context's chunk size, both passes of a chunk back to back
+  static thread_local NttLimbList L;
+  // balanced chunks of at most the context's chunk size, both passes of a chunk back to back; a chunk
+  // ends early where its limbs make more runs than a launch holds
   const int cap = c->ntt_chunk > 0 ? std::min(c->ntt_chunk, MAX_NTT_LIMBS) : MAX_NTT_LIMBS;
   const int nchunks = (n + cap - 1) / cap, per = (n + nchunks - 1) / nchunks;
-  for (int off = 0; off < n; off += per) {
-    L.n = std::min(per, n - off);
-    std::copy(limbs + off, limbs + off + L.n, L.limbs);
+  for (int off = 0; off < n; off += L.n) {
+    fill_runs(L, limbs + off, std::min(per, n - off), c->N);
     switch (c->logN) {
       case 10: ntt_transform_10(c, a, L, inverse, in, out, s); break;
       case 11: ntt_transform_11(c, a, L, inverse, in, out, s); break;

@@ -16,7 +16,7 @@
 //     and uses Harvey's [0, 4q) form otherwise; the inverse tracks a bound B (a multiple
 //     of q) and subtracts only once B passes 2^62;
 //   * one launch covers any list of limbs (any polynomials, any levels): blockIdx.y
-//     indexes a limb descriptor (pointer + prime id) passed by value;
+//     indexes a limb of a list of runs (pointers + prime id) passed by value;
 //   * the first pass may read from a separate source (out of place) or compute its input
 //     (prologue), and the last pass may combine its result with other operands before
 //     storing (epilogue) -- the reference's NTT fusion modes (src/NTT.cuh:39-69,
@@ -116,11 +116,24 @@ inline LimbRef lref(uint64_t* p, int prime) { return LimbRef{p, nullptr, nullptr
 #endif
 constexpr int MAX_NTT_LIMBS = FIDES_MAX_NTT_LIMBS;
 
-struct NttLimbList {
-  int n;
-  int pad;
-  LimbRef limbs[MAX_NTT_LIMBS];
+// A launch's limbs as runs: limb k of a run has every pointer k limbs further (pro: unless the run
+// shares one prologue limb) and prime id prime + k.  Launches of the library's operations have a few
+// runs a polynomial, so the kernel parameters stay small: 448 limb descriptors (28 KB) cost 3-5 us
+// of host time a launch more than 256 bytes, at 3-4.6 us, and runs 0.5.
+struct LimbRun {
+  uint64_t* ptr;
+  const uint64_t *src, *pro, *ep0, *ep1;
+  int16_t prime, aux;
+  int16_t first;     // index of the run's first limb in the launch
+  int16_t pro_step;  // 1: pro advances with the limb
 };
+constexpr int MAX_NTT_RUNS = 96;
+struct NttLimbList {
+  int n, runs;
+  LimbRun run[MAX_NTT_RUNS];
+  uint8_t run_of[MAX_NTT_LIMBS];
+};
+static_assert(MAX_NTT_RUNS <= 256 && MAX_NTT_LIMBS < 32768, "run_of and LimbRun hold the indexes");
 
 // Launch a full forward or inverse transform over `n` limbs (any n; split internally).
 // The prologue/epilogue modes apply to every limb of the call.

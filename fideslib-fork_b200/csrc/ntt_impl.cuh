@@ -372,7 +372,19 @@ __global__ void __launch_bounds__(PassThreads<LOGN, PASS, G, LE>::NT, PassThread
   extern __shared__ uint64_t sm[];
 
   constexpr int N = 1 << LOGN;
-  const LimbRef lr = L.limbs[blockIdx.y];
+  LimbRef lr;
+  {
+    const LimbRun& R = L.run[L.run_of[blockIdx.y]];
+    const int k = (int)blockIdx.y - R.first;
+    const size_t at = (size_t)k * N;
+    lr.ptr = R.ptr + at;
+    lr.src = R.src ? R.src + at : nullptr;
+    lr.pro = R.pro_step ? R.pro + at : R.pro;
+    lr.ep0 = R.ep0 + at;
+    lr.ep1 = R.ep1 ? R.ep1 + at : nullptr;
+    lr.prime = R.prime + k;
+    lr.aux = R.aux;
+  }
   const DevPrime pr = a.primes[lr.prime];
   const char* tw_prime = a.tw + pr.tw;  // this prime's twiddle tables
   const ShoupConst last = FWD ? ShoupConst{0, 0} : a.inv_last[lr.prime];
