@@ -245,7 +245,9 @@ Context* create_context(int logN, int n_q, int K, int dnum, const uint64_t* prim
       il[i] = h_shoup(h_mulmod(ipw[h_brev(1, logN)], d.ninv, q), q);
       const double qd = (double)q;  // exact for q < 2^53; used only for q < 2^50
       auto centred = [&](uint64_t w) { return w > q / 2 ? -(double)(q - w) : (double)w; };
-      f64[i] = F64Prime{qd, 1.0 / qd, centred(d.ninv), centred(il[i].w)};
+      uint64_t pmq = i < n_q ? 1 % q : 0;  // P mod q
+      for (int k = 0; k < K; ++k) pmq = h_mulmod(pmq, primes[n_q + k] % q, q);
+      f64[i] = F64Prime{qd, 1.0 / qd, centred(d.ninv), centred(il[i].w), centred((1ull << 51) % q), centred(pmq)};
       if (logN < 10) return;
       // the twiddle tables (layout in ntt.cuh); the twiddle of global stage s, block m is the
       // (2^s + m)-th power in bit-reversed order

@@ -71,9 +71,10 @@ struct ConvTable {
 enum ConvEngine { CONV_AUTO = 0, CONV_SIMT = 1, CONV_TENSOR = 2 };
 
 // FP64 constants of a prime below 2^50 for the floating-point NTT butterflies: q, 1/q, and
-// the inverse transform's last-stage factors N^-1 and psi_rev^-1[1] N^-1, centred.
+// the inverse transform's last-stage factors N^-1 and psi_rev^-1[1] N^-1; for the inner products
+// 2^51 and, on Q limbs, P modulo q.  The factors are centred.
 struct F64Prime {
-  double q, qinv, ninv, last;
+  double q, qinv, ninv, last, w51, pm;
 };
 
 struct RescaleConst {

@@ -33,4 +33,23 @@ __device__ __forceinline__ uint64_t f_canon(double s, double q, double qinv) {
   return (uint64_t)__double_as_longlong(__dadd_rn(r, F64_TWO52)) & ((1ull << 52) - 1);
 }
 
+// An inner product sum a_i b_i of residues, exact, reduced once.  h starts at 1.25 2^103 and takes
+// the products by fma, which rounds to its ulp of 2^51 while the sum stays in [-2, 6) 2^100; the
+// part of a product that h did not take, at most 2^50 in magnitude, is found exactly and summed in
+// l, exact for at most 7 terms.  Four operations a term, against seven for a reduced product each.
+struct F64Acc {
+  double h = F64ACC_H0, l = 0.0;
+  static constexpr double F64ACC_H0 = 12676506002282294014967032053760.0;  // 1.25 * 2^103
+  __device__ __forceinline__ void mac(double a, double b) {
+    const double n = __fma_rn(a, b, h);
+    l = __dadd_rn(l, __fma_rn(a, b, -__dadd_rn(n, -h)));
+    h = n;
+  }
+  // An integer below 2^53 in magnitude that is congruent to the sum: (h - h0) 2^-51, below 3 2^50 in
+  // magnitude, times 2^51 mod q (w51, centred), plus l.
+  __device__ __forceinline__ double fold(double w51, double q, double qinv) const {
+    return __dadd_rn(f_mulmod(__dmul_rn(__dadd_rn(h, -F64ACC_H0), 0x1p-51), w51, q, qinv), l);
+  }
+};
+
 }  // namespace fides

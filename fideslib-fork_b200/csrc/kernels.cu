@@ -5,6 +5,8 @@
 
 #include "kernels.cuh"
 #include "conv_tc.hpp"
+#include "f64arith.cuh"
+#include "ntt.cuh"
 
 namespace fides {
 
@@ -85,12 +87,14 @@ __global__ void __launch_bounds__(EW_THREADS) conv_kernel(const __grid_constant_
 // stream; one coefficient per thread was measured 13 % slower).  MAXB is the largest digit
 // count of the launch's jobs (0 = any): with it known at compile time every load of a job --
 // all digits, the own-digit and tensor operands -- is issued before its first product.  JG:
-// jobs per group (one CTA runs a group; its jobs share the key tile, read once); the grouped
-// form keeps three CTAs per SM at the cost of a few spilled registers, which measured faster
-// (KSK -9 % with groups of 4) than the unbounded register count (two CTAs per SM).
+// jobs per group (one CTA runs a group; its jobs share the key tile, read once).
 template <int CPT>
 struct KVec {
   uint64_t c[CPT];
+};
+template <int CPT>
+struct KDbl {
+  double c[CPT];
 };
 template <int CPT>
 __device__ __forceinline__ KVec<CPT> kld(const uint64_t* q) {
@@ -104,37 +108,15 @@ __device__ __forceinline__ KVec<CPT> kld(const uint64_t* q) {
   }
   return v;
 }
-
-// FP64 products for limbs of primes q < 2^50 (the NTT's FP64 residues, here on canonical
-// inputs a, b < q): p = fl(ab), e = fma(a, b, -p) = ab - p exactly; k = rint(p (1/q)) from one
-// fma with the rounding constant 1.5 2^52, within 1 of ab / q (p (1/q) is within
-// (ab / q) 2^-52 <= 1/2 of ab / q); p - k q is below 2^53 in magnitude, so fma(-k, q, p) is
-// exact, and so is adding e: r = ab - k q with |r| <= q.  The a side of the inner product (up to
-// four digits and two tensor terms: |sum| <= 6q < 2^53, summed exactly and reduced once) and
-// the own digit's a1 b1 run on the FP64 pipe; the b side keeps the 128-bit integer products on
-// the FMA-heavy pipe.  (Moving the tensor terms' P products and the b side's P a0 b0 to FP64
-// as well was 12 % slower.)
-__device__ __forceinline__ double ksk_f64(uint64_t v) {
-  return __dadd_rn(__longlong_as_double((long long)(0x4330000000000000ull | v)), -4503599627370496.0);
-}
-__device__ __forceinline__ double ksk_mul_f64(uint64_t a, uint64_t b, double q, double qinv) {
-  const double x = ksk_f64(a), y = ksk_f64(b);
-  const double p = __dmul_rn(x, y);
-  const double e = __fma_rn(x, y, -p);
-  const double k = __dadd_rn(__fma_rn(p, qinv, 6755399441055744.0), -6755399441055744.0);
-  return __dadd_rn(__fma_rn(-k, q, p), e);
-}
-// canonical residue of an exact sum |s| < 2^53
-__device__ __forceinline__ uint64_t ksk_canon_f64(double s, double q, double qinv) {
-  const double k = __dadd_rn(__fma_rn(s, qinv, 6755399441055744.0), -6755399441055744.0);
-  double r = __fma_rn(-k, q, s);  // |r| <= q / 2 + 1
-  if (r < 0) r = __dadd_rn(r, q);
-  return (uint64_t)__double_as_longlong(__dadd_rn(r, 4503599627370496.0)) & ((1ull << 52) - 1);
+template <int CPT>
+__device__ __forceinline__ KDbl<CPT> kdbl(const KVec<CPT>& v) {
+  KDbl<CPT> d;
+#pragma unroll
+  for (int c = 0; c < CPT; ++c) d.c[c] = f_from_u64(v.c[c]);
+  return d;
 }
 
-// Three CTAs (24 warps) per SM: 80 registers.  The grouped forms spill a few registers there
-// (measured faster than two CTAs per SM); the single-job forms with up to three digits fit
-// without spills (they took 96-120 registers, two CTAs per SM, when unbounded).
+// Three CTAs (24 warps) per SM: 80 registers.
 template <int MAXB, int JG>
 struct KskMinBlocks {
   static constexpr int value = (JG > 1 || (MAXB >= 1 && MAXB <= 3)) ? 3 : 1;
@@ -145,6 +127,7 @@ __global__ void __launch_bounds__(EW_THREADS, KskMinBlocks<MAXB, JG>::value) ksk
                                                             const ShoupConst* pmod, const F64Prime* f64, int logN,
                                                             int n_q, int K, int dnum, int alpha) {
   using V = KVec<CPT>;
+  using D = KDbl<CPT>;
   const int g0 = L.gstart[blockIdx.z], gn = L.gcount[blockIdx.z];
   const KskJob& J0 = L.j[g0];  // the group's jobs share key, level and extras
   const int l = J0.l, ext = l + K;
@@ -153,126 +136,20 @@ __global__ void __launch_bounds__(EW_THREADS, KskMinBlocks<MAXB, JG>::value) ksk
   const int N = 1 << logN;
   const int n = CPT * (blockIdx.x * blockDim.x + threadIdx.x);
   const int pid = i < l ? i : n_q + (i - l);
-  const DevPrime p = primes[pid];
   const int beta = (l + alpha - 1) / alpha;
   const int own = i < l ? i / alpha : -1;
   const size_t kstride = (size_t)(n_q + K) * N;
   const size_t off = (size_t)i * N + n, koff = (size_t)pid * N + n;
   const bool tensor = J0.a0 && i < l;
-  // FP64 a side: limbs of primes below 2^50, at most 4 digits (so at most 6 summed terms)
-  const bool fa_on = MAXB > 0 && p.q < (1ull << 50);
-  double fq = 0, fqinv = 0;
-  if (fa_on) {
-    fq = f64[pid].q;
-    fqinv = f64[pid].qinv;
-  }
-  // one job: sum_d D_d key_d (+ extras), reduced and stored; ka / kb: the group's key tile, or
-  // vd: the group's digit tile (MAXB > 0; the other one is loaded here).  FA: the a side's
-  // products and the own digit's a1 b1 in FP64.
-  auto run = [&](const KskJob& J, const V* ka_g, const V* kb_g, const V* vd, auto fa_) {
-    constexpr bool FA = decltype(fa_)::value;
-    U128 sa[CPT], sb[CPT];
-    double fs[CPT];  // FA: the a side
-#pragma unroll
-    for (int c = 0; c < CPT; ++c) {
-      sa[c] = sb[c] = U128{0, 0};
-      fs[c] = 0;
-    }
-    V x1{}, y1{};  // a1, b1 of this limb (own digit)
-    auto digit = [&](int d, V v, const V& a_, const V& b_) {
-      if (d == own && J.x2) {  // the own digit is x * x2 (tensor term a1 b1)
-        x1 = v;
-#pragma unroll
-        for (int c = 0; c < CPT; ++c)
-          v.c[c] = FA ? ksk_canon_f64(ksk_mul_f64(v.c[c], y1.c[c], fq, fqinv), fq, fqinv) : mulmod(v.c[c], y1.c[c], p);
-      }
-#pragma unroll
-      for (int c = 0; c < CPT; ++c) {
-        if constexpr (FA)
-          fs[c] = __dadd_rn(fs[c], ksk_mul_f64(v.c[c], a_.c[c], fq, fqinv));
-        else
-          mac128(sa[c], v.c[c], a_.c[c]);
-        mac128(sb[c], v.c[c], b_.c[c]);
-      }
-    };
-    auto tensor_terms = [&](const V& x0, const V& y0) {
-      const ShoupConst pm = pmod[i];
-#pragma unroll
-      for (int c = 0; c < CPT; ++c) {
-        const uint64_t py0 = shoup(y0.c[c], pm.w, pm.ws, p.q), py1 = shoup(y1.c[c], pm.w, pm.ws, p.q);
-        mac128(sb[c], x0.c[c], py0);  // + P a0 b0
-        if constexpr (FA) {           // + P (a0 b1 + a1 b0)
-          fs[c] = __dadd_rn(fs[c], __dadd_rn(ksk_mul_f64(x0.c[c], py1, fq, fqinv), ksk_mul_f64(x1.c[c], py0, fq, fqinv)));
-        } else {
-          mac128(sa[c], x0.c[c], py1);
-          mac128(sa[c], x1.c[c], py0);
-        }
-      }
-    };
-    if constexpr (MAXB > 0) {
-      V v[MAXB], ka[MAXB], kb[MAXB];
-#pragma unroll
-      for (int d = 0; d < MAXB; ++d)
-        if (d < beta) {
-          if (SHARE_DIGITS) {
-            v[d] = vd[d];
-            ka[d] = kld<CPT>(J.key + (size_t)d * kstride + koff);
-            kb[d] = kld<CPT>(J.key + (size_t)(dnum + d) * kstride + koff);
-          } else {
-            v[d] = kld<CPT>((d == own && J.x) ? J.x + off : J.digits + ((size_t)d * ext + i) * N + n);
-            ka[d] = ka_g[d];
-            kb[d] = kb_g[d];
-          }
-        }
-      if (own >= 0 && J.x2) y1 = kld<CPT>(J.x2 + off);
-      V x0{}, y0{};
-      if (tensor) {
-        x0 = kld<CPT>(J.a0 + off);
-        y0 = kld<CPT>(J.b0 + off);
-      }
-#pragma unroll
-      for (int d = 0; d < MAXB; ++d)
-        if (d < beta) digit(d, v[d], ka[d], kb[d]);
-      if (tensor) tensor_terms(x0, y0);
-    } else {
-      if (own >= 0 && J.x2) y1 = kld<CPT>(J.x2 + off);
-      for (int d = 0; d < beta; ++d) {
-        const uint64_t* src = (d == own && J.x) ? J.x + off : J.digits + ((size_t)d * ext + i) * N + n;
-        digit(d, kld<CPT>(src), kld<CPT>(J.key + (size_t)d * kstride + koff),
-              kld<CPT>(J.key + (size_t)(dnum + d) * kstride + koff));
-      }
-      if (tensor) {
-        // every Q limb has one own digit, so x1 / y1 hold a1 / b1 here
-        if (beta > 12) {  // keep the sums below 2^128: at most 15 products of two values < 2^62
-#pragma unroll
-          for (int c = 0; c < CPT; ++c) {
-            sa[c] = U128{reduce128(sa[c], p), 0};
-            sb[c] = U128{reduce128(sb[c], p), 0};
-          }
-        }
-        tensor_terms(kld<CPT>(J.a0 + off), kld<CPT>(J.b0 + off));
-      }
-    }
-    uint64_t ra[CPT], rb[CPT];
-#pragma unroll
-    for (int c = 0; c < CPT; ++c) {
-      if constexpr (FA)
-        ra[c] = ksk_canon_f64(fs[c], fq, fqinv);
-      else
-        ra[c] = reduce128(sa[c], p);
-      rb[c] = reduce128(sb[c], p);
-    }
-    if (J.c0 && i < l) {
-      const ShoupConst pm = pmod[i];
-      const V cv = kld<CPT>(J.c0 + off);
-#pragma unroll
-      for (int c = 0; c < CPT; ++c) rb[c] = addmod(rb[c], shoup(cv.c[c], pm.w, pm.ws, p.q), p.q);
-    }
-    if (J.c0x) {
-      const V cv = kld<CPT>(J.c0x + off);
-#pragma unroll
-      for (int c = 0; c < CPT; ++c) rb[c] = addmod(rb[c], cv.c[c], p.q);
-    }
+  const uint64_t q = primes[pid].q;
+
+  auto ld_digit = [&](const KskJob& J, int d) {
+    return kld<CPT>((d == own && J.x) ? J.x + off : J.digits + ((size_t)d * ext + i) * N + n);
+  };
+  auto ld_key = [&](const KskJob& J, int side, int d) {
+    return kld<CPT>(J.key + (size_t)(side * dnum + d) * kstride + koff);
+  };
+  auto store = [&](const KskJob& J, const uint64_t (&ra)[CPT], const uint64_t (&rb)[CPT]) {
     uint64_t* oa = J.out_a + (size_t)i * N;
     uint64_t* ob = J.out_b + (size_t)i * N;
     if (J.auto_k) {
@@ -290,39 +167,233 @@ __global__ void __launch_bounds__(EW_THREADS, KskMinBlocks<MAXB, JG>::value) ksk
       ob[n] = rb[0];
     }
   };
+
+  // Limbs of primes below 2^50, at most four digits: both sides as exact FP64 inner products
+  // (F64Acc).  Bounds in units of 2^100: the own digit a1 b1 is within 0.75 q (f_mulmod of two
+  // residues), P b0 and P b1 within 0.625 q, P within q / 2, so a side sums between -0.75 - 1.25
+  // and 4 + 1.25 in at most 6 terms.  Memory bounds this form: 461 us for the 16 jobs of 8 products and
+  // 8 rotations at N = 2^16, level 30, 3 digits (2.36 GB, 5.1 TB/s).  With 128-bit integer sums on the b
+  // side (FMA-heavy pipe) and a reduced FP64 product a term on the a side it took 629 us, issue 53 %.
+  if constexpr (MAXB > 0) {
+    if (q < NTT_F64_MAX) {
+      const F64Prime fp = f64[pid];
+      auto run = [&](const KskJob& J, const D* ka_g, const D* kb_g, const D* vd) {
+        V v[MAXB], ka[MAXB], kb[MAXB], y1{}, x0{}, y0{}, c0{};
+#pragma unroll
+        for (int d = 0; d < MAXB; ++d)
+          if (d < beta) {
+            if constexpr (SHARE_DIGITS) {
+              ka[d] = ld_key(J, 0, d);
+              kb[d] = ld_key(J, 1, d);
+            } else {
+              v[d] = ld_digit(J, d);
+            }
+          }
+        if (own >= 0 && J.x2) y1 = kld<CPT>(J.x2 + off);
+        if (tensor) {
+          x0 = kld<CPT>(J.a0 + off);
+          y0 = kld<CPT>(J.b0 + off);
+        }
+        const bool add_c0 = J.c0 && i < l;
+        if (add_c0) c0 = kld<CPT>(J.c0 + off);
+        F64Acc sa[CPT], sb[CPT];
+        D x1{}, fy1{};
+        if (own >= 0 && J.x2) fy1 = kdbl<CPT>(y1);
+#pragma unroll
+        for (int d = 0; d < MAXB; ++d)
+          if (d < beta) {
+            D w;
+            if constexpr (SHARE_DIGITS)
+              w = vd[d];
+            else
+              w = kdbl<CPT>(v[d]);
+            if (d == own && J.x2) {  // the own digit is x * x2 (tensor term a1 b1)
+              x1 = w;
+#pragma unroll
+              for (int c = 0; c < CPT; ++c) w.c[c] = f_mulmod(w.c[c], fy1.c[c], fp.q, fp.qinv);
+            }
+            D fa, fb;
+            if constexpr (SHARE_DIGITS) {
+              fa = kdbl<CPT>(ka[d]);
+              fb = kdbl<CPT>(kb[d]);
+            } else {
+              fa = ka_g[d];
+              fb = kb_g[d];
+            }
+#pragma unroll
+            for (int c = 0; c < CPT; ++c) {
+              sa[c].mac(w.c[c], fa.c[c]);
+              sb[c].mac(w.c[c], fb.c[c]);
+            }
+          }
+        if (tensor) {
+          const D fx0 = kdbl<CPT>(x0), fy0 = kdbl<CPT>(y0);
+#pragma unroll
+          for (int c = 0; c < CPT; ++c) {
+            const double py0 = f_mulmod(fy0.c[c], fp.pm, fp.q, fp.qinv), py1 = f_mulmod(fy1.c[c], fp.pm, fp.q, fp.qinv);
+            sb[c].mac(fx0.c[c], py0);  // + P a0 b0
+            sa[c].mac(fx0.c[c], py1);  // + P (a0 b1 + a1 b0)
+            sa[c].mac(x1.c[c], py0);
+          }
+        }
+        if (add_c0) {
+          const D fc = kdbl<CPT>(c0);
+#pragma unroll
+          for (int c = 0; c < CPT; ++c) sb[c].mac(fc.c[c], fp.pm);
+        }
+        uint64_t ra[CPT], rb[CPT];
+#pragma unroll
+        for (int c = 0; c < CPT; ++c) {
+          ra[c] = f_canon(sa[c].fold(fp.w51, fp.q, fp.qinv), fp.q, fp.qinv);
+          rb[c] = f_canon(sb[c].fold(fp.w51, fp.q, fp.qinv), fp.q, fp.qinv);
+        }
+        if (J.c0x) {
+          const V cv = kld<CPT>(J.c0x + off);
+#pragma unroll
+          for (int c = 0; c < CPT; ++c) rb[c] = addmod(rb[c], cv.c[c], q);
+        }
+        store(J, ra, rb);
+      };
+      if constexpr (SHARE_DIGITS) {
+        D vd[MAXB];  // the group's digit tile (hoisted rotations of one ciphertext), read once
+#pragma unroll
+        for (int d = 0; d < MAXB; ++d)
+          if (d < beta) vd[d] = kdbl<CPT>(ld_digit(J0, d));
+#pragma unroll
+        for (int jj = 0; jj < JG; ++jj)
+          if (jj < gn) run(L.j[g0 + jj], nullptr, nullptr, vd);
+      } else {
+        V ka[MAXB], kb[MAXB];
+        D da[MAXB], db[MAXB];  // the group's key tile, read once
+#pragma unroll
+        for (int d = 0; d < MAXB; ++d)
+          if (d < beta) {
+            ka[d] = ld_key(J0, 0, d);
+            kb[d] = ld_key(J0, 1, d);
+          }
+#pragma unroll
+        for (int d = 0; d < MAXB; ++d)
+          if (d < beta) {
+            da[d] = kdbl<CPT>(ka[d]);
+            db[d] = kdbl<CPT>(kb[d]);
+          }
+#pragma unroll
+        for (int jj = 0; jj < JG; ++jj)
+          if (jj < gn) run(L.j[g0 + jj], da, db, nullptr);
+      }
+      return;
+    }
+  }
+
+  // 128-bit integer sums: larger primes, or any number of digits.
+  const DevPrime p = primes[pid];
+  auto run = [&](const KskJob& J, const V* ka_g, const V* kb_g, const V* vd) {
+    U128 sa[CPT], sb[CPT];
+#pragma unroll
+    for (int c = 0; c < CPT; ++c) sa[c] = sb[c] = U128{0, 0};
+    V x1{}, y1{};  // a1, b1 of this limb (own digit)
+    auto digit = [&](int d, V v, const V& a_, const V& b_) {
+      if (d == own && J.x2) {  // the own digit is x * x2 (tensor term a1 b1)
+        x1 = v;
+#pragma unroll
+        for (int c = 0; c < CPT; ++c) v.c[c] = mulmod(v.c[c], y1.c[c], p);
+      }
+#pragma unroll
+      for (int c = 0; c < CPT; ++c) {
+        mac128(sa[c], v.c[c], a_.c[c]);
+        mac128(sb[c], v.c[c], b_.c[c]);
+      }
+    };
+    auto tensor_terms = [&](const V& x0, const V& y0) {
+      const ShoupConst pm = pmod[i];
+#pragma unroll
+      for (int c = 0; c < CPT; ++c) {
+        const uint64_t py0 = shoup(y0.c[c], pm.w, pm.ws, p.q), py1 = shoup(y1.c[c], pm.w, pm.ws, p.q);
+        mac128(sb[c], x0.c[c], py0);  // + P a0 b0
+        mac128(sa[c], x0.c[c], py1);  // + P (a0 b1 + a1 b0)
+        mac128(sa[c], x1.c[c], py0);
+      }
+    };
+    if constexpr (MAXB > 0) {
+      V v[MAXB], ka[MAXB], kb[MAXB];
+#pragma unroll
+      for (int d = 0; d < MAXB; ++d)
+        if (d < beta) {
+          if (SHARE_DIGITS) {
+            v[d] = vd[d];
+            ka[d] = ld_key(J, 0, d);
+            kb[d] = ld_key(J, 1, d);
+          } else {
+            v[d] = ld_digit(J, d);
+            ka[d] = ka_g[d];
+            kb[d] = kb_g[d];
+          }
+        }
+      if (own >= 0 && J.x2) y1 = kld<CPT>(J.x2 + off);
+      V x0{}, y0{};
+      if (tensor) {
+        x0 = kld<CPT>(J.a0 + off);
+        y0 = kld<CPT>(J.b0 + off);
+      }
+#pragma unroll
+      for (int d = 0; d < MAXB; ++d)
+        if (d < beta) digit(d, v[d], ka[d], kb[d]);
+      if (tensor) tensor_terms(x0, y0);
+    } else {
+      if (own >= 0 && J.x2) y1 = kld<CPT>(J.x2 + off);
+      for (int d = 0; d < beta; ++d) digit(d, ld_digit(J, d), ld_key(J, 0, d), ld_key(J, 1, d));
+      if (tensor) {
+        // every Q limb has one own digit, so x1 / y1 hold a1 / b1 here
+        if (beta > 12) {  // keep the sums below 2^128: at most 15 products of two values < 2^62
+#pragma unroll
+          for (int c = 0; c < CPT; ++c) {
+            sa[c] = U128{reduce128(sa[c], p), 0};
+            sb[c] = U128{reduce128(sb[c], p), 0};
+          }
+        }
+        tensor_terms(kld<CPT>(J.a0 + off), kld<CPT>(J.b0 + off));
+      }
+    }
+    uint64_t ra[CPT], rb[CPT];
+#pragma unroll
+    for (int c = 0; c < CPT; ++c) {
+      ra[c] = reduce128(sa[c], p);
+      rb[c] = reduce128(sb[c], p);
+    }
+    if (J.c0 && i < l) {
+      const ShoupConst pm = pmod[i];
+      const V cv = kld<CPT>(J.c0 + off);
+#pragma unroll
+      for (int c = 0; c < CPT; ++c) rb[c] = addmod(rb[c], shoup(cv.c[c], pm.w, pm.ws, p.q), p.q);
+    }
+    if (J.c0x) {
+      const V cv = kld<CPT>(J.c0x + off);
+#pragma unroll
+      for (int c = 0; c < CPT; ++c) rb[c] = addmod(rb[c], cv.c[c], p.q);
+    }
+    store(J, ra, rb);
+  };
   if constexpr (MAXB > 0 && SHARE_DIGITS) {
     V vd[MAXB];  // the group's digit tile (hoisted rotations of one ciphertext), read once
 #pragma unroll
     for (int d = 0; d < MAXB; ++d)
-      if (d < beta) vd[d] = kld<CPT>((d == own && J0.x) ? J0.x + off : J0.digits + ((size_t)d * ext + i) * N + n);
-    if (fa_on) {
+      if (d < beta) vd[d] = ld_digit(J0, d);
 #pragma unroll
-      for (int jj = 0; jj < JG; ++jj)
-        if (jj < gn) run(L.j[g0 + jj], nullptr, nullptr, vd, std::true_type{});
-    } else {
-#pragma unroll
-      for (int jj = 0; jj < JG; ++jj)
-        if (jj < gn) run(L.j[g0 + jj], nullptr, nullptr, vd, std::false_type{});
-    }
+    for (int jj = 0; jj < JG; ++jj)
+      if (jj < gn) run(L.j[g0 + jj], nullptr, nullptr, vd);
   } else if constexpr (MAXB > 0) {
     V ka[MAXB], kb[MAXB];  // the group's key tile, read once
 #pragma unroll
     for (int d = 0; d < MAXB; ++d)
       if (d < beta) {
-        ka[d] = kld<CPT>(J0.key + (size_t)d * kstride + koff);
-        kb[d] = kld<CPT>(J0.key + (size_t)(dnum + d) * kstride + koff);
+        ka[d] = ld_key(J0, 0, d);
+        kb[d] = ld_key(J0, 1, d);
       }
-    if (fa_on) {
 #pragma unroll
-      for (int jj = 0; jj < JG; ++jj)
-        if (jj < gn) run(L.j[g0 + jj], ka, kb, nullptr, std::true_type{});
-    } else {
-#pragma unroll
-      for (int jj = 0; jj < JG; ++jj)
-        if (jj < gn) run(L.j[g0 + jj], ka, kb, nullptr, std::false_type{});
-    }
+    for (int jj = 0; jj < JG; ++jj)
+      if (jj < gn) run(L.j[g0 + jj], ka, kb, nullptr);
   } else {
-    for (int jj = 0; jj < gn; ++jj) run(L.j[g0 + jj], nullptr, nullptr, nullptr, std::false_type{});
+    for (int jj = 0; jj < gn; ++jj) run(L.j[g0 + jj], nullptr, nullptr, nullptr);
   }
 }
 

@@ -75,3 +75,55 @@ def test_stage_bounds(logp, le):
             bound = max(0.5 if red else 2 * bound, 0.5 + 2 * bound / 8)
     assert bound < 2
 
+
+
+class Acc:
+    """F64Acc (csrc/f64arith.cuh)."""
+    H0 = 1.25 * 2.0 ** 103
+
+    def __init__(self):
+        self.h, self.l = self.H0, 0.0
+
+    def mac(self, a, b):
+        n = fma(a, b, self.h)
+        self.l += fma(a, b, -(n - self.h))
+        self.h = n
+
+    def fold(self, q, qinv):
+        w51 = pow(2, 51, q)
+        w51 = float(w51 - q if w51 > q // 2 else w51)
+        return f_mulmod((self.h - self.H0) * 2.0 ** -51, w51, float(q), qinv) + self.l
+
+
+def canon(s, q, qinv):
+    r = fma(-(fma(s, qinv, RND) - RND), q, s)
+    return int(r + q if r < 0 else r)
+
+
+def test_inner_product_is_exact():
+    """The key-switch inner product's extreme cases: four digits, the own one a product of two
+    residues, and the tensor terms with P b0, P b1."""
+    rng = random.Random(3)
+    for q in primes():
+        qd, qinv = float(q), 1.0 / q
+        pick = lambda: rng.choice([rng.randrange(q), q - 1, q - 1 - rng.randrange(2), 0])  # noqa: E731
+        for it in range(300):
+            acc, want = Acc(), 0
+            for d in range(4):
+                x = float(pick())
+                if d == it % 5:
+                    y = pick()
+                    x, x0 = f_mulmod(x, float(y), qd, qinv), int(x) * y
+                    assert (int(x) - x0) % q == 0 and abs(x) <= 0.75 * q + 1
+                k = pick()
+                acc.mac(x, float(k))
+                want += int(x) * k
+            P = rng.randrange(-(q // 2), q // 2 + 1)
+            for _ in range(2):
+                p = f_mulmod(float(pick()), float(P), qd, qinv)
+                assert abs(p) <= 0.625 * q + 1
+                a = pick()
+                acc.mac(float(a), p)
+                want += a * int(p)
+            s = acc.fold(q, qinv)
+            assert abs(s) < 2.0 ** 53 and canon(s, qd, qinv) == want % q
