@@ -1,8 +1,6 @@
 // Butterfly-rate calibration: the rate at which one B200 runs the NTT's butterflies with no
 // memory traffic at all (the 64-bit integer form, and the FP64 form used for primes below
-// 2^50).  The forward butterfly (ct_bf_small: one 64-bit Shoup product and
-// two 64-bit additions) is bound by the FMA-heavy pipe, where the IMAD family executes,
-// so this rate -- not HBM bandwidth -- is the compute roofline of the NTT passes.
+// 2^50): the compute roofline of the NTT passes.
 #include "ntt_impl.cuh"
 
 namespace fides {
@@ -21,14 +19,13 @@ __global__ void __launch_bounds__(CAL_THREADS) bf_peak_kernel(uint64_t* out, uin
   const uint64_t seed = (uint64_t)(blockIdx.x * blockDim.x + threadIdx.x) * 0x9E3779B97F4A7C15ull;
 #pragma unroll
   for (int r = 0; r < CAL_E; ++r) x[r] = (seed + (uint64_t)r * 0x2545F4914F6CDD1Dull) % q;
-  const uint64_t q2 = 2 * q;
   for (int it = 0; it < rounds; ++it) {
 #pragma unroll
     for (int b = 3; b >= 0; --b) {
       const ShoupConst w = b == 3 ? w0 : b == 2 ? w1 : b == 1 ? w2 : w3;
 #pragma unroll
       for (int r = 0; r < CAL_E; ++r)
-        if (!(r & (1 << b))) nttk::ct_bf_small(x[r], x[r | (1 << b)], w, q, q2);
+        if (!(r & (1 << b))) nttk::ct_bf4(x[r], x[r | (1 << b)], w, q, 4 * q);
     }
   }
   uint64_t s = 0;

@@ -44,6 +44,14 @@ __host__ __device__ __forceinline__ uint64_t submod(uint64_t a, uint64_t b, uint
   return a >= b ? a - b : a + q - b;
 }
 
+// x w mod q in [0, 4q), any x < 2^64: the quotient without its lowest partial product and the carries of
+// the two middle ones (three products instead of four and their carry chain), at most 3 too small.
+__device__ __forceinline__ uint64_t shoup_lazy4(uint64_t x, uint64_t w, uint64_t ws, uint64_t q) {
+  const uint32_t x0 = (uint32_t)x, x1 = (uint32_t)(x >> 32), s0 = (uint32_t)ws, s1 = (uint32_t)(ws >> 32);
+  const uint64_t k = (uint64_t)x1 * s1 + __umulhi(x1, s0) + __umulhi(x0, s1);
+  return x * w - k * q;
+}
+
 // 128-bit accumulator (lo, hi).
 struct U128 {
   uint64_t lo, hi;

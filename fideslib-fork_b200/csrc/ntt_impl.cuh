@@ -67,19 +67,31 @@ __device__ __forceinline__ void ct_bf(uint64_t& x, uint64_t& y, ShoupConst w, ui
   y = a - t + q2;
 }
 
-// Cooley-Tukey butterfly without any conditional subtraction, for q < 2^58: inputs below
-// B give outputs below B + 2q; over at most 17 stages from [0, q) values stay below 35q.
-__device__ __forceinline__ void ct_bf_small(uint64_t& x, uint64_t& y, ShoupConst w, uint64_t q, uint64_t q2) {
-  uint64_t t = shoup_lazy(y, w.w, w.ws, q);
-  uint64_t a = x;
+// The same with shoup_lazy4's product t below 4q (q < 2^61): x + t and x - t + 4q, so values grow by
+// 4q a stage.
+__device__ __forceinline__ void ct_bf4(uint64_t& x, uint64_t& y, ShoupConst w, uint64_t q, uint64_t q4) {
+  const uint64_t t = shoup_lazy4(y, w.w, w.ws, q);
+  const uint64_t a = x;
   x = a + t;
-  y = a - t + q2;
+  y = a - t + q4;
+}
+// Where a forward chunk brings x back below `cm` before its butterflies (x is below 2 cm there): on
+// the chunk's first stage always, on the third with `third`, on the others with `odd`.
+struct Lazy4Red {
+  uint64_t cm;
+  bool third, odd;
+};
+// q < 2^59: values stay below 32q with one subtraction of 16q a chunk (of at most four stages);
+// q < 2^60: below 16q with 8q every second stage; q < 2^61: below 8q with 4q every stage.
+__device__ __forceinline__ Lazy4Red lazy4_red(uint64_t q) {
+  return Lazy4Red{q < (1ull << 59) ? 16 * q : q < (1ull << 60) ? 8 * q : 4 * q, q >= (1ull << 59), q >= (1ull << 60)};
 }
 
 // Gentleman-Sande butterfly with a tracked bound B (a multiple of q, values < B <= 2^63):
 // the sum doubles the bound unless `red` (B > 2^62), in which case it is brought back
 // below B by one conditional subtraction; the difference path leaves a Shoup product in
-// [0, 2q).  With q < 2^62 this degenerates to Harvey's form once B reaches 2q.
+// [0, 2q).  With q < 2^62 this degenerates to Harvey's form once B reaches 2q.  With shoup_lazy4
+// (q < 2^61) it is in [0, 4q) instead: B starts at 2q there, so that a stage's 2B covers it.
 __device__ __forceinline__ void gs_bf(uint64_t& x, uint64_t& y, ShoupConst w, uint64_t q, uint64_t B, bool red) {
   uint64_t s = x + y;
   if (red) s = csub(s, B);
@@ -146,16 +158,22 @@ __device__ __forceinline__ int padu(int u) {
 // Butterflies of pair bits [BLO, BHI] (in u) for a thread whose registers span bits
 // [LO, LO + LE).  FWD walks bits high -> low, inverse low -> high.  tw: the chunk's twiddles of
 // this thread (SLOTS heaps interleaved, see ntt.cuh).
-template <int LE, int LOGP, int LO, int BHI, int BLO, int SLOTS, bool FWD, int PASS, bool SMALL>
+template <int LE, int LOGP, int LO, int BHI, int BLO, int SLOTS, bool FWD, int PASS, bool LAZY4>
 __device__ __forceinline__ void run_chunk(uint64_t (&x)[1 << LE], const ShoupConst* tw, const DevPrime& pr,
                                           ShoupConst last, uint64_t& B, uint64_t pol) {
   constexpr int E = 1 << LE;
+  const Lazy4Red lr4 = lazy4_red(pr.q);
 #pragma unroll
   for (int k = 0; k <= BHI - BLO; ++k) {
     const int b = FWD ? (BHI - k) : (BLO + k);
     const int rb = b - LO;
     const int H = E >> (rb + 1);  // twiddles of this stage
     const bool red = !FWD && B > (1ull << 62);
+    if (FWD && LAZY4 && (k == 0 || (k == 2 ? lr4.third : lr4.odd))) {
+#pragma unroll
+      for (int r = 0; r < E; ++r)
+        if (!(r >> rb & 1)) x[r] = csub(x[r], lr4.cm);
+    }
 #pragma unroll
     for (int hi = 0; hi < H; ++hi) {
       if (!FWD && PASS == COL && b == LOGP - 1) {
@@ -172,11 +190,15 @@ __device__ __forceinline__ void run_chunk(uint64_t (&x)[1 << LE], const ShoupCon
 #pragma unroll
         for (int lr = 0; lr < (1 << rb); ++lr) {
           const int r0 = (hi << (rb + 1)) | lr, r1 = r0 | (1 << rb);
-          if (FWD && SMALL)
-            ct_bf_small(x[r0], x[r1], w, pr.q, pr.q2);
+          if (FWD && LAZY4)
+            ct_bf4(x[r0], x[r1], w, pr.q, 2 * pr.q2);
           else if (FWD)
             ct_bf(x[r0], x[r1], w, pr.q, pr.q2);
-          else
+          else if (LAZY4) {
+            const uint64_t sum = x[r0] + x[r1];
+            x[r1] = shoup_lazy4(x[r0] - x[r1] + B, w.w, w.ws, pr.q);
+            x[r0] = red ? csub(sum, B) : sum;
+          } else
             gs_bf(x[r0], x[r1], w, pr.q, B, red);
         }
       }
@@ -236,9 +258,8 @@ __device__ __forceinline__ void run_chunk_f64(double (&x)[1 << LE], const double
   }
 }
 
-// Bound of the inverse transform's values after `stages` stages from reduced input.
-__device__ __forceinline__ uint64_t inv_bound(uint64_t q, int stages) {
-  uint64_t B = q;
+// Bound of the inverse transform's values after `stages` stages from the bound B of its input.
+__device__ __forceinline__ uint64_t inv_bound(uint64_t B, int stages) {
   for (int i = 0; i < stages; ++i)
     if (B <= (1ull << 62)) B <<= 1;
   return B;
@@ -254,10 +275,10 @@ struct Chunk {
   static constexpr int SLOTS = tw_slots(LOGP, FWD, LE, C), OFF = tw_off(LOGP, FWD, LE, C);
 };
 
-template <int LE, int LOGP, int PASS, bool FWD, bool SMALL, typename CH>
+template <int LE, int LOGP, int PASS, bool FWD, bool LAZY4, typename CH>
 __device__ __forceinline__ void one_chunk(uint64_t (&x)[1 << LE], CH, int t, const ShoupConst* tw, const DevPrime& pr,
                                           ShoupConst last, uint64_t& B, uint64_t pol) {
-  run_chunk<LE, LOGP, CH::LO, CH::BHI, CH::BLO, CH::SLOTS, FWD, PASS, SMALL>(x, tw + CH::OFF + (t >> CH::LO), pr, last,
+  run_chunk<LE, LOGP, CH::LO, CH::BHI, CH::BLO, CH::SLOTS, FWD, PASS, LAZY4>(x, tw + CH::OFF + (t >> CH::LO), pr, last,
                                                                              B, pol);
 }
 template <int LE, int LOGP, int PASS, bool FWD, typename CH>
@@ -277,14 +298,14 @@ __device__ __forceinline__ void pass_sync() {
 }
 
 // The register chunks of one pass, separated by shared-memory exchanges.
-template <int LE, int LOGP, int PASS, bool FWD, bool SMALL, bool WARP, typename SIDX>
+template <int LE, int LOGP, int PASS, bool FWD, bool LAZY4, bool WARP, typename SIDX>
 __device__ __forceinline__ void chunks(uint64_t (&x)[1 << LE], uint64_t* sm, SIDX sidx, int g, int t,
                                        const ShoupConst* tw, const DevPrime& pr, ShoupConst last, uint64_t& B,
                                        bool direct_load, uint64_t pol) {
   constexpr int E = 1 << LE;
   constexpr int NCH = (LOGP + LE - 1) / LE;
   using C0 = Chunk<LE, LOGP, FWD, 0>;
-  one_chunk<LE, LOGP, PASS, FWD, SMALL>(x, C0{}, t, tw, pr, last, B, pol);
+  one_chunk<LE, LOGP, PASS, FWD, LAZY4>(x, C0{}, t, tw, pr, last, B, pol);
   if constexpr (NCH > 1) {
     using C1 = Chunk<LE, LOGP, FWD, 1>;
     if (!direct_load) pass_sync<WARP>();
@@ -293,7 +314,7 @@ __device__ __forceinline__ void chunks(uint64_t (&x)[1 << LE], uint64_t* sm, SID
     pass_sync<WARP>();
 #pragma unroll
     for (int r = 0; r < E; ++r) x[r] = sm[sidx(g, u_of<C1::LO, LE>(t, r))];
-    one_chunk<LE, LOGP, PASS, FWD, SMALL>(x, C1{}, t, tw, pr, last, B, pol);
+    one_chunk<LE, LOGP, PASS, FWD, LAZY4>(x, C1{}, t, tw, pr, last, B, pol);
   }
   if constexpr (NCH > 2) {
     using C1 = Chunk<LE, LOGP, FWD, 1>;
@@ -304,7 +325,7 @@ __device__ __forceinline__ void chunks(uint64_t (&x)[1 << LE], uint64_t* sm, SID
     pass_sync<WARP>();
 #pragma unroll
     for (int r = 0; r < E; ++r) x[r] = sm[sidx(g, u_of<C2::LO, LE>(t, r))];
-    one_chunk<LE, LOGP, PASS, FWD, SMALL>(x, C2{}, t, tw, pr, last, B, pol);
+    one_chunk<LE, LOGP, PASS, FWD, LAZY4>(x, C2{}, t, tw, pr, last, B, pol);
   }
   static_assert(NCH <= 3, "sub-transform too large");
 }
@@ -516,18 +537,19 @@ __global__ void __launch_bounds__(PassThreads<LOGN, PASS, G, LE>::NT, PassThread
     }
   } else {
   const ShoupConst* tw = reinterpret_cast<const ShoupConst*>(tw_prime) + tw0;
-  uint64_t B = pr.q;  // inverse: bound of the values (a multiple of q)
-  if (!FWD && PASS == COL) B = inv_bound(pr.q, PassShape<LOGN, ROW>::LOGP);
-  if (FWD && pr.q < (1ull << 58))
+  const bool lazy4 = pr.q < (1ull << 61);
+  uint64_t B = lazy4 ? pr.q2 : pr.q;  // inverse: bound of the values (a multiple of q)
+  if (!FWD && PASS == COL) B = inv_bound(B, PassShape<LOGN, ROW>::LOGP);
+  if (lazy4)
     chunks<LE, LOGP, PASS, FWD, true, WARP>(x, sm, sidx, g, t, tw, pr, last, B, direct_load && !STAGE_PRO, pol);
   else
     chunks<LE, LOGP, PASS, FWD, false, WARP>(x, sm, sidx, g, t, tw, pr, last, B, direct_load && !STAGE_PRO, pol);
 
   // ---- final reduction of the completed transform
   if (FWD && PASS == ROW) {
-    if (pr.q < (1ull << 58)) {
+    if (lazy4) {
 #pragma unroll
-      for (int r = 0; r < E; ++r) x[r] = shoup(x[r], 1, pr.one_s, pr.q);  // x < 35q
+      for (int r = 0; r < E; ++r) x[r] = shoup(x[r], 1, pr.one_s, pr.q);  // any 64-bit x
     } else {
 #pragma unroll
       for (int r = 0; r < E; ++r) x[r] = csub(csub(x[r], pr.q2), pr.q);   // x < 4q

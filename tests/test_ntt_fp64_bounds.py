@@ -76,6 +76,41 @@ def test_stage_bounds(logp, le):
     assert bound < 2
 
 
+def test_lazy4_product_range():
+    """shoup_lazy4 (csrc/modarith.cuh): y w mod q plus 0 to 3 q, for any 64-bit y and q < 2^61."""
+    from fides_b200 import params
+    rng = random.Random(9)
+    for q in (params.gen_primes(16, 61, 2) + params.gen_primes(16, 60, 2) + params.gen_primes(16, 59, 1) +
+              params.gen_primes(16, 51, 1)):
+        for it in range(3000):
+            w = rng.choice([rng.randrange(q), q - 1 - rng.randrange(3), rng.randrange(3)])
+            y = rng.choice([rng.randrange(1 << 64), (1 << 64) - 1 - rng.randrange(1 << 33), rng.randrange(1 << 33),
+                            rng.randrange(1 << 32) << 32, (rng.randrange(1 << 32) << 32) | 0xffffffff])
+            ws = (w << 64) // q
+            y0, y1, s0, s1 = y & 0xffffffff, y >> 32, ws & 0xffffffff, ws >> 32
+            k = y1 * s1 + (y1 * s0 >> 32) + (y0 * s1 >> 32)
+            assert k < 1 << 64 and 0 <= y * w - k * q < 4 * q
+
+
+@pytest.mark.parametrize("bits", [51, 58, 59, 60, 61])
+def test_lazy4_forward_bounds(bits):
+    """Forward values with the chunk-wise subtractions of Lazy4Red stay below 2^64; x is below 2 cm
+    where it is subtracted."""
+    q = (1 << bits) - 1  # any value of this size
+    cm = 16 * q if q < 1 << 59 else 8 * q if q < 1 << 60 else 4 * q
+    third, odd = q >= 1 << 59, q >= 1 << 60
+    for le in (3, 4):
+        for logp in (5, 6, 7, 8, 9):
+            bound = q
+            for _ in range(2):  # the column pass, then the row pass
+                for c in range(-(-logp // le)):
+                    for k in range(min(le, logp - c * le)):
+                        if k == 0 or (third if k == 2 else odd):
+                            assert bound <= 2 * cm
+                            bound = max(cm, bound - cm)
+                        bound += 4 * q
+                        assert bound <= 1 << 64
+
 
 class Acc:
     """F64Acc (csrc/f64arith.cuh)."""
