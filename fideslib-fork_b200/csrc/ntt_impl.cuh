@@ -440,7 +440,10 @@ __global__ void __launch_bounds__(PassThreads<LOGN, PASS, G, LE>::NT, PassThread
   constexpr int WT = WARP && NT > 32 ? 32 : NT;  // threads that share a staged block
   const int blk = WARP ? tid / WT : 0, lane = tid % WT;
 
-  uint64_t x[E];
+  uint64_t x[E];  // residues, or the bits of FP64 ones
+  const bool f64 = pr.q < NTT_F64_MAX;  // uniform per CTA: one limb per CTA
+  F64Prime fp{};
+  if (f64) fp = a.f64[lr.prime];
 
   // ---- input of this pass: the first pass applies the prologue
   constexpr bool first_pass = FWD ? (PASS == COL) : (PASS == ROW);
@@ -456,6 +459,29 @@ __global__ void __launch_bounds__(PassThreads<LOGN, PASS, G, LE>::NT, PassThread
     if (first_pass && IN == IN_CONV_SW) return in[i];  // + P SwitchModulus(top) below
     if (first_pass && IN == IN_ADD_PMUL) return addmod(in[i], shoup(lr.pro[i], pm.w, pm.ws, pr.q), pr.q);
     return in[i];
+  };
+  // The prologues and epilogues of FP64 limbs are FP64 products too: with the butterflies at 8.75-9.5
+  // operations that pipe has room, and a 64-bit integer product with its reduction takes the FMA-heavy
+  // pipe four times as long.  An input need not be canonical: the first forward stage takes values
+  // within 4q, the first inverse stage within q.  A top limb of a larger prime is switched in integers.
+  const bool fp_switch = (IN == IN_SWITCH || IN == IN_CONV_SW) && opr.q < NTT_F64_MAX;
+  auto centred_top = [&](uint64_t v) -> double {  // SwitchModulus: the centred lift, |.| <= 2^49
+    const double t = f_from_u64(v);
+    return v > (opr.q >> 1) ? __dadd_rn(t, -(double)(long long)opr.q) : t;
+  };
+  auto bits = [](double v) { return (uint64_t)__double_as_longlong(v); };
+  // a signed 64-bit integer: its upper word times 2^32, reduced, plus its lower one (below q / 2)
+  const bool fp_signed = IN == IN_SIGNED && pr.q >= (1ull << 33);
+  auto signed_f64 = [&](uint64_t v) -> double {
+    const double hi = __dadd_rn(__hiloint2double(0x45300000, (int)((uint32_t)(v >> 32) ^ 0x80000000u)),
+                                -(0x1p84 + 0x1p63));
+    const double lo = __dadd_rn(__hiloint2double(0x43300000, (int)(uint32_t)v), -F64_TWO52);
+    return __dadd_rn(f_reduce(hi, fp.q, fp.qinv), lo);
+  };
+  auto load_f64 = [&](size_t i) -> uint64_t {
+    if (!first_pass) return in[i];  // the first pass's doubles
+    if (IN == IN_MUL) return bits(f_mulmod(f_from_u64(in[i]), f_from_u64(lr.pro[i]), fp.q, fp.qinv));  // within 3q/4
+    return bits(f_from_u64(load(i)));
   };
 
   // ---- load chunk 0 (direct when lanes map to consecutive addresses, else staged)
@@ -475,67 +501,179 @@ __global__ void __launch_bounds__(PassThreads<LOGN, PASS, G, LE>::NT, PassThread
     }
     cp_async_commit();
   }
-  if (direct_load) {
+  auto fill = [&](auto ld) {
+    if constexpr (direct_load) {
 #pragma unroll
-    for (int r = 0; r < E; ++r) x[r] = load(gidx(sub, u_of<LO0, LE>(t, r)));
-    if constexpr (STAGE_PRO) {
-      cp_async_wait_all();
-      __syncthreads();
+      for (int r = 0; r < E; ++r) x[r] = ld(gidx(sub, u_of<LO0, LE>(t, r)));
+    } else {
 #pragma unroll
-      for (int r = 0; r < E; ++r)
-        x[r] = addmod(x[r], shoup(switch_modulus(sm[sidx(g, u_of<LO0, LE>(t, r))], opr, pr), pm.w, pm.ws, pr.q), pr.q);
+      for (int k = 0; k < E; ++k) {
+        const int e = k * WT + lane;
+        const int gg = blk * (WT / T) + e / P, u = e % P;
+        sm[sidx(gg, u)] = ld(gidx(sub0 + gg, u));
+      }
+      pass_sync<WARP>();
+#pragma unroll
+      for (int r = 0; r < E; ++r) x[r] = sm[sidx(g, u_of<LO0, LE>(t, r))];
     }
-  } else {
-#pragma unroll
-    for (int k = 0; k < E; ++k) {
-      const int e = k * WT + lane;
-      const int gg = blk * (WT / T) + e / P, u = e % P;
-      sm[sidx(gg, u)] = load(gidx(sub0 + gg, u));
-    }
-    pass_sync<WARP>();
-#pragma unroll
-    for (int r = 0; r < E; ++r) x[r] = sm[sidx(g, u_of<LO0, LE>(t, r))];
-  }
+  };
 
   // ---- epilogue operand: start fetching it into shared memory (after the data region)
   constexpr bool EPS = EpStage<PASS, FWD, OUT>::on;
   uint64_t* sep = sm + G * PADP;
-  if constexpr (EPS) {
-    const uint64_t* e0 = lr.ep0 + (size_t)sub0 * P;
+  auto fetch_epilogue = [&] {
+    if constexpr (EPS) {
+      const uint64_t* e0 = lr.ep0 + (size_t)sub0 * P;
 #pragma unroll
-    for (int k = 0; k < E / 2; ++k) {
-      const int at = blk * (WT * E) + 2 * (k * WT + lane);
-      cp_async16(sep + at, e0 + at);
+      for (int k = 0; k < E / 2; ++k) {
+        const int at = blk * (WT * E) + 2 * (k * WT + lane);
+        cp_async16(sep + at, e0 + at);
+      }
+      cp_async_commit();
     }
-    cp_async_commit();
-  }
+  };
 
-  // ---- chunks
-  const uint64_t pol = l2_evict_last_policy();
-  const bool f64 = pr.q < NTT_F64_MAX;  // uniform per CTA: one limb per CTA
+  // ---- store (the last pass applies the epilogue)
+  constexpr bool last_pass = !first_pass;
+  ShoupConst pinv{0, 0};
+  RescaleConst rsc{0, 0, 0, 0};
+  if (OUT == OUT_MODDOWN || OUT == OUT_SUB_PINV) pinv = a.pinv[lr.prime];
+  if (OUT == OUT_MDRS) pinv = a.pqinv[(size_t)lr.aux * a.n_q + lr.prime];
+  if (OUT == OUT_RESCALE || OUT == OUT_MDRS) rsc = a.rescale[(size_t)lr.aux * a.n_q + lr.prime];
+  auto ep0 = [&](size_t i) -> uint64_t {
+    if constexpr (EPS) return sep[i - (size_t)sub0 * P];
+    return lr.ep0[i];
+  };
+  auto finish = [&](size_t i, uint64_t v, uint64_t e0) {
+    if (OUT == OUT_MODDOWN || OUT == OUT_MDRS) {
+      v = shoup(submod(e0, v, pr.q), pinv.w, pinv.ws, pr.q);
+      if (lr.ep1) {
+        const uint64_t e = lr.ep1[i];
+        v = addmod(v, OUT == OUT_MDRS ? shoup(e, rsc.qinv, rsc.qinv_s, pr.q) : e, pr.q);
+      }
+    } else if (OUT == OUT_RESCALE) {
+      v = addmod(shoup(e0, rsc.qinv, rsc.qinv_s, pr.q), shoup(v, rsc.m, rsc.m_s, pr.q), pr.q);
+    } else if (OUT == OUT_SUB_PINV) {
+      v = shoup(submod(v, e0, pr.q), pinv.w, pinv.ws, pr.q);
+    }
+    data[i] = v;
+  };
+  // the same on a transform's FP64 result, within 2q; every epilogue leaves less than 2q
+  auto centred = [&](uint64_t w) -> double {
+    const double d = f_from_u64(w);
+    return w > (pr.q >> 1) ? __dadd_rn(d, -fp.q) : d;
+  };
+  double f_pinv = 0, f_qinv = 0, f_m = 0, f_q2t = 0;
   if (f64) {
-    // FP64 butterflies; every pass of such a limb stores canonical residues
-    const F64Prime fp = a.f64[lr.prime];
+    if (OUT == OUT_MODDOWN || OUT == OUT_SUB_PINV || OUT == OUT_MDRS) f_pinv = centred(pinv.w);
+    if (OUT == OUT_RESCALE || OUT == OUT_MDRS) f_qinv = centred(rsc.qinv);
+    if (OUT == OUT_RESCALE) f_m = centred(rsc.m);
+    f_q2t = __dadd_rn(2.0 * fp.q, F64_TWO52);
+  }
+  auto finish_f64 = [&](size_t i, uint64_t b, uint64_t e0) {
+    if (!last_pass) {
+      data[i] = b;
+      return;
+    }
+    double v = __longlong_as_double((long long)b);
+    if (OUT == OUT_MODDOWN || OUT == OUT_MDRS) {
+      v = f_mulmod(__dsub_rn(f_from_u64(e0), v), f_pinv, fp.q, fp.qinv);  // |e0 - v| < 3q: within 0.875q
+      if (lr.ep1) {
+        const double e = f_from_u64(lr.ep1[i]);
+        v = __dadd_rn(v, OUT == OUT_MDRS ? f_mulmod(e, f_qinv, fp.q, fp.qinv) : e);
+      }
+    } else if (OUT == OUT_RESCALE) {
+      v = __dadd_rn(f_mulmod(f_from_u64(e0), f_qinv, fp.q, fp.qinv), f_mulmod(v, f_m, fp.q, fp.qinv));
+    } else if (OUT == OUT_SUB_PINV) {
+      v = f_mulmod(__dsub_rn(v, f_from_u64(e0)), f_pinv, fp.q, fp.qinv);
+    }
+    data[i] = f_to_canon(v, f_q2t, pr.q);
+  };
+  constexpr int LOL = Chunk<LE, LOGP, FWD, NCH - 1>::LO;
+  constexpr bool direct_store = (PASS == COL) || (LOL == LOGP - LE);
+  auto drain = [&](auto st) {
+    if constexpr (EPS) {
+      cp_async_wait_all();
+      if (direct_store) pass_sync<WARP>();  // the staged store below synchronises anyway
+    }
+    if constexpr (direct_store) {
+      if constexpr (OUT == OUT_SUB_PINV) {
+        // the epilogue loads ahead of the stores: a store may alias the next load's address, and
+        // sixteen load-store round trips in turn took 15.7 us on 2 limbs, where a plain pass takes 4.4
+        constexpr int H = 8;  // in blocks of eight, which the register budget holds
+#pragma unroll
+        for (int r0 = 0; r0 < E; r0 += H) {
+          uint64_t e[H];
+#pragma unroll
+          for (int r = 0; r < H; ++r) e[r] = lr.ep0[gidx(sub, u_of<LOL, LE>(t, r0 + r))];
+#pragma unroll
+          for (int r = 0; r < H; ++r) st(gidx(sub, u_of<LOL, LE>(t, r0 + r)), x[r0 + r], e[r]);
+        }
+      } else {
+#pragma unroll
+        for (int r = 0; r < E; ++r) {
+          const size_t i = gidx(sub, u_of<LOL, LE>(t, r));
+          st(i, x[r], OUT == OUT_PLAIN ? 0 : ep0(i));
+        }
+      }
+    } else {
+      pass_sync<WARP>();
+#pragma unroll
+      for (int r = 0; r < E; ++r) sm[sidx(g, u_of<LOL, LE>(t, r))] = x[r];
+      pass_sync<WARP>();
+#pragma unroll
+      for (int k = 0; k < E; ++k) {
+        const int e = k * WT + lane;
+        const int gg = blk * (WT / T) + e / P, u = e % P;
+        const size_t i = gidx(sub0 + gg, u);
+        st(i, sm[sidx(gg, u)], OUT == OUT_PLAIN ? 0 : ep0(i));
+      }
+    }
+  };
+
+  const uint64_t pol = l2_evict_last_policy();
+  if (f64) {
+    if (first_pass && IN == IN_SIGNED && fp_signed)
+      fill([&](size_t i) { return bits(signed_f64(lr.pro[i])); });
+    else if (first_pass && IN == IN_SWITCH && fp_switch)
+      fill([&](size_t i) { return bits(f_reduce(centred_top(lr.pro[i]), fp.q, fp.qinv)); });
+    else
+      fill(load_f64);
+    fetch_epilogue();
+    if constexpr (STAGE_PRO) {
+      cp_async_wait_all();
+      __syncthreads();
+      auto add_top = [&](auto lift) {
+#pragma unroll
+        for (int r = 0; r < E; ++r) {
+          const double c = lift(sm[sidx(g, u_of<LO0, LE>(t, r))]);
+          x[r] = bits(__dadd_rn(__longlong_as_double((long long)x[r]), f_mulmod(c, fp.pm, fp.q, fp.qinv)));
+        }
+      };
+      if (fp_switch)
+        add_top(centred_top);
+      else
+        add_top([&](uint64_t v) { return f_from_u64(switch_modulus(v, opr, pr)); });
+    }
     double xf[E];
-    if (first_pass) {
-      // canonical inputs in [0, q): within the bounds of a pass's first stage as they are
 #pragma unroll
-      for (int r = 0; r < E; ++r) xf[r] = f_from_u64(x[r]);
-    } else {
-#pragma unroll
-      for (int r = 0; r < E; ++r) xf[r] = __longlong_as_double((long long)x[r]);  // the first pass's doubles
-    }
+    for (int r = 0; r < E; ++r) xf[r] = __longlong_as_double((long long)x[r]);
     chunks_f64<LE, LOGP, PASS, FWD, WARP>(xf, sm, sidx, g, t, reinterpret_cast<const double*>(tw_prime) + tw0, fp,
-                                    direct_load && !STAGE_PRO, pol);
-    if (first_pass) {
+                                          direct_load && !STAGE_PRO, pol);
 #pragma unroll
-      for (int r = 0; r < E; ++r) x[r] = (uint64_t)__double_as_longlong(xf[r]);
-    } else {
-      const double q2t = __dadd_rn(2.0 * fp.q, F64_TWO52);
+    for (int r = 0; r < E; ++r) x[r] = bits(xf[r]);
+    drain(finish_f64);
+    return;
+  }
+  fill(load);
+  fetch_epilogue();
+  if constexpr (STAGE_PRO) {
+    cp_async_wait_all();
+    __syncthreads();
 #pragma unroll
-      for (int r = 0; r < E; ++r) x[r] = f_to_canon(xf[r], q2t, pr.q);
-    }
-  } else {
+    for (int r = 0; r < E; ++r)
+      x[r] = addmod(x[r], shoup(switch_modulus(sm[sidx(g, u_of<LO0, LE>(t, r))], opr, pr), pm.w, pm.ws, pr.q), pr.q);
+  }
   const ShoupConst* tw = reinterpret_cast<const ShoupConst*>(tw_prime) + tw0;
   const bool lazy4 = pr.q < (1ull << 61);
   uint64_t B = lazy4 ? pr.q2 : pr.q;  // inverse: bound of the values (a multiple of q)
@@ -555,53 +693,7 @@ __global__ void __launch_bounds__(PassThreads<LOGN, PASS, G, LE>::NT, PassThread
       for (int r = 0; r < E; ++r) x[r] = csub(csub(x[r], pr.q2), pr.q);   // x < 4q
     }
   }
-  }
-
-  // ---- store (the last pass applies the epilogue)
-  ShoupConst pinv{0, 0};
-  RescaleConst rsc{0, 0, 0, 0};
-  if (OUT == OUT_MODDOWN || OUT == OUT_SUB_PINV) pinv = a.pinv[lr.prime];
-  if (OUT == OUT_MDRS) pinv = a.pqinv[(size_t)lr.aux * a.n_q + lr.prime];
-  if (OUT == OUT_RESCALE || OUT == OUT_MDRS) rsc = a.rescale[(size_t)lr.aux * a.n_q + lr.prime];
-  auto ep0 = [&](size_t i) -> uint64_t {
-    if constexpr (EPS) return sep[i - (size_t)sub0 * P];
-    return lr.ep0[i];
-  };
-  auto store = [&](size_t i, uint64_t v) {
-    if (OUT == OUT_MODDOWN || OUT == OUT_MDRS) {
-      v = shoup(submod(ep0(i), v, pr.q), pinv.w, pinv.ws, pr.q);
-      if (lr.ep1) {
-        const uint64_t e = lr.ep1[i];
-        v = addmod(v, OUT == OUT_MDRS ? shoup(e, rsc.qinv, rsc.qinv_s, pr.q) : e, pr.q);
-      }
-    } else if (OUT == OUT_RESCALE) {
-      v = addmod(shoup(ep0(i), rsc.qinv, rsc.qinv_s, pr.q), shoup(v, rsc.m, rsc.m_s, pr.q), pr.q);
-    } else if (OUT == OUT_SUB_PINV) {
-      v = shoup(submod(v, lr.ep0[i], pr.q), pinv.w, pinv.ws, pr.q);
-    }
-    data[i] = v;
-  };
-  constexpr int LOL = Chunk<LE, LOGP, FWD, NCH - 1>::LO;
-  constexpr bool direct_store = (PASS == COL) || (LOL == LOGP - LE);
-  if constexpr (EPS) {
-    cp_async_wait_all();
-    if (direct_store) pass_sync<WARP>();  // the staged store below synchronises anyway
-  }
-  if (direct_store) {
-#pragma unroll
-    for (int r = 0; r < E; ++r) store(gidx(sub, u_of<LOL, LE>(t, r)), x[r]);
-  } else {
-    pass_sync<WARP>();
-#pragma unroll
-    for (int r = 0; r < E; ++r) sm[sidx(g, u_of<LOL, LE>(t, r))] = x[r];
-    pass_sync<WARP>();
-#pragma unroll
-    for (int k = 0; k < E; ++k) {
-      const int e = k * WT + lane;
-      const int gg = blk * (WT / T) + e / P, u = e % P;
-      store(gidx(sub0 + gg, u), sm[sidx(gg, u)]);
-    }
-  }
+  drain(finish);
 }
 
 
