@@ -17,6 +17,7 @@
 
 #include "conv_tc.hpp"
 #include "kernels.cuh"
+#include "launch.cuh"
 
 #ifndef FIDES_TC_SMEM_GUARD
 #define FIDES_TC_SMEM_GUARD 0
@@ -198,8 +199,9 @@ __device__ __forceinline__ void tc_epilogue(uint32_t trow, int j0, int nd, const
   }
 }
 
+template <int CAP>
 __global__ void __launch_bounds__(TC_M, 7)
-    conv_tc_kernel(const __grid_constant__ ConvJobList L, const DevPrime* primes, int logN, uint32_t* status) {
+    conv_tc_kernel(const __grid_constant__ ConvJobListT<CAP> L, const DevPrime* primes, int logN, uint32_t* status) {
   extern __shared__ __align__(1024) uint8_t sm[];
   const ConvJob& J = L.j[blockIdx.y];
   const ConvTable& T = J.t;
@@ -235,6 +237,7 @@ __global__ void __launch_bounds__(TC_M, 7)
     dconst[j] = T.tc_dst[j];
     dofs[j] = j < nd ? T.dst_pos[j] << logN : 0;
   }
+  pdl_wait();  // tables only so far
   {  // A: the bytes of the pre-scaled residues of this thread's coefficient
     uint64_t x[TC_MAX_SRC];
 #pragma unroll
@@ -324,29 +327,38 @@ __global__ void __launch_bounds__(TC_M, 7)
 
 }  // namespace
 
-void launch_conv_tc(Context* c, const ConvJob* jobs, int n, cudaStream_t s) {
-  static thread_local ConvJobList L;
+namespace {
+template <int CAP>
+void launch_conv_tc_list(Context* c, const ConvJob* jobs, int m, cudaStream_t s) {
+  static thread_local ConvJobListT<CAP> L;
   static bool attr = false;
   if (!attr) {
-    FIDES_CUDA(cudaFuncSetAttribute(conv_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    FIDES_CUDA(cudaFuncSetAttribute(conv_tc_kernel<CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     attr = true;
   }
+  L.n = m;
+  std::copy(jobs, jobs + m, L.j);
+  int smem = TC_SMEM_FLOOR;
+  double bytes = 0;
+  for (int i = 0; i < m; ++i) {
+    const ConvTable& t = L.j[i].t;
+    if (!t.tc_b) throw Error(-1, "basis conversion has no tensor-core form");
+    smem = std::max(smem, tc_layout(t.tc_kpad, t.tc_nd_pad).total + FIDES_TC_SMEM_GUARD);
+    bytes += 8.0 * c->N * (t.n_src + t.n_dst);
+  }
+  dim3 grid(c->N / TC_M, m);
+  LaunchScope ls(c, s, KK_CONV, bytes);
+  launch_pdl(conv_tc_kernel<CAP>, grid, TC_M, smem, s, L, c->d_prime, c->logN, c->d_status);
+}
+}  // namespace
+
+void launch_conv_tc(Context* c, const ConvJob* jobs, int n, cudaStream_t s) {
   for (int off = 0; off < n; off += MAX_CONV_JOBS) {
     const int m = std::min(MAX_CONV_JOBS, n - off);
-    L.n = m;
-    std::copy(jobs + off, jobs + off + m, L.j);
-    int smem = TC_SMEM_FLOOR;
-    double bytes = 0;
-    for (int i = 0; i < m; ++i) {
-      const ConvTable& t = L.j[i].t;
-      if (!t.tc_b) throw Error(-1, "basis conversion has no tensor-core form");
-      smem = std::max(smem, tc_layout(t.tc_kpad, t.tc_nd_pad).total + FIDES_TC_SMEM_GUARD);
-      bytes += 8.0 * c->N * (t.n_src + t.n_dst);
-    }
-    dim3 grid(c->N / TC_M, m);
-    LaunchScope ls(c, s, KK_CONV, bytes);
-    conv_tc_kernel<<<grid, TC_M, smem, s>>>(L, c->d_prime, c->logN, c->d_status);
-    FIDES_CUDA(cudaGetLastError());
+    if (m <= FEW_JOBS)
+      launch_conv_tc_list<FEW_JOBS>(c, jobs + off, m, s);
+    else
+      launch_conv_tc_list<MAX_CONV_JOBS>(c, jobs + off, m, s);
   }
 }
 

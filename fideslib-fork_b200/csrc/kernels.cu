@@ -6,6 +6,7 @@
 #include "kernels.cuh"
 #include "conv_tc.hpp"
 #include "f64arith.cuh"
+#include "launch.cuh"
 #include "ntt.cuh"
 
 namespace fides {
@@ -44,6 +45,7 @@ __global__ void __launch_bounds__(EW_THREADS) conv_kernel(const __grid_constant_
     dpos[j] = T.dst_pos[j];
   }
   __syncthreads();
+  pdl_wait();
   const int N = 1 << logN;
   const int n = 2 * (blockIdx.x * blockDim.x + threadIdx.x);
   constexpr int R = NS ? NS : MAX_SRC;
@@ -122,10 +124,10 @@ struct KskMinBlocks {
   static constexpr int value = (JG > 1 || (MAXB >= 1 && MAXB <= 3)) ? 3 : 1;
 };
 
-template <int MAXB, int JG, int CPT, bool SHARE_DIGITS = false>
-__global__ void __launch_bounds__(EW_THREADS, KskMinBlocks<MAXB, JG>::value) ksk_kernel(const __grid_constant__ KskJobList L, const DevPrime* primes,
-                                                            const ShoupConst* pmod, const F64Prime* f64, int logN,
-                                                            int n_q, int K, int dnum, int alpha) {
+template <int MAXB, int JG, int CPT, int CAP, bool SHARE_DIGITS = false>
+__global__ void __launch_bounds__(EW_THREADS, KskMinBlocks<MAXB, JG>::value)
+    ksk_kernel(const __grid_constant__ KskJobListT<CAP> L, const DevPrime* primes, const ShoupConst* pmod,
+               const F64Prime* f64, int logN, int n_q, int K, int dnum, int alpha) {
   using V = KVec<CPT>;
   using D = KDbl<CPT>;
   const int g0 = L.gstart[blockIdx.z], gn = L.gcount[blockIdx.z];
@@ -142,6 +144,7 @@ __global__ void __launch_bounds__(EW_THREADS, KskMinBlocks<MAXB, JG>::value) ksk
   const size_t off = (size_t)i * N + n, koff = (size_t)pid * N + n;
   const bool tensor = J0.a0 && i < l;
   const uint64_t q = primes[pid].q;
+  pdl_wait();
 
   auto ld_digit = [&](const KskJob& J, int d) {
     return kld<CPT>((d == own && J.x) ? J.x + off : J.digits + ((size_t)d * ext + i) * N + n);
@@ -403,6 +406,7 @@ __global__ void __launch_bounds__(EW_THREADS) moddown_finish_kernel(const __grid
   const FinJob& J = L.j[blockIdx.z];
   const int j = blockIdx.y;
   if (j >= J.l) return;
+  pdl_wait();
   const size_t off = ((size_t)j << logN) + blockIdx.x * blockDim.x + threadIdx.x;
   const DevPrime p = primes[j];
   const ShoupConst pi = pinv[j];
@@ -416,6 +420,7 @@ __global__ void __launch_bounds__(EW_THREADS) tensor_kernel(const __grid_constan
   const TensorJob& J = L.j[blockIdx.z];
   const int j = blockIdx.y;
   if (j >= J.l) return;
+  pdl_wait();
   const size_t off = ((size_t)j << logN) + blockIdx.x * blockDim.x + threadIdx.x;
   const DevPrime p = primes[j];
   const uint64_t x0 = J.a0[off], x1 = J.a1[off], y0 = J.b0[off], y1 = J.b1[off];
@@ -432,6 +437,7 @@ __global__ void __launch_bounds__(EW_THREADS) switch_kernel(const __grid_constan
   const SwitchJob& J = L.j[blockIdx.z];
   const int j = blockIdx.y;
   if (j >= J.l - 1) return;
+  pdl_wait();
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   const DevPrime om = primes[J.l - 1], nm = primes[j];
   J.out[((size_t)j << logN) + n] = switch_modulus(J.top[n], om, nm);
@@ -443,6 +449,7 @@ __global__ void __launch_bounds__(EW_THREADS) rescale_finish_kernel(const __grid
   const RescaleJob& J = L.j[blockIdx.z];
   const int j = blockIdx.y;
   if (j >= J.l - 1) return;
+  pdl_wait();
   const size_t off = ((size_t)j << logN) + blockIdx.x * blockDim.x + threadIdx.x;
   const DevPrime p = primes[j];
   const RescaleConst r = rs[(size_t)J.l * n_q + j];
@@ -456,6 +463,7 @@ __global__ void __launch_bounds__(EW_THREADS) addsub_kernel(const __grid_constan
   const AddSubJob& J = L.j[blockIdx.z];
   const int j = blockIdx.y;
   if (j >= J.l) return;
+  pdl_wait();
   const size_t off = ((size_t)j << logN) + 2 * (blockIdx.x * blockDim.x + threadIdx.x);
   const DevPrime p = primes[ext_prime(j, J.lq, J.nq)];
   const uint64_t q = p.q;
@@ -489,6 +497,7 @@ __global__ void __launch_bounds__(EW_THREADS) scalar_kernel(const __grid_constan
   const ScalarJob& J = L.j[blockIdx.z];
   const int j = blockIdx.y;
   if (j >= J.l) return;
+  pdl_wait();
   const size_t off = ((size_t)j << logN) + 2 * (blockIdx.x * blockDim.x + threadIdx.x);
   const DevPrime p = primes[j];
   const uint64_t sc = J.s[j];
@@ -513,6 +522,7 @@ __global__ void __launch_bounds__(EW_THREADS) dot_plain_kernel(const __grid_cons
   const int lane = blockIdx.x, j = blockIdx.z;
   const DevPrime p = primes[ext_prime(j, J.lq, J.nq)];
   const size_t off = ((size_t)j << logN) + 2 * (blockIdx.y * blockDim.x + threadIdx.x);
+  pdl_wait();
   auto ld2 = [](const uint64_t* q) { return *reinterpret_cast<const ulonglong2*>(q); };
   U128 a0{0, 0}, a1{0, 0}, b0{0, 0}, b1{0, 0};
   for (int t0 = 0; t0 < J.n; t0 += LC_BLOCK) {  // as lincomb_kernel
@@ -556,6 +566,7 @@ __global__ void __launch_bounds__(EW_THREADS) bsgs_dot_kernel(const __grid_const
   const int i = blockIdx.x % J.ng, lane = blockIdx.x / J.ng, j = blockIdx.z;
   const DevPrime p = primes[ext_prime(j, J.lq, J.nq)];
   const size_t off = ((size_t)j << logN) + blockIdx.y * blockDim.x + threadIdx.x;
+  pdl_wait();
   uint64_t a[NB], b[NB], w[NB];
 #pragma unroll
   for (int k = 0; k < NB; ++k)
@@ -589,6 +600,7 @@ __global__ void __launch_bounds__(EW_THREADS) bsgs_dot2_kernel(const __grid_cons
   const int i = blockIdx.x % J.ng, lane = blockIdx.x / J.ng, j = blockIdx.z;
   const DevPrime p = primes[ext_prime(j, J.lq, J.nq)];
   const size_t off = ((size_t)j << logN) + 2 * ((size_t)blockIdx.y * blockDim.x + threadIdx.x);
+  pdl_wait();
   auto ld2 = [](const uint64_t* q) { return *reinterpret_cast<const ulonglong2*>(q); };
   ulonglong2 a[NB], b[NB], w[NB];
 #pragma unroll
@@ -616,6 +628,7 @@ __global__ void __launch_bounds__(EW_THREADS) lincomb_kernel(const __grid_consta
   const int j = blockIdx.y, lane = blockIdx.z;
   const DevPrime p = primes[ext_prime(j, J.lq, J.nq)];
   const size_t off = ((size_t)j << logN) + 2 * (blockIdx.x * blockDim.x + threadIdx.x);
+  pdl_wait();
   auto ld2 = [](const uint64_t* q) { return *reinterpret_cast<const ulonglong2*>(q); };
   U128 a0{0, 0}, a1{0, 0}, b0{0, 0}, b1{0, 0};
   // terms in blocks of LC_BLOCK whose loads are all issued before their products, so that a
@@ -705,7 +718,7 @@ void launch_conv(Context* c, const ConvJob* jobs, int n, cudaStream_t s) {
       FIDES_CUDA(cudaFuncSetAttribute(conv_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024)); \
       attr = true;                                                                                            \
     }                                                                                                         \
-    conv_kernel<K><<<grid, EW_THREADS, smem, s>>>(L, c->d_prime, c->logN);                                    \
+    launch_pdl(conv_kernel<K>, grid, EW_THREADS, smem, s, L, c->d_prime, c->logN);                                    \
     break;                                                                                                    \
   }
         FIDES_CONV_CASE(1) FIDES_CONV_CASE(2) FIDES_CONV_CASE(3) FIDES_CONV_CASE(4) FIDES_CONV_CASE(5)
@@ -719,11 +732,10 @@ void launch_conv(Context* c, const ConvJob* jobs, int n, cudaStream_t s) {
             FIDES_CUDA(cudaFuncSetAttribute(conv_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
             attr = true;
           }
-          conv_kernel<0><<<grid, EW_THREADS, smem, s>>>(L, c->d_prime, c->logN);
+          launch_pdl(conv_kernel<0>, grid, EW_THREADS, smem, s, L, c->d_prime, c->logN);
         }
       }
-      FIDES_CUDA(cudaGetLastError());
-    }
+        }
   }
 }
 
@@ -732,8 +744,7 @@ void launch_dot_plain(Context* c, const DotJob& job, cudaStream_t s) {
   if (job.lanes < 1 || job.lanes > MAX_DOT_LANES) throw Error(-1, "dot product needs 1..8 lanes");
   dim3 grid(job.lanes, c->N / (2 * EW_THREADS), job.l);
   LaunchScope ls(c, s, KK_ELEM, 8.0 * c->N * job.l * (job.n + job.lanes * (2.0 * job.n + 2)));
-  dot_plain_kernel<<<grid, EW_THREADS, 0, s>>>(job, c->d_prime, c->logN);
-  FIDES_CUDA(cudaGetLastError());
+  launch_pdl(dot_plain_kernel, grid, EW_THREADS, 0, s, job, c->d_prime, c->logN);
 }
 
 void launch_bsgs_dot(Context* c, const BsgsJob& job, cudaStream_t s) {
@@ -755,16 +766,14 @@ void launch_bsgs_dot(Context* c, const BsgsJob& job, cudaStream_t s) {
   LaunchScope ls(c, s, KK_ELEM, 8.0 * c->N * job.l * (terms + job.lanes * 2.0 * (job.nb + job.ng)));
   if (job.nb <= 8 && aligned) {
     dim3 grid2(job.lanes * job.ng, c->N / (2 * EW_THREADS), job.l);
-    bsgs_dot2_kernel<<<grid2, EW_THREADS, 0, s>>>(job, c->d_prime, c->logN);
-    FIDES_CUDA(cudaGetLastError());
-    return;
+    launch_pdl(bsgs_dot2_kernel, grid2, EW_THREADS, 0, s, job, c->d_prime, c->logN);
+      return;
   }
   dim3 grid(job.lanes * job.ng, c->N / EW_THREADS, job.l);
   if (job.nb <= 8)
-    bsgs_dot_kernel<8><<<grid, EW_THREADS, 0, s>>>(job, c->d_prime, c->logN);
+    launch_pdl(bsgs_dot_kernel<8>, grid, EW_THREADS, 0, s, job, c->d_prime, c->logN);
   else
-    bsgs_dot_kernel<MAX_BSGS_BABY><<<grid, EW_THREADS, 0, s>>>(job, c->d_prime, c->logN);
-  FIDES_CUDA(cudaGetLastError());
+    launch_pdl(bsgs_dot_kernel<MAX_BSGS_BABY>, grid, EW_THREADS, 0, s, job, c->d_prime, c->logN);
 }
 
 void launch_lincomb(Context* c, const LinCombJob& job, cudaStream_t s) {
@@ -773,8 +782,7 @@ void launch_lincomb(Context* c, const LinCombJob& job, cudaStream_t s) {
     throw Error(-1, "linear combination needs 1..16 terms of 1..64 limbs in 1..8 lanes");
   dim3 grid(c->N / (2 * EW_THREADS), job.l, job.lanes);
   LaunchScope ls(c, s, KK_ELEM, 8.0 * c->N * job.l * job.lanes * (2.0 * job.n + 2));
-  lincomb_kernel<<<grid, EW_THREADS, 0, s>>>(job, c->d_prime, c->logN);
-  FIDES_CUDA(cudaGetLastError());
+  launch_pdl(lincomb_kernel, grid, EW_THREADS, 0, s, job, c->d_prime, c->logN);
 }
 
 void launch_ksk(Context* c, const KskJob* jobs, int n, cudaStream_t s) {
@@ -834,15 +842,33 @@ void launch_ksk(Context* c, const KskJob* jobs, int n, cudaStream_t s) {
                                           : 2.0 * b * ext);
     }
     LaunchScope ls(c, s, KK_KSK, bytes);
-    auto go = [&](auto kern) { kern<<<grid, EW_THREADS, 0, s>>>(L, c->d_prime, c->d_pmod, c->d_f64, c->logN, c->n_q,
-                                                              c->K, c->dnum, c->alpha); };
+    auto go_list = [&](auto kern, const auto& list) {
+      launch_pdl(kern, grid, EW_THREADS, 0, s, list, c->d_prime, c->d_pmod, c->d_f64, c->logN, c->n_q, c->K, c->dnum,
+                 c->alpha);
+    };
+    if (jg == 1 && m <= FEW_JOBS && maxb <= 4) {
+      static thread_local KskJobListT<FEW_JOBS> few;
+      few.n = m;
+      few.ngroups = L.ngroups;
+      std::copy(L.gstart, L.gstart + L.ngroups, few.gstart);
+      std::copy(L.gcount, L.gcount + L.ngroups, few.gcount);
+      std::copy(L.j, L.j + m, few.j);
+      switch (maxb) {
+        case 1: go_list(ksk_kernel<1, 1, 2, FEW_JOBS>, few); break;
+        case 2: go_list(ksk_kernel<2, 1, 2, FEW_JOBS>, few); break;
+        case 3: go_list(ksk_kernel<3, 1, 2, FEW_JOBS>, few); break;
+        default: go_list(ksk_kernel<4, 1, 2, FEW_JOBS>, few);
+      }
+      continue;
+    }
+    auto go = [&](auto kern) { go_list(kern, L); };
     switch (maxb * 16 + jg + (share_digits ? 128 : 0)) {
 #define FIDES_KSK_CASE(B, G)                    \
   case B * 16 + G:                              \
-    go(ksk_kernel<B, G, 2>);                    \
+    go(ksk_kernel<B, G, 2, MAX_KSK_JOBS>);                    \
     break;                                      \
   case 128 + B * 16 + G:                        \
-    go(ksk_kernel<B, G, 2, true>);              \
+    go(ksk_kernel<B, G, 2, MAX_KSK_JOBS, true>);              \
     break;
       FIDES_KSK_CASE(1, 1) FIDES_KSK_CASE(1, 2) FIDES_KSK_CASE(1, 4)
       FIDES_KSK_CASE(2, 1) FIDES_KSK_CASE(2, 2) FIDES_KSK_CASE(2, 4)
@@ -850,10 +876,9 @@ void launch_ksk(Context* c, const KskJob* jobs, int n, cudaStream_t s) {
       FIDES_KSK_CASE(4, 1) FIDES_KSK_CASE(4, 2) FIDES_KSK_CASE(4, 4)
 #undef FIDES_KSK_CASE
       default:
-        go(ksk_kernel<0, 1, 2>);
+        go(ksk_kernel<0, 1, 2, MAX_KSK_JOBS>);
     }
-    FIDES_CUDA(cudaGetLastError());
-  }
+    }
 }
 
 void launch_moddown_finish(Context* c, const FinJob* jobs, int n, cudaStream_t s) {
@@ -867,9 +892,8 @@ void launch_moddown_finish(Context* c, const FinJob* jobs, int n, cudaStream_t s
     double bytes = 0;
     for (int i = 0; i < m; ++i) bytes += 8.0 * c->N * ((L.j[i].add ? 4.0 : 3.0) * L.j[i].l);
     LaunchScope ls(c, s, KK_ELEM, bytes);
-    moddown_finish_kernel<<<grid, EW_THREADS, 0, s>>>(L, c->d_prime, c->d_pinv, c->logN);
-    FIDES_CUDA(cudaGetLastError());
-  }
+    launch_pdl(moddown_finish_kernel, grid, EW_THREADS, 0, s, L, c->d_prime, c->d_pinv, c->logN);
+    }
 }
 
 void launch_tensor(Context* c, const TensorJob* jobs, int n, cudaStream_t s) {
@@ -883,9 +907,8 @@ void launch_tensor(Context* c, const TensorJob* jobs, int n, cudaStream_t s) {
     double bytes = 0;
     for (int i = 0; i < m; ++i) bytes += 8.0 * c->N * ((L.j[i].d2 ? 7.0 : 6.0) * L.j[i].l);
     LaunchScope ls(c, s, KK_ELEM, bytes);
-    tensor_kernel<<<grid, EW_THREADS, 0, s>>>(L, c->d_prime, c->logN);
-    FIDES_CUDA(cudaGetLastError());
-  }
+    launch_pdl(tensor_kernel, grid, EW_THREADS, 0, s, L, c->d_prime, c->logN);
+    }
 }
 
 void launch_switch_modulus(Context* c, const SwitchJob* jobs, int n, cudaStream_t s) {
@@ -899,9 +922,8 @@ void launch_switch_modulus(Context* c, const SwitchJob* jobs, int n, cudaStream_
     double bytes = 0;
     for (int i = 0; i < m; ++i) bytes += 8.0 * c->N * (1.0 + (L.j[i].l - 1));
     LaunchScope ls(c, s, KK_ELEM, bytes);
-    switch_kernel<<<grid, EW_THREADS, 0, s>>>(L, c->d_prime, c->logN);
-    FIDES_CUDA(cudaGetLastError());
-  }
+    launch_pdl(switch_kernel, grid, EW_THREADS, 0, s, L, c->d_prime, c->logN);
+    }
 }
 
 void launch_rescale_finish(Context* c, const RescaleJob* jobs, int n, cudaStream_t s) {
@@ -915,9 +937,8 @@ void launch_rescale_finish(Context* c, const RescaleJob* jobs, int n, cudaStream
     double bytes = 0;
     for (int i = 0; i < m; ++i) bytes += 8.0 * c->N * (3.0 * (L.j[i].l - 1));
     LaunchScope ls(c, s, KK_ELEM, bytes);
-    rescale_finish_kernel<<<grid, EW_THREADS, 0, s>>>(L, c->d_prime, c->d_rescale, c->logN, c->n_q);
-    FIDES_CUDA(cudaGetLastError());
-  }
+    launch_pdl(rescale_finish_kernel, grid, EW_THREADS, 0, s, L, c->d_prime, c->d_rescale, c->logN, c->n_q);
+    }
 }
 
 void launch_addsub(Context* c, const AddSubJob* jobs, int n, cudaStream_t s) {
@@ -933,9 +954,8 @@ void launch_addsub(Context* c, const AddSubJob* jobs, int n, cudaStream_t s) {
     }
     dim3 grid(c->N / (2 * EW_THREADS), mx, m);
     LaunchScope ls(c, s, KK_ELEM, bytes);
-    addsub_kernel<<<grid, EW_THREADS, 0, s>>>(L, c->d_prime, c->logN);
-    FIDES_CUDA(cudaGetLastError());
-  }
+    launch_pdl(addsub_kernel, grid, EW_THREADS, 0, s, L, c->d_prime, c->logN);
+    }
 }
 
 void launch_scalar(Context* c, const ScalarJob* jobs, int n, cudaStream_t s) {
@@ -952,9 +972,8 @@ void launch_scalar(Context* c, const ScalarJob* jobs, int n, cudaStream_t s) {
     }
     dim3 grid(c->N / (2 * EW_THREADS), mx, m);
     LaunchScope ls(c, s, KK_ELEM, bytes);
-    scalar_kernel<<<grid, EW_THREADS, 0, s>>>(L, c->d_prime, c->logN);
-    FIDES_CUDA(cudaGetLastError());
-  }
+    launch_pdl(scalar_kernel, grid, EW_THREADS, 0, s, L, c->d_prime, c->logN);
+    }
 }
 
 }  // namespace fides

@@ -22,10 +22,16 @@ struct ConvJob {
   uint64_t* dst;        // output j at dst + t.dst_pos[j] * N
 };
 constexpr int MAX_CONV_JOBS = 96;
-struct ConvJobList {
+// Job lists are passed by value; launches of a few jobs take the short form (a large parameter block
+// costs the host up to 3 us a launch).
+template <int CAP>
+struct ConvJobListT {
+  static constexpr int cap = CAP;
   int n, max_src, max_dst, pad;
-  ConvJob j[MAX_CONV_JOBS];
+  ConvJob j[CAP];
 };
+using ConvJobList = ConvJobListT<MAX_CONV_JOBS>;
+constexpr int FEW_JOBS = 8;
 void launch_conv(Context* c, const ConvJob* jobs, int n, cudaStream_t s);
 
 // ---- KSK inner product (fusedDotKSK_2_, ElemenwiseBatchKernels.cu:202-274) with the
@@ -56,11 +62,13 @@ constexpr int MAX_KSK_JOBS = 64;
 // tile once for all of its jobs.  (Groups of 8 read the key half as often but measured 20 %
 // slower on the bench step: half as many CTAs, each running twice as long, and more spills.)
 constexpr int MAX_KSK_GROUP = 4;
-struct KskJobList {
+template <int CAP>
+struct KskJobListT {
   int n, max_ext, ngroups, pad1;
-  uint8_t gstart[MAX_KSK_JOBS], gcount[MAX_KSK_JOBS];
-  KskJob j[MAX_KSK_JOBS];
+  uint8_t gstart[CAP], gcount[CAP];
+  KskJob j[CAP];
 };
+using KskJobList = KskJobListT<MAX_KSK_JOBS>;
 void launch_ksk(Context* c, const KskJob* jobs, int n, cudaStream_t s);
 
 // ---- ModDown epilogue (NTT_MODDOWN, NTTfusions.cuh:237-252): out = (x - conv) P^-1 (+ add)

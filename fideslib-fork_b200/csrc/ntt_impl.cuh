@@ -4,6 +4,7 @@
 #include <algorithm>
 
 #include "f64arith.cuh"
+#include "launch.cuh"
 #include "ntt.cuh"
 
 namespace fides {
@@ -493,6 +494,7 @@ __global__ void __launch_bounds__(PassThreads<LOGN, PASS, G, LE>::NT, PassThread
   // stalls 10x a plain pass's)
   constexpr bool STAGE_PRO = first_pass && IN == IN_CONV_SW;
   static_assert(!STAGE_PRO || PASS == COL, "the conv-switch prologue is a column-pass prologue");
+  pdl_wait();  // nothing before this reads or writes limbs
   if constexpr (STAGE_PRO) {
 #pragma unroll
     for (int k = 0; k < G * P / 2 / NT; ++k) {
@@ -712,8 +714,7 @@ void launch_pass_g(Context* c, const PassArgs& a, const NttLimbList& L, cudaStre
   dim3 grid(((1 << LOGN) >> LOGP) / G, L.n);
   // algorithmic bytes: half of a transform's read + write of each limb (two passes)
   LaunchScope ls(c, s, KK_NTT, 8.0 * (1 << LOGN) * L.n);
-  ntt_pass<LOGN, PASS, FWD, IN, OUT, G, LE><<<grid, T * G, smem, s>>>(a, L);
-  FIDES_CUDA(cudaGetLastError());
+  launch_pdl(ntt_pass<LOGN, PASS, FWD, IN, OUT, G, LE>, grid, T * G, smem, s, a, L);
 }
 
 // The pass with the sub-transforms-per-CTA and residues per thread the context's tables pick
