@@ -33,22 +33,42 @@ __device__ __forceinline__ uint64_t f_canon(double s, double q, double qinv) {
   return (uint64_t)__double_as_longlong(__dadd_rn(r, F64_TWO52)) & ((1ull << 52) - 1);
 }
 
-// An inner product sum a_i b_i of residues, exact, reduced once.  h starts at 1.25 2^103 and takes
-// the products by fma, which rounds to its ulp of 2^51 while the sum stays in [-2, 6) 2^100; the
-// part of a product that h did not take, at most 2^50 in magnitude, is found exactly and summed in
-// l, exact for at most 7 terms.  Four operations a term, against seven for a reduced product each.
-struct F64Acc {
-  double h = F64ACC_H0, l = 0.0;
-  static constexpr double F64ACC_H0 = 12676506002282294014967032053760.0;  // 1.25 * 2^103
+// An inner product sum a_i b_i of residues, exact, reduced once.  h starts at h0 and takes the
+// products by fma, which rounds to its ulp of 2^51 while it stays in [2^103, 2^104); the part of a
+// product that h did not take, at most 2^50 in magnitude, is found exactly and summed in l, exact up
+// to 2^53.  Four operations a term, against seven for a reduced product each.
+// F64Acc: h0 = 1.25 2^103, sums in [-2, 6) 2^100 of at most 7 terms.  F64AccPos: h0 = 2^103, at most 8
+// terms of products of two residues.
+template <bool POS>
+struct F64AccT {
+  static constexpr double H0 = POS ? 0x1p103 : 0x1.4p103;
+  double h = H0, l = 0.0;
   __device__ __forceinline__ void mac(double a, double b) {
     const double n = __fma_rn(a, b, h);
     l = __dadd_rn(l, __fma_rn(a, b, -__dadd_rn(n, -h)));
     h = n;
   }
-  // An integer below 2^53 in magnitude that is congruent to the sum: (h - h0) 2^-51, below 3 2^50 in
-  // magnitude, times 2^51 mod q (w51, centred), plus l.
+  // An integer below 2^53 in magnitude that is congruent to the sum: (h - h0) 2^-51, below 2^52 in
+  // magnitude, times 2^51 mod q (w51, centred), plus l (POS: plus its residue, so within 2q).
   __device__ __forceinline__ double fold(double w51, double q, double qinv) const {
-    return __dadd_rn(f_mulmod(__dmul_rn(__dadd_rn(h, -F64ACC_H0), 0x1p-51), w51, q, qinv), l);
+    const double r = f_mulmod(__dmul_rn(__dadd_rn(h, -H0), 0x1p-51), w51, q, qinv);
+    return __dadd_rn(r, POS ? f_reduce(l, q, qinv) : l);
+  }
+};
+using F64Acc = F64AccT<false>;
+using F64AccPos = F64AccT<true>;
+
+// A sum of any number of products of two residues: folded after every eight.
+struct F64Sum {
+  F64AccPos acc;
+  double done = 0.0;  // within q for each eight terms folded
+  __device__ __forceinline__ void mac(double a, double b) { acc.mac(a, b); }
+  __device__ __forceinline__ void flush(double w51, double q, double qinv) {
+    done = __dadd_rn(done, f_reduce(acc.fold(w51, q, qinv), q, qinv));
+    acc = F64AccPos{};
+  }
+  __device__ __forceinline__ uint64_t residue(double w51, double q, double qinv) const {
+    return f_canon(__dadd_rn(done, acc.fold(w51, q, qinv)), q, qinv);
   }
 };
 

@@ -518,21 +518,15 @@ __global__ void __launch_bounds__(EW_THREADS) scalar_kernel(const __grid_constan
 constexpr int LC_BLOCK = 4;  // terms per block of loads (lincomb_kernel, dot_plain_kernel)
 
 __global__ void __launch_bounds__(EW_THREADS) dot_plain_kernel(const __grid_constant__ DotJob J,
-                                                               const DevPrime* primes, int logN) {
+                                                               const DevPrime* primes, const F64Prime* f64, int logN) {
   const int lane = blockIdx.x, j = blockIdx.z;
-  const DevPrime p = primes[ext_prime(j, J.lq, J.nq)];
+  const int pid = ext_prime(j, J.lq, J.nq);
+  const DevPrime p = primes[pid];
   const size_t off = ((size_t)j << logN) + 2 * (blockIdx.y * blockDim.x + threadIdx.x);
   pdl_wait();
   auto ld2 = [](const uint64_t* q) { return *reinterpret_cast<const ulonglong2*>(q); };
-  U128 a0{0, 0}, a1{0, 0}, b0{0, 0}, b1{0, 0};
-  for (int t0 = 0; t0 < J.n; t0 += LC_BLOCK) {  // as lincomb_kernel
-    if (t0 && t0 % 12 == 0) {
-      a0 = U128{reduce128(a0, p), 0};
-      a1 = U128{reduce128(a1, p), 0};
-      b0 = U128{reduce128(b0, p), 0};
-      b1 = U128{reduce128(b1, p), 0};
-    }
-    ulonglong2 w[LC_BLOCK], x[LC_BLOCK], y[LC_BLOCK];
+  ulonglong2 w[LC_BLOCK], x[LC_BLOCK], y[LC_BLOCK];
+  auto load = [&](int t0) {  // as lincomb_kernel
 #pragma unroll
     for (int u = 0; u < LC_BLOCK; ++u)
       if (t0 + u < J.n) {
@@ -540,17 +534,52 @@ __global__ void __launch_bounds__(EW_THREADS) dot_plain_kernel(const __grid_cons
         x[u] = ld2(J.c0[lane][t0 + u] + off);
         y[u] = ld2(J.c1[lane][t0 + u] + off);
       }
+  };
+  ulonglong2 r0, r1;
+  if (p.q < NTT_F64_MAX) {
+    const F64Prime fp = f64[pid];
+    F64Sum a0, a1, b0, b1;
+    for (int t0 = 0; t0 < J.n; t0 += LC_BLOCK) {
+      if (t0 && t0 % 8 == 0)
+        a0.flush(fp.w51, fp.q, fp.qinv), a1.flush(fp.w51, fp.q, fp.qinv), b0.flush(fp.w51, fp.q, fp.qinv),
+            b1.flush(fp.w51, fp.q, fp.qinv);
+      load(t0);
 #pragma unroll
-    for (int u = 0; u < LC_BLOCK; ++u)
-      if (t0 + u < J.n) {
-        mac128(a0, w[u].x, x[u].x);
-        mac128(a1, w[u].y, x[u].y);
-        mac128(b0, w[u].x, y[u].x);
-        mac128(b1, w[u].y, y[u].y);
+      for (int u = 0; u < LC_BLOCK; ++u)
+        if (t0 + u < J.n) {
+          const double w0 = f_from_u64(w[u].x), w1 = f_from_u64(w[u].y);
+          a0.mac(w0, f_from_u64(x[u].x));
+          a1.mac(w1, f_from_u64(x[u].y));
+          b0.mac(w0, f_from_u64(y[u].x));
+          b1.mac(w1, f_from_u64(y[u].y));
+        }
+    }
+    r0 = make_ulonglong2(a0.residue(fp.w51, fp.q, fp.qinv), a1.residue(fp.w51, fp.q, fp.qinv));
+    r1 = make_ulonglong2(b0.residue(fp.w51, fp.q, fp.qinv), b1.residue(fp.w51, fp.q, fp.qinv));
+  } else {
+    U128 a0{0, 0}, a1{0, 0}, b0{0, 0}, b1{0, 0};
+    for (int t0 = 0; t0 < J.n; t0 += LC_BLOCK) {
+      if (t0 && t0 % 12 == 0) {
+        a0 = U128{reduce128(a0, p), 0};
+        a1 = U128{reduce128(a1, p), 0};
+        b0 = U128{reduce128(b0, p), 0};
+        b1 = U128{reduce128(b1, p), 0};
       }
+      load(t0);
+#pragma unroll
+      for (int u = 0; u < LC_BLOCK; ++u)
+        if (t0 + u < J.n) {
+          mac128(a0, w[u].x, x[u].x);
+          mac128(a1, w[u].y, x[u].y);
+          mac128(b0, w[u].x, y[u].x);
+          mac128(b1, w[u].y, y[u].y);
+        }
+    }
+    r0 = make_ulonglong2(reduce128(a0, p), reduce128(a1, p));
+    r1 = make_ulonglong2(reduce128(b0, p), reduce128(b1, p));
   }
-  *reinterpret_cast<ulonglong2*>(J.out0[lane] + off) = make_ulonglong2(reduce128(a0, p), reduce128(a1, p));
-  *reinterpret_cast<ulonglong2*>(J.out1[lane] + off) = make_ulonglong2(reduce128(b0, p), reduce128(b1, p));
+  *reinterpret_cast<ulonglong2*>(J.out0[lane] + off) = r0;
+  *reinterpret_cast<ulonglong2*>(J.out1[lane] + off) = r1;
 }
 
 // One CTA per (giant step, lane, coefficient tile, limb): a thread loads its coefficient of the
@@ -562,9 +591,10 @@ __global__ void __launch_bounds__(EW_THREADS) dot_plain_kernel(const __grid_cons
 // NB: register capacity for the baby steps.
 template <int NB>
 __global__ void __launch_bounds__(EW_THREADS) bsgs_dot_kernel(const __grid_constant__ BsgsJob J,
-                                                              const DevPrime* primes, int logN) {
+                                                              const DevPrime* primes, const F64Prime* f64, int logN) {
   const int i = blockIdx.x % J.ng, lane = blockIdx.x / J.ng, j = blockIdx.z;
-  const DevPrime p = primes[ext_prime(j, J.lq, J.nq)];
+  const int pid = ext_prime(j, J.lq, J.nq);
+  const DevPrime p = primes[pid];
   const size_t off = ((size_t)j << logN) + blockIdx.y * blockDim.x + threadIdx.x;
   pdl_wait();
   uint64_t a[NB], b[NB], w[NB];
@@ -575,6 +605,25 @@ __global__ void __launch_bounds__(EW_THREADS) bsgs_dot_kernel(const __grid_const
       a[k] = J.x0[lane][k][off];
       b[k] = J.x1[lane][k][off];
     }
+  if (p.q < NTT_F64_MAX) {
+    const F64Prime fp = f64[pid];
+    F64Sum s0, s1;
+#pragma unroll
+    for (int k = 0; k < NB; ++k) {
+      if (k == 8) {
+        s0.flush(fp.w51, fp.q, fp.qinv);
+        s1.flush(fp.w51, fp.q, fp.qinv);
+      }
+      if (k < J.nb && J.pt[i][k]) {
+        const double d = f_from_u64(w[k]);
+        s0.mac(d, f_from_u64(a[k]));
+        s1.mac(d, f_from_u64(b[k]));
+      }
+    }
+    J.out0[lane][i][off] = s0.residue(fp.w51, fp.q, fp.qinv);
+    J.out1[lane][i][off] = s1.residue(fp.w51, fp.q, fp.qinv);
+    return;
+  }
   U128 s0{0, 0}, s1{0, 0};
 #pragma unroll
   for (int k = 0; k < NB; ++k) {
@@ -594,11 +643,15 @@ __global__ void __launch_bounds__(EW_THREADS) bsgs_dot_kernel(const __grid_const
 // bsgs_dot_kernel with two consecutive coefficients per thread (16-byte loads and stores), for
 // at most 8 baby steps (the products stay below 2^128 without an intermediate reduction) and
 // operands whose addresses are 16-byte aligned (checked by the launcher).
+// Primes below 2^50 sum in FP64 (F64AccPos): 8 baby and 8 giant steps on 30 limbs at N = 2^16 take 331 us
+// (1.51 GB), the six transforms of a bootstrap 1360 us against 1770 with 128-bit integer sums.  One CTA
+// walking the giant steps with the baby steps in registers took 549 us there.
 __global__ void __launch_bounds__(EW_THREADS) bsgs_dot2_kernel(const __grid_constant__ BsgsJob J,
-                                                               const DevPrime* primes, int logN) {
+                                                               const DevPrime* primes, const F64Prime* f64, int logN) {
   constexpr int NB = 8;
   const int i = blockIdx.x % J.ng, lane = blockIdx.x / J.ng, j = blockIdx.z;
-  const DevPrime p = primes[ext_prime(j, J.lq, J.nq)];
+  const int pid = ext_prime(j, J.lq, J.nq);
+  const DevPrime p = primes[pid];
   const size_t off = ((size_t)j << logN) + 2 * ((size_t)blockIdx.y * blockDim.x + threadIdx.x);
   pdl_wait();
   auto ld2 = [](const uint64_t* q) { return *reinterpret_cast<const ulonglong2*>(q); };
@@ -610,6 +663,23 @@ __global__ void __launch_bounds__(EW_THREADS) bsgs_dot2_kernel(const __grid_cons
       a[k] = ld2(J.x0[lane][k] + off);
       b[k] = ld2(J.x1[lane][k] + off);
     }
+  if (p.q < NTT_F64_MAX) {
+    const F64Prime fp = f64[pid];
+    F64AccPos t0x, t0y, t1x, t1y;
+#pragma unroll
+    for (int k = 0; k < NB; ++k)
+      if (k < J.nb && J.pt[i][k]) {
+        const double wx = f_from_u64(w[k].x), wy = f_from_u64(w[k].y);
+        t0x.mac(wx, f_from_u64(a[k].x));
+        t0y.mac(wy, f_from_u64(a[k].y));
+        t1x.mac(wx, f_from_u64(b[k].x));
+        t1y.mac(wy, f_from_u64(b[k].y));
+      }
+    auto res = [&](const F64AccPos& t) { return f_canon(t.fold(fp.w51, fp.q, fp.qinv), fp.q, fp.qinv); };
+    *reinterpret_cast<ulonglong2*>(J.out0[lane][i] + off) = ulonglong2{res(t0x), res(t0y)};
+    *reinterpret_cast<ulonglong2*>(J.out1[lane][i] + off) = ulonglong2{res(t1x), res(t1y)};
+    return;
+  }
   U128 s0x{0, 0}, s0y{0, 0}, s1x{0, 0}, s1y{0, 0};
 #pragma unroll
   for (int k = 0; k < NB; ++k)
@@ -624,44 +694,73 @@ __global__ void __launch_bounds__(EW_THREADS) bsgs_dot2_kernel(const __grid_cons
 }
 
 __global__ void __launch_bounds__(EW_THREADS) lincomb_kernel(const __grid_constant__ LinCombJob J,
-                                                             const DevPrime* primes, int logN) {
+                                                             const DevPrime* primes, const F64Prime* f64, int logN) {
   const int j = blockIdx.y, lane = blockIdx.z;
-  const DevPrime p = primes[ext_prime(j, J.lq, J.nq)];
+  const int pid = ext_prime(j, J.lq, J.nq);
+  const DevPrime p = primes[pid];
   const size_t off = ((size_t)j << logN) + 2 * (blockIdx.x * blockDim.x + threadIdx.x);
   pdl_wait();
   auto ld2 = [](const uint64_t* q) { return *reinterpret_cast<const ulonglong2*>(q); };
-  U128 a0{0, 0}, a1{0, 0}, b0{0, 0}, b1{0, 0};
   // terms in blocks of LC_BLOCK whose loads are all issued before their products, so that a
-  // thread waits for memory once per block rather than once per term; the sums are reduced
-  // every 12 terms (below 2^128: a residue plus 12 products of values below 2^62)
-  for (int t0 = 0; t0 < J.n; t0 += LC_BLOCK) {
-    if (t0 && t0 % 12 == 0) {
-      a0 = U128{reduce128(a0, p), 0};
-      a1 = U128{reduce128(a1, p), 0};
-      b0 = U128{reduce128(b0, p), 0};
-      b1 = U128{reduce128(b1, p), 0};
-    }
-    ulonglong2 x[LC_BLOCK], y[LC_BLOCK];
+  // thread waits for memory once per block rather than once per term; the 128-bit sums are reduced
+  // every 12 terms (below 2^128: a residue plus 12 products of values below 2^62), the FP64 ones every 8
+  ulonglong2 x[LC_BLOCK], y[LC_BLOCK];
+  auto load = [&](int t0) {
 #pragma unroll
     for (int u = 0; u < LC_BLOCK; ++u)
       if (t0 + u < J.n) {
         x[u] = ld2(J.x0[lane][t0 + u] + off);
         y[u] = ld2(J.x1[lane][t0 + u] + off);
       }
+  };
+  ulonglong2 r0, r1;
+  if (p.q < NTT_F64_MAX) {
+    const F64Prime fp = f64[pid];
+    F64Sum a0, a1, b0, b1;
+    for (int t0 = 0; t0 < J.n; t0 += LC_BLOCK) {
+      if (t0 && t0 % 8 == 0)
+        a0.flush(fp.w51, fp.q, fp.qinv), a1.flush(fp.w51, fp.q, fp.qinv), b0.flush(fp.w51, fp.q, fp.qinv),
+            b1.flush(fp.w51, fp.q, fp.qinv);
+      load(t0);
 #pragma unroll
-    for (int u = 0; u < LC_BLOCK; ++u)
-      if (t0 + u < J.n) {
-        const uint64_t w = J.s[t0 + u][j];
-        mac128(a0, w, x[u].x);
-        mac128(a1, w, x[u].y);
-        mac128(b0, w, y[u].x);
-        mac128(b1, w, y[u].y);
+      for (int u = 0; u < LC_BLOCK; ++u)
+        if (t0 + u < J.n) {
+          const double w = f_from_u64(J.s[t0 + u][j]);
+          a0.mac(w, f_from_u64(x[u].x));
+          a1.mac(w, f_from_u64(x[u].y));
+          b0.mac(w, f_from_u64(y[u].x));
+          b1.mac(w, f_from_u64(y[u].y));
+        }
+    }
+    r0 = make_ulonglong2(a0.residue(fp.w51, fp.q, fp.qinv), a1.residue(fp.w51, fp.q, fp.qinv));
+    r1 = make_ulonglong2(b0.residue(fp.w51, fp.q, fp.qinv), b1.residue(fp.w51, fp.q, fp.qinv));
+  } else {
+    U128 a0{0, 0}, a1{0, 0}, b0{0, 0}, b1{0, 0};
+    for (int t0 = 0; t0 < J.n; t0 += LC_BLOCK) {
+      if (t0 && t0 % 12 == 0) {
+        a0 = U128{reduce128(a0, p), 0};
+        a1 = U128{reduce128(a1, p), 0};
+        b0 = U128{reduce128(b0, p), 0};
+        b1 = U128{reduce128(b1, p), 0};
       }
+      load(t0);
+#pragma unroll
+      for (int u = 0; u < LC_BLOCK; ++u)
+        if (t0 + u < J.n) {
+          const uint64_t w = J.s[t0 + u][j];
+          mac128(a0, w, x[u].x);
+          mac128(a1, w, x[u].y);
+          mac128(b0, w, y[u].x);
+          mac128(b1, w, y[u].y);
+        }
+    }
+    r0 = make_ulonglong2(reduce128(a0, p), reduce128(a1, p));
+    r1 = make_ulonglong2(reduce128(b0, p), reduce128(b1, p));
   }
   const uint64_t ad = J.add0[j];
   *reinterpret_cast<ulonglong2*>(J.out0[lane] + off) =
-      make_ulonglong2(addmod(reduce128(a0, p), ad, p.q), addmod(reduce128(a1, p), ad, p.q));
-  *reinterpret_cast<ulonglong2*>(J.out1[lane] + off) = make_ulonglong2(reduce128(b0, p), reduce128(b1, p));
+      make_ulonglong2(addmod(r0.x, ad, p.q), addmod(r0.y, ad, p.q));
+  *reinterpret_cast<ulonglong2*>(J.out1[lane] + off) = r1;
 }
 
 template <typename List, typename Job>
@@ -744,7 +843,7 @@ void launch_dot_plain(Context* c, const DotJob& job, cudaStream_t s) {
   if (job.lanes < 1 || job.lanes > MAX_DOT_LANES) throw Error(-1, "dot product needs 1..8 lanes");
   dim3 grid(job.lanes, c->N / (2 * EW_THREADS), job.l);
   LaunchScope ls(c, s, KK_ELEM, 8.0 * c->N * job.l * (job.n + job.lanes * (2.0 * job.n + 2)));
-  launch_pdl(dot_plain_kernel, grid, EW_THREADS, 0, s, job, c->d_prime, c->logN);
+  launch_pdl(dot_plain_kernel, grid, EW_THREADS, 0, s, job, c->d_prime, c->d_f64, c->logN);
 }
 
 void launch_bsgs_dot(Context* c, const BsgsJob& job, cudaStream_t s) {
@@ -766,14 +865,14 @@ void launch_bsgs_dot(Context* c, const BsgsJob& job, cudaStream_t s) {
   LaunchScope ls(c, s, KK_ELEM, 8.0 * c->N * job.l * (terms + job.lanes * 2.0 * (job.nb + job.ng)));
   if (job.nb <= 8 && aligned) {
     dim3 grid2(job.lanes * job.ng, c->N / (2 * EW_THREADS), job.l);
-    launch_pdl(bsgs_dot2_kernel, grid2, EW_THREADS, 0, s, job, c->d_prime, c->logN);
-      return;
+    launch_pdl(bsgs_dot2_kernel, grid2, EW_THREADS, 0, s, job, c->d_prime, c->d_f64, c->logN);
+    return;
   }
   dim3 grid(job.lanes * job.ng, c->N / EW_THREADS, job.l);
   if (job.nb <= 8)
-    launch_pdl(bsgs_dot_kernel<8>, grid, EW_THREADS, 0, s, job, c->d_prime, c->logN);
+    launch_pdl(bsgs_dot_kernel<8>, grid, EW_THREADS, 0, s, job, c->d_prime, c->d_f64, c->logN);
   else
-    launch_pdl(bsgs_dot_kernel<MAX_BSGS_BABY>, grid, EW_THREADS, 0, s, job, c->d_prime, c->logN);
+    launch_pdl(bsgs_dot_kernel<MAX_BSGS_BABY>, grid, EW_THREADS, 0, s, job, c->d_prime, c->d_f64, c->logN);
 }
 
 void launch_lincomb(Context* c, const LinCombJob& job, cudaStream_t s) {
@@ -782,7 +881,7 @@ void launch_lincomb(Context* c, const LinCombJob& job, cudaStream_t s) {
     throw Error(-1, "linear combination needs 1..16 terms of 1..64 limbs in 1..8 lanes");
   dim3 grid(c->N / (2 * EW_THREADS), job.l, job.lanes);
   LaunchScope ls(c, s, KK_ELEM, 8.0 * c->N * job.l * job.lanes * (2.0 * job.n + 2));
-  launch_pdl(lincomb_kernel, grid, EW_THREADS, 0, s, job, c->d_prime, c->logN);
+  launch_pdl(lincomb_kernel, grid, EW_THREADS, 0, s, job, c->d_prime, c->d_f64, c->logN);
 }
 
 void launch_ksk(Context* c, const KskJob* jobs, int n, cudaStream_t s) {
