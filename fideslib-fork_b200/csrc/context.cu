@@ -77,6 +77,11 @@ uint32_t h_auto_index(int logN, int rotation) {
   return (uint32_t)h_powmod(5, (uint64_t)(2 * N - r), (uint64_t)(2 * N));
 }
 
+static double h_centred(uint64_t w, uint64_t q) { return w > q / 2 ? -(double)(q - w) : (double)w; }
+static InvFinal inv_final(uint64_t sum, uint64_t diff, uint64_t q) {
+  return InvFinal{h_shoup(sum, q), h_shoup(diff, q), h_centred(sum, q), h_centred(diff, q)};
+}
+
 static bool h_is_prime(uint64_t n) {
   static const uint64_t b[] = {2, 3, 5, 7, 11, 13, 17, 19, 23, 29, 31, 37};
   if (n < 2) return false;
@@ -216,7 +221,7 @@ Context* create_context(int logN, int n_q, int K, int dnum, const uint64_t* prim
     FIDES_CUDA(cudaSetDevice(device));
     // ---- per-prime constants and twiddles
     std::vector<DevPrime> hp(np);
-    std::vector<ShoupConst> il(np);
+    std::vector<InvFinal> fin(np);
     std::vector<F64Prime> f64(np);
     // NTT twiddles (the transforms start at N = 2^10): 8-byte entries where the FP64 butterflies
     // run, 16-byte ones elsewhere
@@ -232,8 +237,7 @@ Context* create_context(int logN, int n_q, int K, int dnum, const uint64_t* prim
       d.one_s = (uint64_t)(((u128)1 << 64) / q);
       d.r64 = (uint64_t)(((u128)1 << 64) % q);
       d.r64_s = h_shoup(d.r64, q).ws;
-      d.ninv = h_invmod(N % q, q);
-      d.ninv_s = h_shoup(d.ninv, q).ws;
+      const uint64_t ninv = h_invmod(N % q, q);
       d.tw = tw_at[i];
       std::vector<uint64_t> pw(N), ipw(N);
       uint64_t ip = h_invmod(c->psi[i], q);
@@ -242,12 +246,12 @@ Context* create_context(int logN, int n_q, int K, int dnum, const uint64_t* prim
         pw[j] = h_mulmod(pw[j - 1], c->psi[i], q);
         ipw[j] = h_mulmod(ipw[j - 1], ip, q);
       }
-      il[i] = h_shoup(h_mulmod(ipw[h_brev(1, logN)], d.ninv, q), q);
       const double qd = (double)q;  // exact for q < 2^53; used only for q < 2^50
-      auto centred = [&](uint64_t w) { return w > q / 2 ? -(double)(q - w) : (double)w; };
+      auto centred = [&](uint64_t w) { return h_centred(w, q); };
+      fin[i] = inv_final(ninv, h_mulmod(ipw[h_brev(1, logN)], ninv, q), q);
       uint64_t pmq = i < n_q ? 1 % q : 0;  // P mod q
       for (int k = 0; k < K; ++k) pmq = h_mulmod(pmq, primes[n_q + k] % q, q);
-      f64[i] = F64Prime{qd, 1.0 / qd, centred(d.ninv), centred(il[i].w), centred((1ull << 51) % q), centred(pmq)};
+      f64[i] = F64Prime{qd, 1.0 / qd, centred((1ull << 51) % q), centred(pmq)};
       if (logN < 10) return;
       // the twiddle tables (layout in ntt.cuh); the twiddle of global stage s, block m is the
       // (2^s + m)-th power in bit-reversed order
@@ -319,19 +323,17 @@ Context* create_context(int logN, int n_q, int K, int dnum, const uint64_t* prim
     }
     // ---- conversion tables
     struct HostConv {
-      std::vector<int> src_pos, src_prime, dst_pos, dst_prime;
-      std::vector<ShoupConst> pre;
+      std::vector<int> src_prime, dst_prime;
+      int src0 = 0, dst_skip = 0, dst_gap = 0;
+      std::vector<uint64_t> pre;  // (Q_src / q_i)^-1 mod q_i
       std::vector<uint64_t> mat;
       std::vector<uint8_t> tc_b;  // empty: no tensor-core form
       std::vector<TcDest> tc_dst;
       int kpad = 0, ndp = 0, lift = 0;
     };
-    auto build_conv = [&](const std::vector<int>& sp, const std::vector<int>& spr, const std::vector<int>& dp,
-                          const std::vector<int>& dpr, int lift) {
+    auto build_conv = [&](const std::vector<int>& spr, const std::vector<int>& dpr, int lift) {
       HostConv h;
-      h.src_pos = sp;
       h.src_prime = spr;
-      h.dst_pos = dp;
       h.dst_prime = dpr;
       h.lift = lift;
       int ns = (int)spr.size(), nd = (int)dpr.size();
@@ -346,7 +348,7 @@ Context* create_context(int logN, int n_q, int K, int dnum, const uint64_t* prim
         uint64_t qi = primes[spr[i]], hq = 1;
         for (int k = 0; k < ns; ++k)
           if (k != i) hq = h_mulmod(hq, primes[spr[k]] % qi, qi);
-        h.pre[i] = h_shoup(h_invmod(hq, qi), qi);
+        h.pre[i] = h_invmod(hq, qi);
         for (int j = 0; j < nd; ++j) {
           uint64_t pj = primes[dpr[j]], v = 1 % pj;
           for (int k = 0; k < ns; ++k)
@@ -367,41 +369,56 @@ Context* create_context(int logN, int n_q, int K, int dnum, const uint64_t* prim
         int b = c->beta(l);
         for (int d = 0; d < b; ++d) {
           int s0 = d * c->alpha, s1 = std::min((d + 1) * c->alpha, l);
-          std::vector<int> sp, spr, dp, dpr;
-          for (int i = s0; i < s1; ++i) sp.push_back(i), spr.push_back(i);
+          std::vector<int> spr, dpr;
+          for (int i = s0; i < s1; ++i) spr.push_back(i);
           for (int i = 0; i < l; ++i)
-            if (i < s0 || i >= s1) dp.push_back(i), dpr.push_back(i);
-          for (int k = 0; k < K; ++k) dp.push_back(l + k), dpr.push_back(n_q + k);
-          hmu[lift][l].push_back(build_conv(sp, spr, dp, dpr, lift));
+            if (i < s0 || i >= s1) dpr.push_back(i);
+          for (int k = 0; k < K; ++k) dpr.push_back(n_q + k);
+          hmu[lift][l].push_back(build_conv(spr, dpr, lift));
+          HostConv& h = hmu[lift][l].back();
+          h.src0 = h.dst_skip = s0;
+          h.dst_gap = s1 - s0;
         }
         if (K > 0) {
-          std::vector<int> sp, spr, dp, dpr;
-          for (int k = 0; k < K; ++k) sp.push_back(k), spr.push_back(n_q + k);
-          for (int j = 0; j < l; ++j) dp.push_back(j), dpr.push_back(j);
-          hmd[lift][l] = build_conv(sp, spr, dp, dpr, lift);
+          std::vector<int> spr, dpr;
+          for (int k = 0; k < K; ++k) spr.push_back(n_q + k);
+          for (int j = 0; j < l; ++j) dpr.push_back(j);
+          hmd[lift][l] = build_conv(spr, dpr, lift);
         }
       }
+    // ---- the sources' factors, folded into the inverse transforms that precede the conversions
+    auto scaled = [&](int prime, uint64_t pre) {
+      const uint64_t q = primes[prime];
+      return inv_final(h_mulmod(fin[prime].sum.w, pre, q), h_mulmod(fin[prime].diff.w, pre, q), q);
+    };
+    std::vector<std::vector<InvFinal>> fin_up(n_q + 1);
+    for (int l = 1; l <= n_q; ++l)
+      for (const HostConv& h : hmu[0][l])
+        for (size_t i = 0; i < h.pre.size(); ++i) fin_up[l].push_back(scaled(h.src_prime[i], h.pre[i]));
+    std::vector<InvFinal> fin_down;
+    if (K > 0)
+      for (int k = 0; k < K; ++k) fin_down.push_back(scaled(n_q + k, hmd[0][1].pre[k]));
     // ---- pack everything into one device blob
     std::vector<char> blob;
-    size_t o_prime, o_tw, o_il, o_pinv, o_pmod, o_rs, o_pq, o_f64;
+    size_t o_prime, o_tw, o_fin, o_fin_down, o_pinv, o_pmod, o_rs, o_pq, o_f64;
     append(blob, hp, o_prime);
     append(blob, twid, o_tw);
-    append(blob, il, o_il);
+    append(blob, fin, o_fin);
+    append(blob, fin_down, o_fin_down);
+    std::vector<size_t> o_fin_up(n_q + 1, 0);
+    for (int l = 1; l <= n_q; ++l) append(blob, fin_up[l], o_fin_up[l]);
     append(blob, pinv, o_pinv);
     append(blob, pmod, o_pmod);
     append(blob, rs, o_rs);
     append(blob, pqinv, o_pq);
     append(blob, f64, o_f64);
     struct Off {
-      size_t sp, spr, pre, dp, dpr, mat, tcb, tcd;
-      int ns, nd, kpad, ndp, lift;
+      size_t spr, dpr, mat, tcb, tcd;
+      int ns, nd, kpad, ndp, lift, src0, dst_skip, dst_gap;
     };
     auto put = [&](const HostConv& h) {
       Off o;
-      append(blob, h.src_pos, o.sp);
       append(blob, h.src_prime, o.spr);
-      append(blob, h.pre, o.pre);
-      append(blob, h.dst_pos, o.dp);
       append(blob, h.dst_prime, o.dpr);
       append(blob, h.mat, o.mat);
       append(blob, h.tc_b, o.tcb);
@@ -411,6 +428,9 @@ Context* create_context(int logN, int n_q, int K, int dnum, const uint64_t* prim
       o.kpad = h.tc_b.empty() ? 0 : h.kpad;
       o.ndp = h.ndp;
       o.lift = h.lift;
+      o.src0 = h.src0;
+      o.dst_skip = h.dst_skip;
+      o.dst_gap = h.dst_gap;
       return o;
     };
     std::vector<std::vector<Off>> omu[2] = {std::vector<std::vector<Off>>(n_q + 1),
@@ -426,7 +446,10 @@ Context* create_context(int logN, int n_q, int K, int dnum, const uint64_t* prim
     char* base = static_cast<char*>(c->d_tables);
     c->d_prime = reinterpret_cast<DevPrime*>(base + o_prime);
     c->d_tw = base + o_tw;
-    c->d_inv_last = reinterpret_cast<ShoupConst*>(base + o_il);
+    c->d_inv_fin = reinterpret_cast<InvFinal*>(base + o_fin);
+    c->moddown_fin = reinterpret_cast<const InvFinal*>(base + o_fin_down);
+    c->modup_fin.resize(n_q + 1);
+    for (int l = 1; l <= n_q; ++l) c->modup_fin[l] = reinterpret_cast<const InvFinal*>(base + o_fin_up[l]);
     c->d_pinv = reinterpret_cast<ShoupConst*>(base + o_pinv);
     c->d_pmod = reinterpret_cast<ShoupConst*>(base + o_pmod);
     c->d_rescale = reinterpret_cast<RescaleConst*>(base + o_rs);
@@ -436,10 +459,10 @@ Context* create_context(int logN, int n_q, int K, int dnum, const uint64_t* prim
       ConvTable t;
       t.n_src = o.ns;
       t.n_dst = o.nd;
-      t.src_pos = reinterpret_cast<const int*>(base + o.sp);
+      t.src0 = o.src0;
       t.src_prime = reinterpret_cast<const int*>(base + o.spr);
-      t.pre = reinterpret_cast<const ShoupConst*>(base + o.pre);
-      t.dst_pos = reinterpret_cast<const int*>(base + o.dp);
+      t.dst_skip = o.dst_skip;
+      t.dst_gap = o.dst_gap;
       t.dst_prime = reinterpret_cast<const int*>(base + o.dpr);
       t.mat = reinterpret_cast<const uint64_t*>(base + o.mat);
       t.lift = o.lift;

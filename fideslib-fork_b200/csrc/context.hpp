@@ -42,14 +42,26 @@ struct __align__(16) TcDest {
   uint64_t qinv;  // bits of the double nearest 1 / q
 };
 
+// Last-stage factors of an inverse transform of one limb: N^-1 (sums) and psi_rev^-1[1] N^-1
+// (differences), times an optional factor of the limb, as Shoup constants and, for primes below 2^50,
+// as centred doubles.
+struct __align__(16) InvFinal {
+  ShoupConst sum, diff;
+  double fsum, fdiff;
+};
+
 // Table of one approximate basis conversion (ApproxSwitchCRTBasis):
-//   y_i = [x_i * pre_i]_{q_src_i};  out_j = [sum_i y_i * mat[i][j]]_{q_dst_j}.
+//   out_j = [sum_i y_i * mat[i][j]]_{q_dst_j},  y_i = [x_i * (Q_src / q_i)^-1]_{q_src_i}.
+// The sources y_i come from the inverse transform that precedes every conversion: its last stage
+// multiplies by InvFinal factors that hold (Q_src / q_i)^-1 (modup_fin, moddown_fin).
 struct ConvTable {
   int n_src = 0, n_dst = 0;
-  const int* src_pos = nullptr;    // limb index of source i in the input poly
+  int src0 = 0;                    // source i is limb src0 + i of the input poly
   const int* src_prime = nullptr;  // prime id of source i
-  const ShoupConst* pre = nullptr; // [n_src]
-  const int* dst_pos = nullptr;    // limb index of output j in the output poly
+  // limb index of output j in the output poly: the outputs are consecutive but for the source digit
+  // (dst_gap limbs from dst_skip on)
+  int dst_skip = 0, dst_gap = 0;
+  __host__ __device__ int dst_pos(int j) const { return j < dst_skip ? j : j + dst_gap; }
   const int* dst_prime = nullptr;  // prime id of output j
   const uint64_t* mat = nullptr;   // [n_src][n_dst]
   // Tensor-core form (conv_tc.cu); tc_b == nullptr when the table does not fit it.
@@ -70,11 +82,9 @@ struct ConvTable {
 // Basis-conversion engine: tensor cores (INT8 split on tcgen05) or 64-bit SIMT.
 enum ConvEngine { CONV_AUTO = 0, CONV_SIMT = 1, CONV_TENSOR = 2 };
 
-// FP64 constants of a prime below 2^50 for the floating-point NTT butterflies: q, 1/q, and
-// the inverse transform's last-stage factors N^-1 and psi_rev^-1[1] N^-1; for the inner products
-// 2^51 and, on Q limbs, P modulo q.  The factors are centred.
+// FP64 constants of a prime below 2^50: q, 1/q, and, centred, 2^51 and (on Q limbs) P modulo q.
 struct F64Prime {
-  double q, qinv, ninv, last, w51, pm;
+  double q, qinv, w51, pm;
 };
 
 struct RescaleConst {
@@ -99,7 +109,9 @@ struct Context {
   // device tables
   DevPrime* d_prime = nullptr;       // [n_q + K]
   char* d_tw = nullptr;              // NTT twiddle tables, one block per prime at DevPrime::tw (ntt.cuh)
-  ShoupConst* d_inv_last = nullptr;  // [n_q + K]: psi_rev^-1[1] * N^-1 (last GS stage)
+  InvFinal* d_inv_fin = nullptr;     // [n_q + K]: the inverse transform's last stage
+  std::vector<const InvFinal*> modup_fin;   // [l]: the same times (Q_d / q_i)^-1 of limb i's digit d, device [l]
+  const InvFinal* moddown_fin = nullptr;    // [K]: the same times (P / p_k)^-1, device
   F64Prime* d_f64 = nullptr;         // [n_q + K]
   ShoupConst* d_pinv = nullptr;      // [n_q]: P^-1 mod q_j
   ShoupConst* d_pmod = nullptr;      // [n_q]: P mod q_j

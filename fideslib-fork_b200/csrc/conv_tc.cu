@@ -206,6 +206,7 @@ __global__ void __launch_bounds__(TC_M, 7)
   const ConvJob& J = L.j[blockIdx.y];
   const ConvTable& T = J.t;
   const int ns = T.n_src, nd = T.n_dst, kpad = T.tc_kpad, ndp = T.tc_nd_pad;
+  const int nchunks = (ndp + TC_DCHUNK - 1) / TC_DCHUNK;
   const TcLayout Ly = tc_layout(kpad, ndp);
   const int tid = threadIdx.x, warp = tid >> 5;
   const int N = 1 << logN;
@@ -235,24 +236,20 @@ __global__ void __launch_bounds__(TC_M, 7)
   }
   for (int j = tid; j < ndp; j += TC_M) {  // destination constants
     dconst[j] = T.tc_dst[j];
-    dofs[j] = j < nd ? T.dst_pos[j] << logN : 0;
+    dofs[j] = j < nd ? T.dst_pos(j) << logN : 0;
   }
   pdl_wait();  // tables only so far
-  {  // A: the bytes of the pre-scaled residues of this thread's coefficient
+  {  // A: the bytes of the sources (pre-scaled residues) of this thread's coefficient
     uint64_t x[TC_MAX_SRC];
 #pragma unroll
     for (int i = 0; i < TC_MAX_SRC; ++i)
-      if (i < ns) x[i] = J.src[(size_t)T.src_pos[i] * N + coef];
+      if (i < ns) x[i] = J.src[(size_t)(T.src0 + i) * N + coef];
     uint64_t lifted = 0;  // reduced-noise lift: the count is source row ns of the product
+    if (T.lift) {
 #pragma unroll
-    for (int i = 0; i < TC_MAX_SRC; ++i)
-      if (i < ns) {
-        const ShoupConst pc = T.pre[i];
-        const uint64_t q = primes[T.src_prime[i]].q;
-        x[i] = shoup(x[i], pc.w, pc.ws, q);
-        lifted += x[i] > (q >> 1);
-      }
-    if (!T.lift) lifted = 0;
+      for (int i = 0; i < TC_MAX_SRC; ++i)
+        if (i < ns) lifted += x[i] > (primes[T.src_prime[i]].q >> 1);
+    }
 #pragma unroll
     for (int p = 0; p < TC_MAX_SRC / 2; ++p) {
       if (p >= kpad / 16) break;
@@ -269,17 +266,16 @@ __global__ void __launch_bounds__(TC_M, 7)
   bool ok = true;
   int failed_chunk = -1;
   const uint32_t tbase = *slot;
-  const uint32_t a0 = smem_addr(sA), b0 = smem_addr(sB);
+  const uint32_t sa = smem_addr(sA), sb = smem_addr(sB);
   const uint32_t trow = tbase + ((uint32_t)(warp * 32) << 16);
-  const int nchunks = (ndp + TC_DCHUNK - 1) / TC_DCHUNK;
   uint64_t* out = J.dst + coef;
   for (int c = 0; ok && c < nchunks; ++c) {
     const int ndc = min(TC_DCHUNK, ndp - c * TC_DCHUNK);  // even: N = 8 ndc is a multiple of 16
     if (tid == 0) {
       const uint32_t idesc = idesc_u8(8 * ndc);
       for (int kc = 0; kc < kpad / 32; ++kc) {
-        const uint64_t da = smem_desc(a0 + kc * 2 * (TC_M * 16), TC_M * 16, 128);
-        const uint64_t db = smem_desc(b0 + (kc * 2 * (8 * ndp) + c * TC_DCHUNK * 8) * 16, 8 * ndp * 16, 128);
+        const uint64_t da = smem_desc(sa + kc * 2 * (TC_M * 16), TC_M * 16, 128);
+        const uint64_t db = smem_desc(sb + (kc * 2 * (8 * ndp) + c * TC_DCHUNK * 8) * 16, 8 * ndp * 16, 128);
         mma_u8(tbase, da, db, idesc, kc > 0);
       }
       mma_commit(bar_a);

@@ -34,15 +34,13 @@ __global__ void __launch_bounds__(EW_THREADS) conv_kernel(const __grid_constant_
   const ConvTable& T = J.t;
   extern __shared__ uint64_t sm[];
   const int ns = NS ? NS : T.n_src, nd = T.n_dst, lift = T.lift;
-  ShoupConst* pre = reinterpret_cast<ShoupConst*>(sm);       // [ns]
-  DevPrime* dp = reinterpret_cast<DevPrime*>(sm + 2 * ns);   // [nd]
-  uint64_t* mat = sm + 2 * ns + 8 * nd;                      // [ns + lift][nd]
+  DevPrime* dp = reinterpret_cast<DevPrime*>(sm);             // [nd]
+  uint64_t* mat = sm + sizeof(DevPrime) / 8 * nd;             // [ns + lift][nd]
   int* dpos = reinterpret_cast<int*>(mat + (ns + lift) * nd); // [nd]
   for (int i = threadIdx.x; i < (ns + lift) * nd; i += blockDim.x) mat[i] = T.mat[i];
-  for (int i = threadIdx.x; i < ns; i += blockDim.x) pre[i] = T.pre[i];
   for (int j = threadIdx.x; j < nd; j += blockDim.x) {
     dp[j] = primes[T.dst_prime[j]];
-    dpos[j] = T.dst_pos[j];
+    dpos[j] = T.dst_pos(j);
   }
   __syncthreads();
   pdl_wait();
@@ -54,12 +52,14 @@ __global__ void __launch_bounds__(EW_THREADS) conv_kernel(const __grid_constant_
 #pragma unroll
   for (int i = 0; i < R; ++i) {
     if (NS == 0 && i >= ns) break;
-    const uint64_t q = primes[T.src_prime[i]].q;
-    const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(J.src + (size_t)T.src_pos[i] * N + n);
-    y0[i] = shoup(v.x, pre[i].w, pre[i].ws, q);
-    y1[i] = shoup(v.y, pre[i].w, pre[i].ws, q);
-    lift0 += y0[i] > (q >> 1);
-    lift1 += y1[i] > (q >> 1);
+    const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(J.src + (size_t)(T.src0 + i) * N + n);
+    y0[i] = v.x;
+    y1[i] = v.y;
+    if (lift) {
+      const uint64_t half = primes[T.src_prime[i]].q >> 1;
+      lift0 += y0[i] > half;
+      lift1 += y1[i] > half;
+    }
   }
   uint64_t* dst = J.dst + n;
   for (int j = 0; j < nd; ++j) {
@@ -804,7 +804,7 @@ void launch_conv(Context* c, const ConvJob* jobs, int n, cudaStream_t s) {
       double bytes = 0;
       for (int i = 0; i < m; ++i) {
         const ConvTable& t = L.j[i].t;
-        smem = std::max(smem, (size_t)(t.n_src + t.lift) * t.n_dst * 8 + (size_t)t.n_src * 16 + (size_t)t.n_dst * 68);
+        smem = std::max(smem, (size_t)(t.n_src + t.lift) * t.n_dst * 8 + (size_t)t.n_dst * (sizeof(DevPrime) + 4));
         bytes += 8.0 * c->N * (t.n_src + t.n_dst);
       }
       dim3 grid(c->N / (2 * EW_THREADS), m);

@@ -18,8 +18,8 @@ int kernel_binary_version(int device);
 // ---- basis conversion (ModUp: DecompAndModUpConv, Conv.cu:274-423; ModDown: ModDown2, Conv.cu:27-133)
 struct ConvJob {
   ConvTable t;
-  const uint64_t* src;  // source limb i at src + t.src_pos[i] * N (coefficient domain)
-  uint64_t* dst;        // output j at dst + t.dst_pos[j] * N
+  const uint64_t* src;  // source y_i at src + (t.src0 + i) * N (coefficient domain, ConvTable)
+  uint64_t* dst;        // output j at dst + t.dst_pos(j) * N
 };
 constexpr int MAX_CONV_JOBS = 96;
 // Job lists are passed by value; launches of a few jobs take the short form (a large parameter block

@@ -18,8 +18,6 @@ struct __align__(16) DevPrime {
   uint64_t one_s; // floor(2^64 / q): Shoup companion of 1
   uint64_t r64;   // 2^64 mod q
   uint64_t r64_s; // Shoup companion of r64
-  uint64_t ninv;  // N^-1 mod q
-  uint64_t ninv_s;
   uint64_t tw;    // byte offset of the prime's NTT twiddle tables (ntt.cuh)
 };
 

@@ -19,7 +19,7 @@ void fill_runs(NttLimbList& L, const LimbRef* limbs, int n, size_t N) {
       const LimbRef& y = limbs[i - 1];
       LimbRun& r = L.run[L.runs - 1];
       joins = next(y.ptr, x.ptr) && next(y.src, x.src) && next(y.ep0, x.ep0) && next(y.ep1, x.ep1) &&
-              x.prime == y.prime + 1 && x.aux == y.aux;
+              x.prime == y.prime + 1 && x.aux == y.aux && (y.fin ? x.fin == y.fin + 1 : !x.fin);
       if (joins) {
         const bool same = x.pro == y.pro, step = next(y.pro, x.pro);
         if (i - r.first == 1) r.pro_step = !same && step;
@@ -28,7 +28,7 @@ void fill_runs(NttLimbList& L, const LimbRef* limbs, int n, size_t N) {
     }
     if (!joins) {
       if (L.runs == MAX_NTT_RUNS) break;
-      L.run[L.runs++] = LimbRun{x.ptr, x.src, x.pro, x.ep0, x.ep1, (int16_t)x.prime, (int16_t)x.aux, (int16_t)i, 0};
+      L.run[L.runs++] = LimbRun{x.ptr, x.src, x.pro, x.ep0, x.ep1, x.fin, (int16_t)x.prime, (int16_t)x.aux, (int16_t)i, 0};
     }
     L.run_of[i] = (uint8_t)(L.runs - 1);
     L.n = i + 1;
@@ -48,7 +48,7 @@ void ntt_limbs(Context* c, const LimbRef* limbs, int n, bool inverse, cudaStream
   a.primes = c->d_prime;
   a.tw = c->d_tw;
   a.f64 = c->d_f64;
-  a.inv_last = c->d_inv_last;
+  a.inv_fin = c->d_inv_fin;
   a.pinv = c->d_pinv;
   a.rescale = c->d_rescale;
   a.pmod = c->d_pmod;

@@ -106,10 +106,10 @@ struct LimbRef {
   const uint64_t* ep1;
   int prime;
   int aux;  // IN_SWITCH / IN_CONV_SW / OUT_RESCALE / OUT_MDRS: the level l being rescaled (top prime l - 1)
-  uint64_t pad;
+  const InvFinal* fin;    // inverse only: last-stage factors of this limb (null: the prime's own)
 };
 
-inline LimbRef lref(uint64_t* p, int prime) { return LimbRef{p, nullptr, nullptr, nullptr, nullptr, prime, 0, 0}; }
+inline LimbRef lref(uint64_t* p, int prime) { return LimbRef{p, nullptr, nullptr, nullptr, nullptr, prime, 0, nullptr}; }
 
 #ifndef FIDES_MAX_NTT_LIMBS
 #define FIDES_MAX_NTT_LIMBS 448
@@ -123,6 +123,7 @@ constexpr int MAX_NTT_LIMBS = FIDES_MAX_NTT_LIMBS;
 struct LimbRun {
   uint64_t* ptr;
   const uint64_t *src, *pro, *ep0, *ep1;
+  const InvFinal* fin;
   int16_t prime, aux;
   int16_t first;     // index of the run's first limb in the launch
   int16_t pro_step;  // 1: pro advances with the limb

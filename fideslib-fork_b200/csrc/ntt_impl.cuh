@@ -133,7 +133,7 @@ struct PassArgs {
   const DevPrime* primes;
   const char* tw;              // twiddle tables of all primes (DevPrime::tw)
   const F64Prime* f64;         // [prime]
-  const ShoupConst* inv_last;  // [prime]: psi_rev^-1[1] * N^-1
+  const InvFinal* inv_fin;     // [prime]: the inverse transform's last stage
   const ShoupConst* pinv;      // [Q prime]: P^-1 mod q (OUT_MODDOWN)
   const RescaleConst* rescale; // [level][Q prime] (OUT_RESCALE, OUT_MDRS)
   const ShoupConst* pmod;      // [Q prime]: P mod q (IN_CONV_SW, IN_ADD_PMUL)
@@ -161,7 +161,7 @@ __device__ __forceinline__ int padu(int u) {
 // this thread (SLOTS heaps interleaved, see ntt.cuh).
 template <int LE, int LOGP, int LO, int BHI, int BLO, int SLOTS, bool FWD, int PASS, bool LAZY4>
 __device__ __forceinline__ void run_chunk(uint64_t (&x)[1 << LE], const ShoupConst* tw, const DevPrime& pr,
-                                          ShoupConst last, uint64_t& B, uint64_t pol) {
+                                          const InvFinal& fin, uint64_t& B, uint64_t pol) {
   constexpr int E = 1 << LE;
   const Lazy4Red lr4 = lazy4_red(pr.q);
 #pragma unroll
@@ -178,13 +178,13 @@ __device__ __forceinline__ void run_chunk(uint64_t (&x)[1 << LE], const ShoupCon
 #pragma unroll
     for (int hi = 0; hi < H; ++hi) {
       if (!FWD && PASS == COL && b == LOGP - 1) {
-        // last inverse stage (global stage 0): fold N^-1 into both outputs
+        // last inverse stage (global stage 0): fold N^-1 (times the limb's factor) into both outputs
 #pragma unroll
         for (int lr = 0; lr < (1 << rb); ++lr) {
           const int r0 = (hi << (rb + 1)) | lr, r1 = r0 | (1 << rb);
           uint64_t a = x[r0], c = x[r1];
-          x[r0] = shoup(a + c, pr.ninv, pr.ninv_s, pr.q);
-          x[r1] = shoup(a - c + B, last.w, last.ws, pr.q);
+          x[r0] = shoup(a + c, fin.sum.w, fin.sum.ws, pr.q);
+          x[r1] = shoup(a - c + B, fin.diff.w, fin.diff.ws, pr.q);
         }
       } else {
         const ShoupConst w = ld_tw(tw + (H + hi) * SLOTS, pol);
@@ -211,7 +211,7 @@ __device__ __forceinline__ void run_chunk(uint64_t (&x)[1 << LE], const ShoupCon
 // run_chunk on FP64 residues (q < 2^50): the same stages, pairs and twiddles.
 template <int LE, int LOGP, int LO, int BHI, int BLO, int SLOTS, bool FWD, int PASS>
 __device__ __forceinline__ void run_chunk_f64(double (&x)[1 << LE], const double* tw, const F64Prime& fp,
-                                              uint64_t pol) {
+                                              const InvFinal& fin, uint64_t pol) {
   constexpr int E = 1 << LE, NS = BHI - BLO + 1;
 #pragma unroll
   for (int k = 0; k < NS; ++k) {
@@ -230,8 +230,8 @@ __device__ __forceinline__ void run_chunk_f64(double (&x)[1 << LE], const double
         for (int lr = 0; lr < (1 << rb); ++lr) {
           const int r0 = (hi << (rb + 1)) | lr, r1 = r0 | (1 << rb);
           const double a = x[r0], c = x[r1];
-          x[r0] = f_mulmod(__dadd_rn(a, c), fp.ninv, fp.q, fp.qinv);
-          x[r1] = f_mulmod(__dsub_rn(a, c), fp.last, fp.q, fp.qinv);
+          x[r0] = f_mulmod(__dadd_rn(a, c), fin.fsum, fp.q, fp.qinv);
+          x[r1] = f_mulmod(__dsub_rn(a, c), fin.fdiff, fp.q, fp.qinv);
         }
       } else {
         if (H == 1)
@@ -278,14 +278,14 @@ struct Chunk {
 
 template <int LE, int LOGP, int PASS, bool FWD, bool LAZY4, typename CH>
 __device__ __forceinline__ void one_chunk(uint64_t (&x)[1 << LE], CH, int t, const ShoupConst* tw, const DevPrime& pr,
-                                          ShoupConst last, uint64_t& B, uint64_t pol) {
-  run_chunk<LE, LOGP, CH::LO, CH::BHI, CH::BLO, CH::SLOTS, FWD, PASS, LAZY4>(x, tw + CH::OFF + (t >> CH::LO), pr, last,
+                                          const InvFinal& fin, uint64_t& B, uint64_t pol) {
+  run_chunk<LE, LOGP, CH::LO, CH::BHI, CH::BLO, CH::SLOTS, FWD, PASS, LAZY4>(x, tw + CH::OFF + (t >> CH::LO), pr, fin,
                                                                              B, pol);
 }
 template <int LE, int LOGP, int PASS, bool FWD, typename CH>
 __device__ __forceinline__ void one_chunk_f64(double (&x)[1 << LE], CH, int t, const double* tw, const F64Prime& fp,
-                                              uint64_t pol) {
-  run_chunk_f64<LE, LOGP, CH::LO, CH::BHI, CH::BLO, CH::SLOTS, FWD, PASS>(x, tw + CH::OFF + 2 * (t >> CH::LO), fp, pol);
+                                              const InvFinal& fin, uint64_t pol) {
+  run_chunk_f64<LE, LOGP, CH::LO, CH::BHI, CH::BLO, CH::SLOTS, FWD, PASS>(x, tw + CH::OFF + 2 * (t >> CH::LO), fp, fin, pol);
 }
 
 // Barrier between a pass's shared-memory exchanges: of the CTA, or of the warp where every
@@ -301,12 +301,12 @@ __device__ __forceinline__ void pass_sync() {
 // The register chunks of one pass, separated by shared-memory exchanges.
 template <int LE, int LOGP, int PASS, bool FWD, bool LAZY4, bool WARP, typename SIDX>
 __device__ __forceinline__ void chunks(uint64_t (&x)[1 << LE], uint64_t* sm, SIDX sidx, int g, int t,
-                                       const ShoupConst* tw, const DevPrime& pr, ShoupConst last, uint64_t& B,
+                                       const ShoupConst* tw, const DevPrime& pr, const InvFinal& fin, uint64_t& B,
                                        bool direct_load, uint64_t pol) {
   constexpr int E = 1 << LE;
   constexpr int NCH = (LOGP + LE - 1) / LE;
   using C0 = Chunk<LE, LOGP, FWD, 0>;
-  one_chunk<LE, LOGP, PASS, FWD, LAZY4>(x, C0{}, t, tw, pr, last, B, pol);
+  one_chunk<LE, LOGP, PASS, FWD, LAZY4>(x, C0{}, t, tw, pr, fin, B, pol);
   if constexpr (NCH > 1) {
     using C1 = Chunk<LE, LOGP, FWD, 1>;
     if (!direct_load) pass_sync<WARP>();
@@ -315,7 +315,7 @@ __device__ __forceinline__ void chunks(uint64_t (&x)[1 << LE], uint64_t* sm, SID
     pass_sync<WARP>();
 #pragma unroll
     for (int r = 0; r < E; ++r) x[r] = sm[sidx(g, u_of<C1::LO, LE>(t, r))];
-    one_chunk<LE, LOGP, PASS, FWD, LAZY4>(x, C1{}, t, tw, pr, last, B, pol);
+    one_chunk<LE, LOGP, PASS, FWD, LAZY4>(x, C1{}, t, tw, pr, fin, B, pol);
   }
   if constexpr (NCH > 2) {
     using C1 = Chunk<LE, LOGP, FWD, 1>;
@@ -326,7 +326,7 @@ __device__ __forceinline__ void chunks(uint64_t (&x)[1 << LE], uint64_t* sm, SID
     pass_sync<WARP>();
 #pragma unroll
     for (int r = 0; r < E; ++r) x[r] = sm[sidx(g, u_of<C2::LO, LE>(t, r))];
-    one_chunk<LE, LOGP, PASS, FWD, LAZY4>(x, C2{}, t, tw, pr, last, B, pol);
+    one_chunk<LE, LOGP, PASS, FWD, LAZY4>(x, C2{}, t, tw, pr, fin, B, pol);
   }
   static_assert(NCH <= 3, "sub-transform too large");
 }
@@ -334,12 +334,13 @@ __device__ __forceinline__ void chunks(uint64_t (&x)[1 << LE], uint64_t* sm, SID
 // chunks() on FP64 residues; the shared-memory exchanges move the doubles' bits.
 template <int LE, int LOGP, int PASS, bool FWD, bool WARP, typename SIDX>
 __device__ __forceinline__ void chunks_f64(double (&x)[1 << LE], uint64_t* smu, SIDX sidx, int g, int t,
-                                           const double* tw, const F64Prime& fp, bool direct_load, uint64_t pol) {
+                                           const double* tw, const F64Prime& fp, const InvFinal& fin, bool direct_load,
+                                           uint64_t pol) {
   constexpr int E = 1 << LE;
   constexpr int NCH = (LOGP + LE - 1) / LE;
   double* sm = reinterpret_cast<double*>(smu);
   using C0 = Chunk<LE, LOGP, FWD, 0>;
-  one_chunk_f64<LE, LOGP, PASS, FWD>(x, C0{}, t, tw, fp, pol);
+  one_chunk_f64<LE, LOGP, PASS, FWD>(x, C0{}, t, tw, fp, fin, pol);
   if constexpr (NCH > 1) {
     using C1 = Chunk<LE, LOGP, FWD, 1>;
     if (!direct_load) pass_sync<WARP>();
@@ -348,7 +349,7 @@ __device__ __forceinline__ void chunks_f64(double (&x)[1 << LE], uint64_t* smu, 
     pass_sync<WARP>();
 #pragma unroll
     for (int r = 0; r < E; ++r) x[r] = sm[sidx(g, u_of<C1::LO, LE>(t, r))];
-    one_chunk_f64<LE, LOGP, PASS, FWD>(x, C1{}, t, tw, fp, pol);
+    one_chunk_f64<LE, LOGP, PASS, FWD>(x, C1{}, t, tw, fp, fin, pol);
   }
   if constexpr (NCH > 2) {
     using C1 = Chunk<LE, LOGP, FWD, 1>;
@@ -359,7 +360,7 @@ __device__ __forceinline__ void chunks_f64(double (&x)[1 << LE], uint64_t* smu, 
     pass_sync<WARP>();
 #pragma unroll
     for (int r = 0; r < E; ++r) x[r] = sm[sidx(g, u_of<C2::LO, LE>(t, r))];
-    one_chunk_f64<LE, LOGP, PASS, FWD>(x, C2{}, t, tw, fp, pol);
+    one_chunk_f64<LE, LOGP, PASS, FWD>(x, C2{}, t, tw, fp, fin, pol);
   }
 }
 
@@ -406,10 +407,12 @@ __global__ void __launch_bounds__(PassThreads<LOGN, PASS, G, LE>::NT, PassThread
     lr.ep1 = R.ep1 ? R.ep1 + at : nullptr;
     lr.prime = R.prime + k;
     lr.aux = R.aux;
+    lr.fin = R.fin ? R.fin + k : nullptr;
   }
   const DevPrime pr = a.primes[lr.prime];
   const char* tw_prime = a.tw + pr.tw;  // this prime's twiddle tables
-  const ShoupConst last = FWD ? ShoupConst{0, 0} : a.inv_last[lr.prime];
+  InvFinal fin{};
+  if (!FWD && PASS == COL) fin = *(lr.fin ? lr.fin : a.inv_fin + lr.prime);
   uint64_t* data = lr.ptr;
   const int tid = threadIdx.x;
   int g, t;
@@ -661,7 +664,7 @@ __global__ void __launch_bounds__(PassThreads<LOGN, PASS, G, LE>::NT, PassThread
 #pragma unroll
     for (int r = 0; r < E; ++r) xf[r] = __longlong_as_double((long long)x[r]);
     chunks_f64<LE, LOGP, PASS, FWD, WARP>(xf, sm, sidx, g, t, reinterpret_cast<const double*>(tw_prime) + tw0, fp,
-                                          direct_load && !STAGE_PRO, pol);
+                                          fin, direct_load && !STAGE_PRO, pol);
 #pragma unroll
     for (int r = 0; r < E; ++r) x[r] = bits(xf[r]);
     drain(finish_f64);
@@ -681,9 +684,9 @@ __global__ void __launch_bounds__(PassThreads<LOGN, PASS, G, LE>::NT, PassThread
   uint64_t B = lazy4 ? pr.q2 : pr.q;  // inverse: bound of the values (a multiple of q)
   if (!FWD && PASS == COL) B = inv_bound(B, PassShape<LOGN, ROW>::LOGP);
   if (lazy4)
-    chunks<LE, LOGP, PASS, FWD, true, WARP>(x, sm, sidx, g, t, tw, pr, last, B, direct_load && !STAGE_PRO, pol);
+    chunks<LE, LOGP, PASS, FWD, true, WARP>(x, sm, sidx, g, t, tw, pr, fin, B, direct_load && !STAGE_PRO, pol);
   else
-    chunks<LE, LOGP, PASS, FWD, false, WARP>(x, sm, sidx, g, t, tw, pr, last, B, direct_load && !STAGE_PRO, pol);
+    chunks<LE, LOGP, PASS, FWD, false, WARP>(x, sm, sidx, g, t, tw, pr, fin, B, direct_load && !STAGE_PRO, pol);
 
   // ---- final reduction of the completed transform
   if (FWD && PASS == ROW) {

@@ -39,7 +39,8 @@ void check_level(Context* c, int l, int min_l = 1) {
   if (l < min_l || l > c->n_q) throw Error(-4, "level " + std::to_string(l) + " out of range");
 }
 
-// ModUp, first phase: INTT of xs[i] (times ys[i] when given) into tmps[i].
+// ModUp, first phase: INTT of xs[i] (times ys[i] when given) into tmps[i], limb j times
+// (Q_d / q_j)^-1 of its digit d: the conversion's sources.
 void modup_intt(Context* c, const uint64_t* const* xs, const uint64_t* const* ys, const int* ls,
                 uint64_t* const* tmps, int n, cudaStream_t s) {
   const size_t N = c->N;
@@ -49,6 +50,7 @@ void modup_intt(Context* c, const uint64_t* const* xs, const uint64_t* const* ys
       LimbRef r = lref(tmps[i] + j * N, j);
       r.src = xs[i] + j * N;
       if (ys) r.pro = ys[i] + j * N;
+      r.fin = c->modup_fin[ls[i]] + j;
       refs.push_back(r);
     }
   ntt_limbs(c, refs.data(), (int)refs.size(), true, s, ys ? IN_MUL : IN_PLAIN);
@@ -94,7 +96,10 @@ void moddown_prep(Context* c, uint64_t* const* exts, const int* ls, uint64_t* co
   if (K == 0) throw Error(-1, "ModDown needs special primes");
   std::vector<LimbRef> refs;
   for (int i = 0; i < n; ++i)
-    for (int k = 0; k < K; ++k) refs.push_back(lref(exts[i] + (ls[i] + k) * N, c->n_q + k));
+    for (int k = 0; k < K; ++k) {
+      refs.push_back(lref(exts[i] + (ls[i] + k) * N, c->n_q + k));
+      refs.back().fin = c->moddown_fin + k;  // times (P / p_k)^-1
+    }
   ntt_limbs(c, refs.data(), (int)refs.size(), true, s);
   std::vector<ConvJob> jobs;
   for (int i = 0; i < n; ++i) jobs.push_back(ConvJob{c->moddown_table(ls[i]), exts[i] + ls[i] * N, convs[i]});
