@@ -38,7 +38,7 @@ struct __align__(16) ShoupConst {
 
 // Destination-prime constants of the tensor-core conversion epilogue.
 struct __align__(16) TcDest {
-  uint64_t q;
+  uint64_t nq;    // -q modulo 2^64
   uint64_t qinv;  // bits of the double nearest 1 / q
 };
 

@@ -1,10 +1,10 @@
 // Tensor-core basis conversion (tcgen05, kind::i8).  The arithmetic identity is stated in
 // conv_tc.hpp; this file holds the table builder and the kernel.
 //
-// One CTA converts 128 coefficients (the MMA's M, one TMEM lane each) of one job:
+// One CTA converts runs of 128 coefficients (the MMA's M, one TMEM lane each) of one job:
 //   1. warp 0 allocates 64 TMEM columns; the CTA starts cp.async copies of the table's B image
-//      (the shared-memory form of the byte matrix) and, while they are in flight, writes A: the
-//      eight bytes of every pre-scaled residue y_i of its 128 coefficients, K-major;
+//      (the shared-memory form of the byte matrix) and of A, K-major: the eight bytes of every source
+//      residue of its 128 coefficients, as they lie in memory;
 //   2. per chunk of 8 destination limbs (64 columns: 8 byte planes each), thread 0 issues
 //      K/32 MMAs (M 128, N 8 x limbs, K 32) and commits them to an mbarrier;
 //   3. after a bounded wait, each warp reads its 32 TMEM lanes (tcgen05.ld 32x32b), folds the
@@ -36,7 +36,7 @@ void build_tc_image(const uint64_t* mat, int ns, int nd, const std::vector<int>&
   for (int j = 0; j < nd; ++j) {
     const uint64_t p = primes[dst_prime[j]];
     const double qinv = 1.0 / (double)p;
-    dst[j].q = p;
+    dst[j].nq = 0 - p;
     std::memcpy(&dst[j].qinv, &qinv, sizeof(double));
     for (int i = 0; i < ns; ++i)
       for (int a = 0; a < 8; ++a) {
@@ -60,13 +60,12 @@ constexpr uint32_t TC_COLS = 64;   // TMEM columns held by one CTA (8 limbs x 8 
 constexpr int TC_SMEM_FLOOR = 29 * 1024;
 
 struct TcLayout {
-  int o_dst, o_pos, o_a, o_b, total;
+  int o_dst, o_a, o_b, total;
 };
 __host__ __device__ inline TcLayout tc_layout(int kpad, int ndp) {
   TcLayout L;
   L.o_dst = 16;  // [0, 8): mbarrier, [8, 12): TMEM address
-  L.o_pos = L.o_dst + ndp * (int)sizeof(TcDest);
-  L.o_a = (L.o_pos + ndp * 4 + 127) & ~127;
+  L.o_a = (L.o_dst + ndp * (int)sizeof(TcDest) + 127) & ~127;
   L.o_b = L.o_a + TC_M * kpad;
   L.total = L.o_b + kpad * 8 * ndp;
   return L;
@@ -137,6 +136,9 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&d)[8]) {
                : "r"(taddr));
 }
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tc_cp_async8(void* smem, const void* gmem) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_addr(smem)), "l"(gmem) : "memory");
+}
 __device__ __forceinline__ void tc_cp_async16(void* smem, const void* gmem) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(smem)), "l"(gmem) : "memory");
 }
@@ -148,33 +150,35 @@ __device__ __forceinline__ void pin8(uint32_t (&d)[8]) {
 // sum_c 2^(8c) d[c] mod q for planes d[c] < 2^23 and a prime 2^48 < q < 2^62.
 // V = x + 2^32 y with x, y < 2^49 (V < 2^79.01 for K <= 128) is reduced by floating-point
 // Barrett reduction (the double-precision quotient estimate of NTL's MulMod): the integers
-// x, y convert to doubles exactly (2^52 exponent trick), and vd = fl(V), qinv = fl(1/q) give
+// x, y are formed with the exponent of 2^52 above them, so that they are doubles after one
+// subtraction, and vd = fl(V), qinv = fl(1/q) give
 // vd qinv within 2^-20 of V/q (V/q < 2^31.01); the fma adds 2^-17 with one more rounding of
 // at most 2^-21, so t lies in (V/q + 2^-17.6, V/q + 2^-16.6) and qh = floor(t) is
 // floor(V/q) or one more (qh < 2^32).  V - qh q lies in [-q, q), is computed exactly in
-// wrapping 64-bit arithmetic and needs one correction.  (Checked against 128-bit arithmetic
+// wrapping 64-bit arithmetic (nq = -q) and needs one correction.  (Checked against 128-bit arithmetic
 // on 40 M random, extreme and next-to-a-multiple-of-q plane sets over 4000 primes.)
-__device__ __forceinline__ uint64_t tc_fold(const uint32_t (&d)[8], uint64_t q, double qinv) {
+__device__ __forceinline__ uint64_t tc_fold(const uint32_t (&d)[8], uint64_t nq, double qinv) {
+  constexpr uint64_t EXP52 = 0x4330000000000000ull;
   const uint32_t a0 = d[0] + (d[1] << 8), a1 = d[2] + (d[3] << 8);  // < 2^32
   const uint32_t a2 = d[4] + (d[5] << 8), a3 = d[6] + (d[7] << 8);
-  const uint64_t x = (uint64_t)a0 + ((uint64_t)a1 << 16);  // planes 0-3, < 2^49
-  const uint64_t y = (uint64_t)a2 + ((uint64_t)a3 << 16);  // planes 4-7 (weight 2^32), < 2^49
+  const uint64_t x = (uint64_t)a1 * 65536u + (EXP52 | a0);  // 2^52's exponent, planes 0-3 (< 2^49)
+  const uint64_t y = (uint64_t)a3 * 65536u + (EXP52 | a2);  // planes 4-7 (weight 2^32)
   const double two52 = 4503599627370496.0;
-  const double xd = __longlong_as_double((long long)(0x4330000000000000ull | x)) - two52;
-  const double yd = __longlong_as_double((long long)(0x4330000000000000ull | y)) - two52;
+  const double xd = __longlong_as_double((long long)x) - two52, yd = __longlong_as_double((long long)y) - two52;
   const double vd = fma(yd, 4294967296.0, xd);
   const uint32_t qh = (uint32_t)__double2loint(__dadd_rd(fma(vd, qinv, 0x1p-17), two52));  // floor, < 2^32
-  uint64_t r = x + (y << 32) - (uint64_t)qh * q;
-  return r + ((uint64_t)((int64_t)r >> 63) & q);
+  uint64_t r = x - EXP52 + ((uint64_t)(uint32_t)y << 32) + (uint64_t)qh * nq;
+  if ((int64_t)r < 0) r -= nq;
+  return r;
 }
 
 // Stores the folded outputs of one chunk of NDC destination limbs (8 byte-plane columns each,
 // starting at TMEM address trow).  The TMEM loads of the next pair are in flight while the
 // current pair is folded; tcgen05.wait::ld waits for all of them, so each wait follows the
-// fold of the pair loaded before it.  dofs[j] = output limb position of destination j times N.
+// fold of the pair loaded before it.
 template <int NDC, bool CHECK>
-__device__ __forceinline__ void tc_epilogue(uint32_t trow, int j0, int nd, const TcDest* dconst, const int* dofs,
-                                            uint64_t* out) {
+__device__ __forceinline__ void tc_epilogue(uint32_t trow, int j0, int nd, const TcDest* dconst, const ConvTable& T,
+                                            int logN, uint64_t* out) {
   uint32_t d[2][2][8];
   tmem_ld8(trow, d[0][0]);
   tmem_ld8(trow + 8, d[0][1]);
@@ -192,16 +196,22 @@ __device__ __forceinline__ void tc_epilogue(uint32_t trow, int j0, int nd, const
       const int j = j0 + 2 * h + u;
       if (!CHECK || j < nd) {
         const TcDest P = dconst[j];
-        out[dofs[j]] = tc_fold(d[cur][u], P.q, __longlong_as_double((long long)P.qinv));
+        out[(size_t)T.dst_pos(j) << logN] = tc_fold(d[cur][u], P.nq, __longlong_as_double((long long)P.qinv));
       }
     }
     if (h + 1 < NDC / 2) tmem_wait_ld();
   }
 }
 
+// Each CTA converts `tiles` runs of 128 coefficients: the B image and the tables are fetched once, and
+// the next run's sources are on their way while the last chunk of the current one is folded.  The kernel
+// is bound by its instructions (issue 67-69 %, FMA-heavy pipe 41 %, DRAM 30 %): with a CTA a run and the
+// sources staged through registers 48 ModUp conversions at N = 2^16, level 30 took 242 us and 32 ModDown
+// conversions 159, now 211 and 156 (136 and 90 at the rate of a copy).
 template <int CAP>
 __global__ void __launch_bounds__(TC_M, 7)
-    conv_tc_kernel(const __grid_constant__ ConvJobListT<CAP> L, const DevPrime* primes, int logN, uint32_t* status) {
+    conv_tc_kernel(const __grid_constant__ ConvJobListT<CAP> L, const DevPrime* primes, int logN, uint32_t* status,
+                   int tiles) {
   extern __shared__ __align__(1024) uint8_t sm[];
   const ConvJob& J = L.j[blockIdx.y];
   const ConvTable& T = J.t;
@@ -209,12 +219,9 @@ __global__ void __launch_bounds__(TC_M, 7)
   const int nchunks = (ndp + TC_DCHUNK - 1) / TC_DCHUNK;
   const TcLayout Ly = tc_layout(kpad, ndp);
   const int tid = threadIdx.x, warp = tid >> 5;
-  const int N = 1 << logN;
-  const int coef = blockIdx.x * TC_M + tid;
   uint64_t* bar = reinterpret_cast<uint64_t*>(sm);
   uint32_t* slot = reinterpret_cast<uint32_t*>(sm + 8);
   TcDest* dconst = reinterpret_cast<TcDest*>(sm + Ly.o_dst);
-  int* dofs = reinterpret_cast<int*>(sm + Ly.o_pos);
   uint8_t* sA = sm + Ly.o_a;
   uint8_t* sB = sm + Ly.o_b;
   const uint32_t bar_a = smem_addr(bar);
@@ -232,77 +239,73 @@ __global__ void __launch_bounds__(TC_M, 7)
   {  // B image: 16-byte cp.async copies (kpad 8 ndp bytes, a multiple of 256), waited for below
     const int n16 = kpad * ndp / 2;
     for (int k = tid; k < n16; k += TC_M) tc_cp_async16(sB + 16 * k, T.tc_b + 16 * k);
-    asm volatile("cp.async.commit_group;" ::: "memory");
   }
-  for (int j = tid; j < ndp; j += TC_M) {  // destination constants
-    dconst[j] = T.tc_dst[j];
-    dofs[j] = j < nd ? T.dst_pos(j) << logN : 0;
-  }
+  for (int j = tid; j < ndp; j += TC_M) dconst[j] = T.tc_dst[j];  // destination constants
   pdl_wait();  // tables only so far
-  {  // A: the bytes of the sources (pre-scaled residues) of this thread's coefficient
-    uint64_t x[TC_MAX_SRC];
-#pragma unroll
-    for (int i = 0; i < TC_MAX_SRC; ++i)
-      if (i < ns) x[i] = J.src[(size_t)(T.src0 + i) * N + coef];
-    uint64_t lifted = 0;  // reduced-noise lift: the count is source row ns of the product
-    if (T.lift) {
-#pragma unroll
-      for (int i = 0; i < TC_MAX_SRC; ++i)
-        if (i < ns) lifted += x[i] > (primes[T.src_prime[i]].q >> 1);
-    }
-#pragma unroll
-    for (int p = 0; p < TC_MAX_SRC / 2; ++p) {
-      if (p >= kpad / 16) break;
-      const uint64_t lo = 2 * p < ns ? x[2 * p] : (2 * p == ns ? lifted : 0),
-                     hi = 2 * p + 1 < ns ? x[2 * p + 1] : (2 * p + 1 == ns ? lifted : 0);
-      *reinterpret_cast<ulonglong2*>(sA + p * (TC_M * 16) + tid * 16) = make_ulonglong2(lo, hi);
-    }
-  }
-  asm volatile("cp.async.wait_all;" ::: "memory");  // this thread's part of the B image
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // A and B, visible to the MMAs
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
+  // A: the bytes of the sources of one run, the eight of source i at 16-byte K slice i / 2.  The K rows past
+  // the last source are not written: B is zero there.
+  const int coef0 = blockIdx.x * tiles * TC_M + tid;
+  auto load_a = [&](int coef) {
+    const uint64_t* src = J.src + ((size_t)T.src0 << logN) + coef;
+    uint8_t* dst = sA + tid * 16;
+    for (int i = 0; i < ns; ++i)
+      tc_cp_async8(dst + (i >> 1) * (TC_M * 16) + (i & 1) * 8, src + ((size_t)i << logN));
+  };
+  load_a(coef0);
   bool ok = true;
-  int failed_chunk = -1;
-  const uint32_t tbase = *slot;
+  int phase = 0;  // of the mbarrier: one commit a chunk
   const uint32_t sa = smem_addr(sA), sb = smem_addr(sB);
-  const uint32_t trow = tbase + ((uint32_t)(warp * 32) << 16);
-  uint64_t* out = J.dst + coef;
-  for (int c = 0; ok && c < nchunks; ++c) {
-    const int ndc = min(TC_DCHUNK, ndp - c * TC_DCHUNK);  // even: N = 8 ndc is a multiple of 16
-    if (tid == 0) {
-      const uint32_t idesc = idesc_u8(8 * ndc);
-      for (int kc = 0; kc < kpad / 32; ++kc) {
-        const uint64_t da = smem_desc(sa + kc * 2 * (TC_M * 16), TC_M * 16, 128);
-        const uint64_t db = smem_desc(sb + (kc * 2 * (8 * ndp) + c * TC_DCHUNK * 8) * 16, 8 * ndp * 16, 128);
-        mma_u8(tbase, da, db, idesc, kc > 0);
-      }
-      mma_commit(bar_a);
+  uint32_t tbase = 0;
+  for (int tile = 0; ok && tile < tiles; ++tile) {
+    asm volatile("cp.async.wait_all;" ::: "memory");  // this thread's sources and part of the B image
+    if (T.lift) {  // reduced-noise lift: the number of sources above q / 2 is source row ns of the product
+      uint64_t lifted = 0;
+      for (int i = 0; i < ns; ++i)
+        lifted += *reinterpret_cast<const uint64_t*>(sA + (i >> 1) * (TC_M * 16) + tid * 16 + (i & 1) * 8) >
+                  (primes[T.src_prime[i]].q >> 1);
+      *reinterpret_cast<uint64_t*>(sA + (ns >> 1) * (TC_M * 16) + tid * 16 + (ns & 1) * 8) = lifted;
     }
-    ok = __syncthreads_and(bar_wait_bounded(bar_a, c & 1));
-    if (!ok) {
-      failed_chunk = c;
-      break;
-    }
-    tc_fence_after();
-    const int j0 = c * TC_DCHUNK;
-    if (ndc == TC_DCHUNK && j0 + TC_DCHUNK <= nd)
-      tc_epilogue<TC_DCHUNK, false>(trow, j0, nd, dconst, dofs, out);
-    else if (ndc == 2)
-      tc_epilogue<2, true>(trow, j0, nd, dconst, dofs, out);
-    else if (ndc == 4)
-      tc_epilogue<4, true>(trow, j0, nd, dconst, dofs, out);
-    else if (ndc == 6)
-      tc_epilogue<6, true>(trow, j0, nd, dconst, dofs, out);
-    else
-      tc_epilogue<8, true>(trow, j0, nd, dconst, dofs, out);
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // A and B, visible to the MMAs
     tc_fence_before();
-    __syncthreads();  // TMEM columns are free for the next chunk
+    __syncthreads();
     tc_fence_after();
+    tbase = *slot;
+    const uint32_t trow = tbase + ((uint32_t)(warp * 32) << 16);
+    uint64_t* out = J.dst + coef0 + tile * TC_M;
+    for (int c = 0; c < nchunks; ++c) {
+      const int ndc = min(TC_DCHUNK, ndp - c * TC_DCHUNK);  // even: N = 8 ndc is a multiple of 16
+      if (tid == 0) {
+        const uint32_t idesc = idesc_u8(8 * ndc);
+        for (int kc = 0; kc < kpad / 32; ++kc) {
+          const uint64_t da = smem_desc(sa + kc * 2 * (TC_M * 16), TC_M * 16, 128);
+          const uint64_t db = smem_desc(sb + (kc * 2 * (8 * ndp) + c * TC_DCHUNK * 8) * 16, 8 * ndp * 16, 128);
+          mma_u8(tbase, da, db, idesc, kc > 0);
+        }
+        mma_commit(bar_a);
+      }
+      ok = __syncthreads_and(bar_wait_bounded(bar_a, phase));
+      if (!ok) break;
+      phase ^= 1;
+      tc_fence_after();
+      if (c + 1 == nchunks && tile + 1 < tiles) load_a(coef0 + (tile + 1) * TC_M);  // the MMAs have read A
+      const int j0 = c * TC_DCHUNK;
+      if (ndc == TC_DCHUNK && j0 + TC_DCHUNK <= nd)
+        tc_epilogue<TC_DCHUNK, false>(trow, j0, nd, dconst, T, logN, out);
+      else if (ndc == 2)
+        tc_epilogue<2, true>(trow, j0, nd, dconst, T, logN, out);
+      else if (ndc == 4)
+        tc_epilogue<4, true>(trow, j0, nd, dconst, T, logN, out);
+      else if (ndc == 6)
+        tc_epilogue<6, true>(trow, j0, nd, dconst, T, logN, out);
+      else
+        tc_epilogue<8, true>(trow, j0, nd, dconst, T, logN, out);
+      tc_fence_before();
+      __syncthreads();  // TMEM columns are free for the next chunk
+      tc_fence_after();
+    }
   }
   if (!ok) {
-    // The commit of chunk failed_chunk has not arrived: its MMAs may still own the TMEM
+    // The commit of the chunk in flight has not arrived: its MMAs may still own the TMEM
     // columns.  tcgen05.commit arrives on the mbarrier only after every MMA this thread issued
     // before it has completed, so a second bounded wait on the same phase either sees them
     // finish (the dealloc below is then safe) or gives up after about another second, when
@@ -311,7 +314,7 @@ __global__ void __launch_bounds__(TC_M, 7)
     // host's next synchronising call returns FIDES_ERR_TIMEOUT until it is cleared).
     if (tid == 0) {
       atomicOr(status, 1u);
-      bar_wait_bounded(bar_a, failed_chunk & 1);
+      bar_wait_bounded(bar_a, phase);
     }
     __syncthreads();
   }
@@ -342,9 +345,12 @@ void launch_conv_tc_list(Context* c, const ConvJob* jobs, int m, cudaStream_t s)
     smem = std::max(smem, tc_layout(t.tc_kpad, t.tc_nd_pad).total + FIDES_TC_SMEM_GUARD);
     bytes += 8.0 * c->N * (t.n_src + t.n_dst);
   }
-  dim3 grid(c->N / TC_M, m);
+  // runs a CTA: as many as leave four waves of seven CTAs an SM
+  int tiles = 1;
+  while (tiles < 8 && (long)(c->N / TC_M) * m / (2 * tiles) >= 4 * 7 * 148) tiles *= 2;
+  dim3 grid(c->N / TC_M / tiles, m);
   LaunchScope ls(c, s, KK_CONV, bytes);
-  launch_pdl(conv_tc_kernel<CAP>, grid, TC_M, smem, s, L, c->d_prime, c->logN, c->d_status);
+  launch_pdl(conv_tc_kernel<CAP>, grid, TC_M, smem, s, L, c->d_prime, c->logN, c->d_status, tiles);
 }
 }  // namespace
 
