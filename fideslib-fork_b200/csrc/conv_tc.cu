@@ -130,23 +130,22 @@ __device__ bool bar_wait_bounded(uint32_t bar, uint32_t phase) {
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&d)[8]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-               : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]), "=r"(d[4]), "=r"(d[5]), "=r"(d[6]), "=r"(d[7])
-               : "r"(taddr));
+// The planes of two destination limbs: 16 columns, waited for.
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&d)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, "
+      "[%16];\n\ttcgen05.wait::ld.sync.aligned;"
+      : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]), "=r"(d[4]), "=r"(d[5]), "=r"(d[6]), "=r"(d[7]), "=r"(d[8]),
+        "=r"(d[9]), "=r"(d[10]), "=r"(d[11]), "=r"(d[12]), "=r"(d[13]), "=r"(d[14]), "=r"(d[15])
+      : "r"(taddr)
+      : "memory");
 }
-__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tc_cp_async8(void* smem, const void* gmem) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_addr(smem)), "l"(gmem) : "memory");
 }
 __device__ __forceinline__ void tc_cp_async16(void* smem, const void* gmem) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(smem)), "l"(gmem) : "memory");
 }
-// Orders later uses of d after tcgen05.wait::ld.
-__device__ __forceinline__ void pin8(uint32_t (&d)[8]) {
-  asm volatile("" : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3]), "+r"(d[4]), "+r"(d[5]), "+r"(d[6]), "+r"(d[7]));
-}
-
 // sum_c 2^(8c) d[c] mod q for planes d[c] < 2^23 and a prime 2^48 < q < 2^62.
 // V = x + 2^32 y with x, y < 2^49 (V < 2^79.01 for K <= 128) is reduced by floating-point
 // Barrett reduction (the double-precision quotient estimate of NTL's MulMod): the integers
@@ -157,49 +156,47 @@ __device__ __forceinline__ void pin8(uint32_t (&d)[8]) {
 // floor(V/q) or one more (qh < 2^32).  V - qh q lies in [-q, q), is computed exactly in
 // wrapping 64-bit arithmetic (nq = -q) and needs one correction.  (Checked against 128-bit arithmetic
 // on 40 M random, extreme and next-to-a-multiple-of-q plane sets over 4000 primes.)
-__device__ __forceinline__ uint64_t tc_fold(const uint32_t (&d)[8], uint64_t nq, double qinv) {
-  constexpr uint64_t EXP52 = 0x4330000000000000ull;
+// Written out in wide multiply-adds: as C++ the same steps took 4 % more of the kernel's time.
+__device__ __forceinline__ uint64_t tc_fold(const uint32_t* d, uint64_t nq, double qinv) {
   const uint32_t a0 = d[0] + (d[1] << 8), a1 = d[2] + (d[3] << 8);  // < 2^32
   const uint32_t a2 = d[4] + (d[5] << 8), a3 = d[6] + (d[7] << 8);
-  const uint64_t x = (uint64_t)a1 * 65536u + (EXP52 | a0);  // 2^52's exponent, planes 0-3 (< 2^49)
-  const uint64_t y = (uint64_t)a3 * 65536u + (EXP52 | a2);  // planes 4-7 (weight 2^32)
+  constexpr uint32_t EXP52 = 0x43300000u;  // upper word of 2^52
+  uint64_t x, y;                           // 2^52's exponent over planes 0-3 and 4-7 (weight 2^32), each < 2^49
+  asm("{.reg .b64 t;\n\tmov.b64 t, {%1, %3};\n\tmad.wide.u32 %0, %2, 65536, t;}" : "=l"(x) : "r"(a0), "r"(a1), "r"(EXP52));
+  asm("{.reg .b64 t;\n\tmov.b64 t, {%1, %3};\n\tmad.wide.u32 %0, %2, 65536, t;}" : "=l"(y) : "r"(a2), "r"(a3), "r"(EXP52));
   const double two52 = 4503599627370496.0;
   const double xd = __longlong_as_double((long long)x) - two52, yd = __longlong_as_double((long long)y) - two52;
   const double vd = fma(yd, 4294967296.0, xd);
   const uint32_t qh = (uint32_t)__double2loint(__dadd_rd(fma(vd, qinv, 0x1p-17), two52));  // floor, < 2^32
-  uint64_t r = x - EXP52 + ((uint64_t)(uint32_t)y << 32) + (uint64_t)qh * nq;
+  // x + 2^32 y + qh nq without the exponent
+  uint64_t r;
+  asm("{.reg .b64 t;\n\t.reg .b32 l, h;\n\t"
+      "mad.wide.u32 t, %1, %2, %4;\n\tmov.b64 {l, h}, t;\n\tmad.lo.u32 h, %1, %3, h;\n\t"
+      "add.u32 h, h, %5;\n\tsub.u32 h, h, %6;\n\tmov.b64 %0, {l, h};}"
+      : "=l"(r)
+      : "r"(qh), "r"((uint32_t)nq), "r"((uint32_t)(nq >> 32)), "l"(x), "r"((uint32_t)y), "r"(EXP52));
   if ((int64_t)r < 0) r -= nq;
   return r;
 }
 
 // Stores the folded outputs of one chunk of NDC destination limbs (8 byte-plane columns each,
-// starting at TMEM address trow).  The TMEM loads of the next pair are in flight while the
-// current pair is folded; tcgen05.wait::ld waits for all of them, so each wait follows the
-// fold of the pair loaded before it.
+// starting at TMEM address trow), two limbs a TMEM load.  (Loading the next pair while one is folded
+// gained nothing: the warps of seven CTAs an SM cover the wait.)
 template <int NDC, bool CHECK>
-__device__ __forceinline__ void tc_epilogue(uint32_t trow, int j0, int nd, const TcDest* dconst, const ConvTable& T,
+__device__ __forceinline__ void tc_epilogue(uint32_t trow, int j0, int nd, const TcDest* dconst, const ConvJob& J,
                                             int logN, uint64_t* out) {
-  uint32_t d[2][2][8];
-  tmem_ld8(trow, d[0][0]);
-  tmem_ld8(trow + 8, d[0][1]);
-  tmem_wait_ld();
 #pragma unroll
   for (int h = 0; h < NDC / 2; ++h) {
-    const int cur = h & 1, nxt = cur ^ 1;
-    if (h + 1 < NDC / 2) {
-      tmem_ld8(trow + 8 * (2 * h + 2), d[nxt][0]);
-      tmem_ld8(trow + 8 * (2 * h + 3), d[nxt][1]);
-    }
+    uint32_t d[16];
+    tmem_ld16(trow + 16 * h, d);
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
-      pin8(d[cur][u]);
       const int j = j0 + 2 * h + u;
       if (!CHECK || j < nd) {
         const TcDest P = dconst[j];
-        out[(size_t)T.dst_pos(j) << logN] = tc_fold(d[cur][u], P.nq, __longlong_as_double((long long)P.qinv));
+        out[(size_t)J.t.dst_pos(j) << logN] = tc_fold(d + 8 * u, P.nq, __longlong_as_double((long long)P.qinv));
       }
     }
-    if (h + 1 < NDC / 2) tmem_wait_ld();
   }
 }
 
@@ -290,15 +287,15 @@ __global__ void __launch_bounds__(TC_M, 7)
       if (c + 1 == nchunks && tile + 1 < tiles) load_a(coef0 + (tile + 1) * TC_M);  // the MMAs have read A
       const int j0 = c * TC_DCHUNK;
       if (ndc == TC_DCHUNK && j0 + TC_DCHUNK <= nd)
-        tc_epilogue<TC_DCHUNK, false>(trow, j0, nd, dconst, T, logN, out);
+        tc_epilogue<TC_DCHUNK, false>(trow, j0, nd, dconst, J, logN, out);
       else if (ndc == 2)
-        tc_epilogue<2, true>(trow, j0, nd, dconst, T, logN, out);
+        tc_epilogue<2, true>(trow, j0, nd, dconst, J, logN, out);
       else if (ndc == 4)
-        tc_epilogue<4, true>(trow, j0, nd, dconst, T, logN, out);
+        tc_epilogue<4, true>(trow, j0, nd, dconst, J, logN, out);
       else if (ndc == 6)
-        tc_epilogue<6, true>(trow, j0, nd, dconst, T, logN, out);
+        tc_epilogue<6, true>(trow, j0, nd, dconst, J, logN, out);
       else
-        tc_epilogue<8, true>(trow, j0, nd, dconst, T, logN, out);
+        tc_epilogue<8, true>(trow, j0, nd, dconst, J, logN, out);
       tc_fence_before();
       __syncthreads();  // TMEM columns are free for the next chunk
       tc_fence_after();
