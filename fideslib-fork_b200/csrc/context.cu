@@ -386,6 +386,7 @@ Context* create_context(int logN, int n_q, int K, int dnum, const uint64_t* prim
           hmd[lift][l] = build_conv(spr, dpr, lift);
         }
       }
+    c->pinv = pinv;
     // ---- the sources' factors, folded into the inverse transforms that precede the conversions
     auto scaled = [&](int prime, uint64_t pre) {
       const uint64_t q = primes[prime];

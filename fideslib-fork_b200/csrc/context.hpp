@@ -105,6 +105,7 @@ struct Context {
   int device = 0;
   int logN = 0, N = 0, n_q = 0, K = 0, dnum = 0, alpha = 0;
   std::vector<uint64_t> primes, psi;
+  std::vector<ShoupConst> pinv;      // [n_q]: P^-1 mod q_j (the host's copy of d_pinv)
 
   // device tables
   DevPrime* d_prime = nullptr;       // [n_q + K]

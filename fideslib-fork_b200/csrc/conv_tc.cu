@@ -14,6 +14,7 @@
 // MMA LBO apart.  A is stored as [K/16][128 rows][16 B], B as [K/16][8 nd_pad rows][16 B].
 #include <algorithm>
 #include <cstring>
+#include <type_traits>
 
 #include "conv_tc.hpp"
 #include "kernels.cuh"
@@ -182,9 +183,10 @@ __device__ __forceinline__ uint64_t tc_fold(const uint32_t* d, uint64_t nq, doub
 // Stores the folded outputs of one chunk of NDC destination limbs (8 byte-plane columns each,
 // starting at TMEM address trow), two limbs a TMEM load.  (Loading the next pair while one is folded
 // gained nothing: the warps of seven CTAs an SM cover the wait.)
-template <int NDC, bool CHECK>
+// TOP: the job's last output becomes (top - v) P^-1 (ConvJob::top).
+template <int NDC, bool CHECK, bool TOP>
 __device__ __forceinline__ void tc_epilogue(uint32_t trow, int j0, int nd, const TcDest* dconst, const ConvJob& J,
-                                            int logN, uint64_t* out) {
+                                            int logN, uint64_t* out, uint64_t top) {
 #pragma unroll
   for (int h = 0; h < NDC / 2; ++h) {
     uint32_t d[16];
@@ -194,7 +196,9 @@ __device__ __forceinline__ void tc_epilogue(uint32_t trow, int j0, int nd, const
       const int j = j0 + 2 * h + u;
       if (!CHECK || j < nd) {
         const TcDest P = dconst[j];
-        out[(size_t)J.t.dst_pos(j) << logN] = tc_fold(d + 8 * u, P.nq, __longlong_as_double((long long)P.qinv));
+        uint64_t v = tc_fold(d + 8 * u, P.nq, __longlong_as_double((long long)P.qinv));
+        if (TOP && j == nd - 1) v = shoup(submod(top, v, 0 - P.nq), J.top_pinv.w, J.top_pinv.ws, 0 - P.nq);
+        out[(size_t)J.t.dst_pos(j) << logN] = v;
       }
     }
   }
@@ -286,16 +290,24 @@ __global__ void __launch_bounds__(TC_M, 7)
       tc_fence_after();
       if (c + 1 == nchunks && tile + 1 < tiles) load_a(coef0 + (tile + 1) * TC_M);  // the MMAs have read A
       const int j0 = c * TC_DCHUNK;
-      if (ndc == TC_DCHUNK && j0 + TC_DCHUNK <= nd)
-        tc_epilogue<TC_DCHUNK, false>(trow, j0, nd, dconst, J, logN, out);
-      else if (ndc == 2)
-        tc_epilogue<2, true>(trow, j0, nd, dconst, J, logN, out);
-      else if (ndc == 4)
-        tc_epilogue<4, true>(trow, j0, nd, dconst, J, logN, out);
-      else if (ndc == 6)
-        tc_epilogue<6, true>(trow, j0, nd, dconst, J, logN, out);
+      auto fold_chunk = [&](auto top_) {
+        constexpr bool TOP = decltype(top_)::value;
+        const uint64_t top = TOP ? J.top[coef0 + tile * TC_M] : 0;
+        if (ndc == TC_DCHUNK && j0 + TC_DCHUNK <= nd)
+          tc_epilogue<TC_DCHUNK, false, TOP>(trow, j0, nd, dconst, J, logN, out, top);
+        else if (ndc == 2)
+          tc_epilogue<2, true, TOP>(trow, j0, nd, dconst, J, logN, out, top);
+        else if (ndc == 4)
+          tc_epilogue<4, true, TOP>(trow, j0, nd, dconst, J, logN, out, top);
+        else if (ndc == 6)
+          tc_epilogue<6, true, TOP>(trow, j0, nd, dconst, J, logN, out, top);
+        else
+          tc_epilogue<8, true, TOP>(trow, j0, nd, dconst, J, logN, out, top);
+      };
+      if (J.top && c + 1 == nchunks)
+        fold_chunk(std::true_type{});
       else
-        tc_epilogue<8, true>(trow, j0, nd, dconst, J, logN, out);
+        fold_chunk(std::false_type{});
       tc_fence_before();
       __syncthreads();  // TMEM columns are free for the next chunk
       tc_fence_after();

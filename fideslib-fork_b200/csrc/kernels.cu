@@ -81,7 +81,13 @@ __global__ void __launch_bounds__(EW_THREADS) conv_kernel(const __grid_constant_
       mac128(a0, lift0, m);
       mac128(a1, lift1, m);
     }
-    *reinterpret_cast<ulonglong2*>(dst + (size_t)dpos[j] * N) = make_ulonglong2(reduce128(a0, p), reduce128(a1, p));
+    uint64_t r0 = reduce128(a0, p), r1 = reduce128(a1, p);
+    if (J.top && j == nd - 1) {
+      const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(J.top + n);
+      r0 = shoup(submod(t.x, r0, p.q), J.top_pinv.w, J.top_pinv.ws, p.q);
+      r1 = shoup(submod(t.y, r1, p.q), J.top_pinv.w, J.top_pinv.ws, p.q);
+    }
+    *reinterpret_cast<ulonglong2*>(dst + (size_t)dpos[j] * N) = make_ulonglong2(r0, r1);
   }
 }
 

@@ -20,6 +20,10 @@ struct ConvJob {
   ConvTable t;
   const uint64_t* src;  // source y_i at src + (t.src0 + i) * N (coefficient domain, ConvTable)
   uint64_t* dst;        // output j at dst + t.dst_pos(j) * N
+  // ModDown before a rescale: the last output v becomes (top - v) top_pinv, the coefficients of the
+  // limb being dropped (top: INTT of that limb of the extended polynomial; top_pinv = P^-1)
+  const uint64_t* top = nullptr;
+  ShoupConst top_pinv{0, 0};
 };
 constexpr int MAX_CONV_JOBS = 96;
 // Job lists are passed by value; launches of a few jobs take the short form (a large parameter block

@@ -39,8 +39,7 @@ void fill_runs(NttLimbList& L, const LimbRef* limbs, int n, size_t N) {
 void ntt_limbs(Context* c, const LimbRef* limbs, int n, bool inverse, cudaStream_t s, NttIn in, NttOut out) {
   if (n <= 0) return;
   if (c->logN < 10) throw Error(-1, "GPU NTT needs logN >= 10");
-  const bool ok = inverse ? ((in == IN_PLAIN || in == IN_MUL || in == IN_ADD_PMUL) &&
-                             (out == OUT_PLAIN || out == OUT_SUB_PINV))
+  const bool ok = inverse ? ((in == IN_PLAIN || in == IN_MUL) && out == OUT_PLAIN)
                           : ((in == IN_PLAIN || in == IN_SWITCH || in == IN_CONV_SW || in == IN_SIGNED) &&
                              (out == OUT_PLAIN || out == OUT_MODDOWN || out == OUT_RESCALE || out == OUT_MDRS));
   if (!ok) throw Error(-1, "NTT prologue/epilogue not available in this direction");

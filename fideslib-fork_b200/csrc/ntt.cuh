@@ -34,16 +34,14 @@ enum NttIn {
   IN_MUL = 1,      // inverse only: x = src[i] * pro[i] mod q   (tensor term a1 b1)
   IN_SWITCH = 2,   // forward only: x = SwitchModulus(pro[i]) from prime aux - 1 (rescale)
   IN_CONV_SW = 3,  // forward only: x = src[i] + P SwitchModulus(pro[i]) from prime aux - 1
-  IN_ADD_PMUL = 4, // inverse only: x = src[i] + P pro[i]
-  IN_SIGNED = 5,   // forward only: x = pro[i] read as a signed 64-bit integer, reduced mod q (encode)
+  IN_SIGNED = 4,   // forward only: x = pro[i] read as a signed 64-bit integer, reduced mod q (encode)
 };
 // What the last pass stores to ptr.
 enum NttOut {
   OUT_PLAIN = 0,
   OUT_MODDOWN = 1,   // forward only: out = (ep0[i] - v) P^-1 (+ ep1[i])     (ModDown finish)
   OUT_RESCALE = 2,   // forward only: out = qinv_l ep0[i] + QlQlInv_l v, l = aux (rescale finish)
-  OUT_MDRS = 3,      // forward only: out = (ep0[i] - v) (P q_(l-1))^-1 (+ q_(l-1)^-1 ep1[i]), l = aux
-  OUT_SUB_PINV = 4,  // inverse only: out = (v - ep0[i]) P^-1
+  OUT_MDRS = 3,      // forward only: out = (ep0[i] - v) (P q_(l-1))^-1, l = aux
 };
 
 // ---- Twiddle tables.  A pass runs the stages of one register chunk (2^le residues per thread) after

@@ -136,7 +136,7 @@ struct PassArgs {
   const InvFinal* inv_fin;     // [prime]: the inverse transform's last stage
   const ShoupConst* pinv;      // [Q prime]: P^-1 mod q (OUT_MODDOWN)
   const RescaleConst* rescale; // [level][Q prime] (OUT_RESCALE, OUT_MDRS)
-  const ShoupConst* pmod;      // [Q prime]: P mod q (IN_CONV_SW, IN_ADD_PMUL)
+  const ShoupConst* pmod;      // [Q prime]: P mod q (IN_CONV_SW)
   const ShoupConst* pqinv;     // [level][Q prime]: (P q_(level-1))^-1 mod q (OUT_MDRS)
   int logN;
   int log1;  // size of the column sub-transform
@@ -455,13 +455,12 @@ __global__ void __launch_bounds__(PassThreads<LOGN, PASS, G, LE>::NT, PassThread
   DevPrime opr;
   if (IN == IN_SWITCH || IN == IN_CONV_SW) opr = a.primes[lr.aux - 1];
   ShoupConst pm{0, 0};
-  if (IN == IN_CONV_SW || IN == IN_ADD_PMUL) pm = a.pmod[lr.prime];
+  if (IN == IN_CONV_SW) pm = a.pmod[lr.prime];
   auto load = [&](size_t i) -> uint64_t {
     if (first_pass && IN == IN_SWITCH) return switch_modulus(lr.pro[i], opr, pr);
     if (first_pass && IN == IN_SIGNED) return signed_mod(lr.pro[i], pr);
     if (first_pass && IN == IN_MUL) return mulmod(in[i], lr.pro[i], pr);
     if (first_pass && IN == IN_CONV_SW) return in[i];  // + P SwitchModulus(top) below
-    if (first_pass && IN == IN_ADD_PMUL) return addmod(in[i], shoup(lr.pro[i], pm.w, pm.ws, pr.q), pr.q);
     return in[i];
   };
   // The prologues and epilogues of FP64 limbs are FP64 products too: with the butterflies at 8.75-9.5
@@ -542,9 +541,9 @@ __global__ void __launch_bounds__(PassThreads<LOGN, PASS, G, LE>::NT, PassThread
   constexpr bool last_pass = !first_pass;
   ShoupConst pinv{0, 0};
   RescaleConst rsc{0, 0, 0, 0};
-  if (OUT == OUT_MODDOWN || OUT == OUT_SUB_PINV) pinv = a.pinv[lr.prime];
+  if (OUT == OUT_MODDOWN) pinv = a.pinv[lr.prime];
   if (OUT == OUT_MDRS) pinv = a.pqinv[(size_t)lr.aux * a.n_q + lr.prime];
-  if (OUT == OUT_RESCALE || OUT == OUT_MDRS) rsc = a.rescale[(size_t)lr.aux * a.n_q + lr.prime];
+  if (OUT == OUT_RESCALE) rsc = a.rescale[(size_t)lr.aux * a.n_q + lr.prime];
   auto ep0 = [&](size_t i) -> uint64_t {
     if constexpr (EPS) return sep[i - (size_t)sub0 * P];
     return lr.ep0[i];
@@ -552,14 +551,9 @@ __global__ void __launch_bounds__(PassThreads<LOGN, PASS, G, LE>::NT, PassThread
   auto finish = [&](size_t i, uint64_t v, uint64_t e0) {
     if (OUT == OUT_MODDOWN || OUT == OUT_MDRS) {
       v = shoup(submod(e0, v, pr.q), pinv.w, pinv.ws, pr.q);
-      if (lr.ep1) {
-        const uint64_t e = lr.ep1[i];
-        v = addmod(v, OUT == OUT_MDRS ? shoup(e, rsc.qinv, rsc.qinv_s, pr.q) : e, pr.q);
-      }
+      if (OUT == OUT_MODDOWN && lr.ep1) v = addmod(v, lr.ep1[i], pr.q);
     } else if (OUT == OUT_RESCALE) {
       v = addmod(shoup(e0, rsc.qinv, rsc.qinv_s, pr.q), shoup(v, rsc.m, rsc.m_s, pr.q), pr.q);
-    } else if (OUT == OUT_SUB_PINV) {
-      v = shoup(submod(v, e0, pr.q), pinv.w, pinv.ws, pr.q);
     }
     data[i] = v;
   };
@@ -570,9 +564,8 @@ __global__ void __launch_bounds__(PassThreads<LOGN, PASS, G, LE>::NT, PassThread
   };
   double f_pinv = 0, f_qinv = 0, f_m = 0, f_q2t = 0;
   if (f64) {
-    if (OUT == OUT_MODDOWN || OUT == OUT_SUB_PINV || OUT == OUT_MDRS) f_pinv = centred(pinv.w);
-    if (OUT == OUT_RESCALE || OUT == OUT_MDRS) f_qinv = centred(rsc.qinv);
-    if (OUT == OUT_RESCALE) f_m = centred(rsc.m);
+    if (OUT == OUT_MODDOWN || OUT == OUT_MDRS) f_pinv = centred(pinv.w);
+    if (OUT == OUT_RESCALE) f_qinv = centred(rsc.qinv), f_m = centred(rsc.m);
     f_q2t = __dadd_rn(2.0 * fp.q, F64_TWO52);
   }
   auto finish_f64 = [&](size_t i, uint64_t b, uint64_t e0) {
@@ -583,14 +576,9 @@ __global__ void __launch_bounds__(PassThreads<LOGN, PASS, G, LE>::NT, PassThread
     double v = __longlong_as_double((long long)b);
     if (OUT == OUT_MODDOWN || OUT == OUT_MDRS) {
       v = f_mulmod(__dsub_rn(f_from_u64(e0), v), f_pinv, fp.q, fp.qinv);  // |e0 - v| < 3q: within 0.875q
-      if (lr.ep1) {
-        const double e = f_from_u64(lr.ep1[i]);
-        v = __dadd_rn(v, OUT == OUT_MDRS ? f_mulmod(e, f_qinv, fp.q, fp.qinv) : e);
-      }
+      if (OUT == OUT_MODDOWN && lr.ep1) v = __dadd_rn(v, f_from_u64(lr.ep1[i]));
     } else if (OUT == OUT_RESCALE) {
       v = __dadd_rn(f_mulmod(f_from_u64(e0), f_qinv, fp.q, fp.qinv), f_mulmod(v, f_m, fp.q, fp.qinv));
-    } else if (OUT == OUT_SUB_PINV) {
-      v = f_mulmod(__dsub_rn(v, f_from_u64(e0)), f_pinv, fp.q, fp.qinv);
     }
     data[i] = f_to_canon(v, f_q2t, pr.q);
   };
@@ -602,24 +590,10 @@ __global__ void __launch_bounds__(PassThreads<LOGN, PASS, G, LE>::NT, PassThread
       if (direct_store) pass_sync<WARP>();  // the staged store below synchronises anyway
     }
     if constexpr (direct_store) {
-      if constexpr (OUT == OUT_SUB_PINV) {
-        // the epilogue loads ahead of the stores: a store may alias the next load's address, and
-        // sixteen load-store round trips in turn took 15.7 us on 2 limbs, where a plain pass takes 4.4
-        constexpr int H = 8;  // in blocks of eight, which the register budget holds
 #pragma unroll
-        for (int r0 = 0; r0 < E; r0 += H) {
-          uint64_t e[H];
-#pragma unroll
-          for (int r = 0; r < H; ++r) e[r] = lr.ep0[gidx(sub, u_of<LOL, LE>(t, r0 + r))];
-#pragma unroll
-          for (int r = 0; r < H; ++r) st(gidx(sub, u_of<LOL, LE>(t, r0 + r)), x[r0 + r], e[r]);
-        }
-      } else {
-#pragma unroll
-        for (int r = 0; r < E; ++r) {
-          const size_t i = gidx(sub, u_of<LOL, LE>(t, r));
-          st(i, x[r], OUT == OUT_PLAIN ? 0 : ep0(i));
-        }
+      for (int r = 0; r < E; ++r) {
+        const size_t i = gidx(sub, u_of<LOL, LE>(t, r));
+        st(i, x[r], OUT == OUT_PLAIN ? 0 : ep0(i));
       }
     } else {
       pass_sync<WARP>();
@@ -765,14 +739,9 @@ void run_transform(Context* c, const PassArgs& a, const NttLimbList& L, bool inv
   } else {
     if (in == IN_MUL)
       launch_pass<LOGN, ROW, false, IN_MUL, OUT_PLAIN>(c, a, L, s);
-    else if (in == IN_ADD_PMUL)
-      launch_pass<LOGN, ROW, false, IN_ADD_PMUL, OUT_PLAIN>(c, a, L, s);
     else
       launch_pass<LOGN, ROW, false, IN_PLAIN, OUT_PLAIN>(c, a, L, s);
-    if (out == OUT_SUB_PINV)
-      launch_pass<LOGN, COL, false, IN_PLAIN, OUT_SUB_PINV>(c, a, L, s);
-    else
-      launch_pass<LOGN, COL, false, IN_PLAIN, OUT_PLAIN>(c, a, L, s);
+    launch_pass<LOGN, COL, false, IN_PLAIN, OUT_PLAIN>(c, a, L, s);
   }
 }
 

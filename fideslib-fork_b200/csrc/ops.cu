@@ -88,21 +88,31 @@ void modup_stage(Context* c, const uint64_t* const* xs, const uint64_t* const* y
 }
 
 // ModDown, first phase: INTT of the special limbs of the extended polys exts[i] (in place)
-// and their conversion to the Q basis into convs[i] (coefficient form).
-void moddown_prep(Context* c, uint64_t* const* exts, const int* ls, uint64_t* const* convs, int n,
+// and their conversion to the Q basis into convs[i] (coefficient form).  The first n_rescaled polys are
+// rescaled afterwards: the limb they drop is transformed along (in place), and the conversion leaves its
+// coefficients (INTT(x_t) - conv_t) P^-1 in the last limb of convs[i] (ConvJob::top).
+void moddown_prep(Context* c, uint64_t* const* exts, const int* ls, uint64_t* const* convs, int n, int n_rescaled,
                   cudaStream_t s) {
   const size_t N = c->N;
   const int K = c->K;
   if (K == 0) throw Error(-1, "ModDown needs special primes");
   std::vector<LimbRef> refs;
-  for (int i = 0; i < n; ++i)
+  for (int i = 0; i < n; ++i) {
+    if (i < n_rescaled) refs.push_back(lref(exts[i] + (ls[i] - 1) * N, ls[i] - 1));
     for (int k = 0; k < K; ++k) {
       refs.push_back(lref(exts[i] + (ls[i] + k) * N, c->n_q + k));
       refs.back().fin = c->moddown_fin + k;  // times (P / p_k)^-1
     }
+  }
   ntt_limbs(c, refs.data(), (int)refs.size(), true, s);
   std::vector<ConvJob> jobs;
-  for (int i = 0; i < n; ++i) jobs.push_back(ConvJob{c->moddown_table(ls[i]), exts[i] + ls[i] * N, convs[i]});
+  for (int i = 0; i < n; ++i) {
+    jobs.push_back(ConvJob{c->moddown_table(ls[i]), exts[i] + ls[i] * N, convs[i]});
+    if (i < n_rescaled) {
+      jobs.back().top = exts[i] + (ls[i] - 1) * N;
+      jobs.back().top_pinv = c->pinv[ls[i] - 1];
+    }
+  }
   launch_conv(c, jobs.data(), (int)jobs.size(), s);
 }
 
@@ -128,64 +138,51 @@ void moddown_finish(Context* c, uint64_t* const* exts, const int* ls, uint64_t* 
 // adding adds[i] when given.
 void moddown_stage(Context* c, uint64_t* const* exts, const int* ls, uint64_t* const* convs, uint64_t* const* outs,
                    const uint64_t* const* adds, int n, cudaStream_t s) {
-  moddown_prep(c, exts, ls, convs, n, s);
+  moddown_prep(c, exts, ls, convs, n, 0, s);
   moddown_finish(c, exts, ls, convs, outs, adds, n, s);
 }
 
-// ModDown fused with the rescale that follows it.  With u = ModDown(x) + add the value
-// being rescaled from level l (top prime q_t = q_(l-1)), linearity of the transforms over
-// Z_q gives, residue for residue:
-//   top   = INTT(u_t) = (INTT(x_t + P add_t) - conv_t) P^-1                (coefficients)
-//   out_j = (x_j - NTT(conv_j + P SwitchModulus(top))) (P q_t)^-1 + q_t^-1 add_j,  j < l - 1
+// ModDown fused with the rescale that follows it.  With u = ModDown(x) the value being rescaled from
+// level l (top prime q_t = q_(l-1)), linearity of the transforms over Z_q gives, residue for residue:
+//   top   = INTT(u_t) = (INTT(x_t) - conv_t) P^-1                      (coefficients, moddown_prep)
+//   out_j = (x_j - NTT(conv_j + P SwitchModulus(top))) (P q_t)^-1,  j < l - 1
 // so the result equals ModDown followed by Rescale (reference: NTT<NTT_MODDOWN> then
 // rescale, src/CKKS/LimbPartitionMGPU.cu:89-232) bit for bit, with one INTT and l - 1 NTTs
 // in place of l NTTs, one INTT and l - 1 NTTs.
-// Second phase of a ModDown fused with the rescale (after moddown_prep): the top limb's INTT
-// and the forward transforms of the other limbs with the conv + P SwitchModulus(top) prologue.
+// Second phase (after moddown_prep): the forward transforms of the other limbs with the
+// conv + P SwitchModulus(top) prologue.
 void moddown_rescale_finish(Context* c, uint64_t* const* exts, const int* ls, uint64_t* const* convs,
-                            uint64_t* const* tops, uint64_t* const* outs, const uint64_t* const* adds, int n,
-                            cudaStream_t s) {
+                            uint64_t* const* outs, int n, cudaStream_t s) {
   const size_t N = c->N;
-  std::vector<LimbRef> top_add, top_plain, fwd;
+  std::vector<LimbRef> fwd;
   for (int i = 0; i < n; ++i) {
     const int l = ls[i];
-    const uint64_t* add = adds ? adds[i] : nullptr;
-    LimbRef t = lref(tops[i], l - 1);
-    t.src = exts[i] + (size_t)(l - 1) * N;
-    t.pro = add ? add + (size_t)(l - 1) * N : nullptr;
-    t.ep0 = convs[i] + (size_t)(l - 1) * N;
-    (add ? top_add : top_plain).push_back(t);
     for (int j = 0; j < l - 1; ++j) {
       LimbRef r = lref(outs[i] + j * N, j);
       r.src = convs[i] + j * N;
-      r.pro = tops[i];
+      r.pro = convs[i] + (size_t)(l - 1) * N;
       r.ep0 = exts[i] + j * N;
-      r.ep1 = add ? add + j * N : nullptr;
       r.aux = l;
       fwd.push_back(r);
     }
   }
-  ntt_limbs(c, top_add.data(), (int)top_add.size(), true, s, IN_ADD_PMUL, OUT_SUB_PINV);
-  ntt_limbs(c, top_plain.data(), (int)top_plain.size(), true, s, IN_PLAIN, OUT_SUB_PINV);
   ntt_limbs(c, fwd.data(), (int)fwd.size(), false, s, IN_CONV_SW, OUT_MDRS);
 }
 
 void moddown_rescale_stage(Context* c, uint64_t* const* exts, const int* ls, uint64_t* const* convs,
-                           uint64_t* const* tops, uint64_t* const* outs, const uint64_t* const* adds, int n,
-                           cudaStream_t s) {
-  moddown_prep(c, exts, ls, convs, n, s);
-  moddown_rescale_finish(c, exts, ls, convs, tops, outs, adds, n, s);
+                           uint64_t* const* outs, int n, cudaStream_t s) {
+  moddown_prep(c, exts, ls, convs, n, n, s);
+  moddown_rescale_finish(c, exts, ls, convs, outs, n, s);
 }
 
-// Scratch limbs of one key switch at level l: INTT copy, digits, A, B, two conversions,
-// two rescale tops.
+// Scratch limbs of one key switch at level l: INTT copy, digits, A, B, two conversions.
 size_t ks_limbs(Context* c, int l) {
   const int ext = l + c->K;
-  return (size_t)l + (size_t)c->beta(l) * ext + 2 * (size_t)ext + 2 * (size_t)l + 2;
+  return (size_t)l + (size_t)c->beta(l) * ext + 2 * (size_t)ext + 2 * (size_t)l;
 }
 
 // Key switch of n items whose inputs are xs[i] (or xs[i] * ys[i]); with `rescale` the
-// outputs f0/f1 (+ add0/add1) are rescaled to level l - 1 in the same ModDown.
+// outputs f0/f1 are rescaled to level l - 1 in the same ModDown (no addends then).
 void keyswitch_stage(Context* c, const uint64_t* const* xs, const uint64_t* const* ys, const int* ls,
                      const uint64_t* const* keys, uint64_t* const* f0, uint64_t* const* f1,
                      const uint64_t* const* add0, const uint64_t* const* add1, int n, cudaStream_t s,
@@ -197,7 +194,7 @@ void keyswitch_stage(Context* c, const uint64_t* const* xs, const uint64_t* cons
   Scratch sc(c, sizeof(uint64_t) * N * total, s);
   Bump bp{sc.u64(), N};
   std::vector<int> ls2(2 * n);
-  std::vector<uint64_t*> tmp(n), dig(n), ex(2 * n), conv(2 * n), outs(2 * n), tops(2 * n);
+  std::vector<uint64_t*> tmp(n), dig(n), ex(2 * n), conv(2 * n), outs(2 * n);
   std::vector<const uint64_t*> adds(2 * n);
   std::vector<KskJob> kj;
   for (int i = 0; i < n; ++i) {
@@ -216,8 +213,6 @@ void keyswitch_stage(Context* c, const uint64_t* const* xs, const uint64_t* cons
     ex[2 * i + 1] = A;
     conv[2 * i] = bp.take(l);
     conv[2 * i + 1] = bp.take(l);
-    tops[2 * i] = bp.take(1);
-    tops[2 * i + 1] = bp.take(1);
     outs[2 * i] = f0[i];
     outs[2 * i + 1] = f1[i];
     adds[2 * i] = add0 ? add0[i] : nullptr;
@@ -227,7 +222,7 @@ void keyswitch_stage(Context* c, const uint64_t* const* xs, const uint64_t* cons
   modup_stage(c, xs, ys, ls, tmp.data(), dig.data(), n, s);
   launch_ksk(c, kj.data(), n, s);
   if (rescale)
-    moddown_rescale_stage(c, ex.data(), ls2.data(), conv.data(), tops.data(), outs.data(), adds.data(), 2 * n, s);
+    moddown_rescale_stage(c, ex.data(), ls2.data(), conv.data(), outs.data(), 2 * n, s);
   else
     moddown_stage(c, ex.data(), ls2.data(), conv.data(), outs.data(), adds.data(), 2 * n, s);
 }
@@ -434,7 +429,7 @@ void op_mixed_batch(Context* c, const HMultItem* hm, int nh, const uint64_t* rel
   const int n = nh + nr;
   std::vector<const uint64_t*> hx(nh), hy(nh), rx(nr);
   std::vector<int> ls(n), ls2(2 * n);
-  std::vector<uint64_t*> tmp(n), dig(n), ex(2 * n), conv(2 * n), tops(2 * n), outs(2 * n);
+  std::vector<uint64_t*> tmp(n), dig(n), ex(2 * n), conv(2 * n), outs(2 * n);
   std::vector<KskJob> kj;
   for (int i = 0; i < n; ++i) {
     const bool mult = i < nh;
@@ -465,18 +460,16 @@ void op_mixed_batch(Context* c, const HMultItem* hm, int nh, const uint64_t* rel
     ex[2 * i + 1] = A;
     conv[2 * i] = bp.take(l);
     conv[2 * i + 1] = bp.take(l);
-    tops[2 * i] = bp.take(1);
-    tops[2 * i + 1] = bp.take(1);
     ls2[2 * i] = ls2[2 * i + 1] = l;
   }
   if (nh) modup_intt(c, hx.data(), hy.data(), ls.data(), tmp.data(), nh, s);
   if (nr) modup_intt(c, rx.data(), nullptr, ls.data() + nh, tmp.data() + nh, nr, s);
   modup_convert(c, ls.data(), tmp.data(), dig.data(), n, s);
   launch_ksk(c, kj.data(), n, s);
-  moddown_prep(c, ex.data(), ls2.data(), conv.data(), 2 * n, s);
+  moddown_prep(c, ex.data(), ls2.data(), conv.data(), 2 * n, rescale ? 2 * nh : 0, s);
   if (nh) {
     if (rescale)
-      moddown_rescale_finish(c, ex.data(), ls2.data(), conv.data(), tops.data(), outs.data(), nullptr, 2 * nh, s);
+      moddown_rescale_finish(c, ex.data(), ls2.data(), conv.data(), outs.data(), 2 * nh, s);
     else
       moddown_finish(c, ex.data(), ls2.data(), conv.data(), outs.data(), nullptr, 2 * nh, s);
   }
@@ -680,16 +673,13 @@ void op_moddown_rescale_batch(Context* c, uint64_t* const* exts, const int* ls, 
   size_t total = 0;
   for (int i = 0; i < n; ++i) {
     check_level(c, ls[i], 2);
-    total += ls[i] + 1;
+    total += ls[i];
   }
   Scratch sc(c, sizeof(uint64_t) * c->N * total, s);
   Bump bp{sc.u64(), (size_t)c->N};
-  std::vector<uint64_t*> conv(n), tops(n);
-  for (int i = 0; i < n; ++i) {
-    conv[i] = bp.take(ls[i]);
-    tops[i] = bp.take(1);
-  }
-  moddown_rescale_stage(c, exts, ls, conv.data(), tops.data(), outs, nullptr, n, s);
+  std::vector<uint64_t*> conv(n);
+  for (int i = 0; i < n; ++i) conv[i] = bp.take(ls[i]);
+  moddown_rescale_stage(c, exts, ls, conv.data(), outs, n, s);
 }
 
 void op_hoisted(Context* c, const HoistItem& it, cudaStream_t s) { op_hoisted_batch(c, &it, 1, s); }

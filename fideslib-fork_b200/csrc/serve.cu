@@ -89,7 +89,7 @@ struct Server {
   size_t request_bytes(const fides_request& r) const {
     const int l = r.level, ext = l + c->K;
     // the scratch of one key switch (ops.cu ks_limbs): INTT copy, digits, the two extended
-    // KSK outputs, two conversions and the two rescale tops; HMult and HRotate need no more
+    // KSK outputs, two conversions, and two limbs over; HMult and HRotate need no more
     const size_t limbs = (size_t)l + (size_t)c->beta(l) * ext + 2 * (size_t)ext + 2 * (size_t)l + 2;
     (void)r.op;
     return limbs * c->limb_bytes();
