@@ -80,9 +80,12 @@ constexpr int tw_sub(int logp, bool fwd, int le) { return tw_off(logp, fwd, le, 
 constexpr size_t tw_table(int logN, bool fwd, int le) {
   return (size_t)tw_sub((logN + 1) / 2, fwd, le) + ((size_t)tw_sub(logN / 2, fwd, le) << ((logN + 1) / 2));
 }
-// Passes with 8 residues per thread exist for these rings (measured faster for small launches at
-// N >= 2^15; smaller rings keep 16 only).
-constexpr bool ntt_has_le3(int logN) { return logN >= 15; }
+// Passes with 8 residues per thread exist for these rings.
+constexpr bool ntt_has_le3(int logN) { return logN >= 12; }
+// At N >= 2^15 the context's tables choose between 16 and 8; below, launches of up to this many limbs
+// take 8: their time is that of one CTA, and its threads then run half the butterflies one after another
+// (one rotation at N = 2^13, level 3: 48 -> 41 us; one product at N = 2^14, level 9: 63 -> 49).
+constexpr int NTT_LE3_SMALL = 32;
 // Start of the table of (direction, le) in a prime's block, and the block's size, in entries.
 constexpr size_t tw_start(int logN, bool fwd, int le) {
   size_t o = 0;

@@ -707,7 +707,7 @@ void launch_pass_le(Context* c, const PassArgs& a, const NttLimbList& L, cudaStr
 template <int LOGN, int PASS, bool FWD, int IN, int OUT>
 void launch_pass(Context* c, const PassArgs& a, const NttLimbList& L, cudaStream_t s) {
   if constexpr (ntt_has_le3(LOGN)) {
-    if (c->ntt_residues(!FWD, PASS, L.n) == 8) {
+    if (LOGN >= 15 ? c->ntt_residues(!FWD, PASS, L.n) == 8 : L.n <= NTT_LE3_SMALL) {
       launch_pass_le<LOGN, PASS, FWD, IN, OUT, 3>(c, a, L, s);
       return;
     }
