@@ -42,7 +42,7 @@ void autotune_ntt(Context* c, float* best_ms) {
   uint8_t saved[2][2][4], saved_r[2][2][4];
   std::copy(&c->ntt_g[0][0][0], &c->ntt_g[0][0][0] + 16, &saved[0][0][0]);
   std::copy(&c->ntt_r[0][0][0], &c->ntt_r[0][0][0] + 16, &saved_r[0][0][0]);
-  const bool r8 = c->logN >= 15;  // passes with 8 residues per thread exist (ntt_impl.cuh HasLe3)
+  const bool r8 = c->logN >= 15;  // the table chooses the residues per thread
   const int saved_chunk = c->ntt_chunk;
   c->ntt_chunk = 0;  // the shapes are timed on unsplit launches
   const bool saved_profiling = c->profiling;

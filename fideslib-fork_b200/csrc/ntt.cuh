@@ -11,9 +11,10 @@
 //   * each thread keeps 2^LE elements in registers (16, or 8 at N >= 2^15 where the
 //     autotuner picks it) and runs LE stages per chunk; chunks exchange through padded
 //     shared memory;
-//   * lazy butterflies with one 64-bit Shoup product each (primes < 2^62): the forward
-//     transform skips every conditional subtraction for q < 2^58 (values stay below 35q)
-//     and uses Harvey's [0, 4q) form otherwise; the inverse tracks a bound B (a multiple
+//   * primes below 2^50 run FP64 butterflies (exact integers in doubles, ntt_impl.cuh), larger ones lazy
+//     butterflies with one 64-bit Shoup product each (primes < 2^62): below 2^61 the forward transform
+//     lets values grow by 4q a stage and subtracts once a chunk, at every second or at every stage, by
+//     the size of q; above it keeps Harvey's [0, 4q) form; the inverse tracks a bound B (a multiple
 //     of q) and subtracts only once B passes 2^62;
 //   * one launch covers any list of limbs (any polynomials, any levels): blockIdx.y
 //     indexes a limb of a list of runs (pointers + prime id) passed by value;
