@@ -208,7 +208,8 @@ __device__ __forceinline__ void tc_epilogue(uint32_t trow, int j0, int nd, const
 // the next run's sources are on their way while the last chunk of the current one is folded.  The kernel
 // is bound by its instructions (issue 67-69 %, FMA-heavy pipe 41 %, DRAM 30 %): with a CTA a run and the
 // sources staged through registers 48 ModUp conversions at N = 2^16, level 30 took 242 us and 32 ModDown
-// conversions 159, now 211 and 156 (136 and 90 at the rate of a copy).
+// conversions 159; 211 and 156 with several runs, 183 and 138 with tc_fold's wide multiply-adds as well
+// (136 and 90 at the rate of a copy).
 template <int CAP>
 __global__ void __launch_bounds__(TC_M, 7)
     conv_tc_kernel(const __grid_constant__ ConvJobListT<CAP> L, const DevPrime* primes, int logN, uint32_t* status,
