@@ -779,6 +779,7 @@ class Context:
         """_scalars of each entry, one row each; integers of 64 bits in one array operation (11 constants
         at 17 limbs take 6 us, 43 one residue at a time)."""
         import numpy as np
+        scalars = list(scalars)
         if all(type(v) is int and -1 << 63 <= v < 1 << 63 for v in scalars):
             q = np.array(self.q[:l], dtype=np.int64)
             return np.remainder(np.array(scalars, dtype=np.int64)[:, None], q).astype(np.uint64)

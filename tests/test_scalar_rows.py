@@ -17,3 +17,14 @@ def test_scalar_rows_match_single_residues():
         want = np.stack([ctx._scalars(v, 4) for v in rows])
         assert got.dtype == want.dtype == np.uint64 and got.flags.c_contiguous
         assert np.array_equal(got, want)
+
+
+def test_scalar_rows_of_any_iterable():
+    """The constants may come from an iterator or a view, which can be walked once or not be indexed."""
+    import fides_b200 as F
+    ctx = SimpleNamespace(q=[(1 << 60) - 93, 12289])
+    ctx._scalars = lambda v, l: F.Context._scalars(ctx, v, l)
+    for rows in ([5, -7, 1 << 40], [5, -(1 << 100)], [[1, 2], 3]):
+        want = np.stack([ctx._scalars(v, 2) for v in rows])
+        for it in (iter(rows), (v for v in rows), map(lambda v: v, rows), dict(enumerate(rows)).values(), tuple(rows)):
+            assert np.array_equal(F.Context._scalar_rows(ctx, it, 2), want)
