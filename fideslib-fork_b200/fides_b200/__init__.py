@@ -780,7 +780,7 @@ class Context:
         at 17 limbs take 6 us, 43 one residue at a time)."""
         import numpy as np
         scalars = list(scalars)
-        if all(type(v) is int and -1 << 63 <= v < 1 << 63 for v in scalars):
+        if scalars and all(type(v) is int and -1 << 63 <= v < 1 << 63 for v in scalars):
             q = np.array(self.q[:l], dtype=np.int64)
             return np.remainder(np.array(scalars, dtype=np.int64)[:, None], q).astype(np.uint64)
         return np.stack([self._scalars(v, l) for v in scalars])

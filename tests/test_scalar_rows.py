@@ -28,3 +28,15 @@ def test_scalar_rows_of_any_iterable():
         want = np.stack([ctx._scalars(v, 2) for v in rows])
         for it in (iter(rows), (v for v in rows), map(lambda v: v, rows), dict(enumerate(rows)).values(), tuple(rows)):
             assert np.array_equal(F.Context._scalar_rows(ctx, it, 2), want)
+
+
+def test_no_constants_are_refused():
+    """The library reads one row of residues per ciphertext: an empty list must not reach it."""
+    import pytest
+
+    import fides_b200 as F
+    ctx = SimpleNamespace(q=[(1 << 60) - 93, 12289])
+    ctx._scalars = lambda v, l: F.Context._scalars(ctx, v, l)
+    for none in ([], (), iter(())):
+        with pytest.raises(ValueError):
+            F.Context._scalar_rows(ctx, none, 2)
