@@ -35,7 +35,9 @@ void launch_pdl(void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, 
   cfg.attrs = &at;
   cfg.numAttrs = 1;
   void* p[] = {const_cast<void*>(static_cast<const void*>(&args))...};
-  FIDES_CUDA(cudaLaunchKernelExC(&cfg, reinterpret_cast<const void*>(kernel), p));
+  const cudaError_t e = cudaLaunchKernelExC(&cfg, reinterpret_cast<const void*>(kernel), p);
+  if (e != cudaSuccess) cudaGetLastError();  // reported here, not by the thread's next check as well
+  FIDES_CUDA(e);
 }
 
 }  // namespace fides

@@ -84,3 +84,34 @@ def test_server_wait_timeout_leaves_ticket_valid(fides):
     for out in outs[1:]:
         assert torch.equal(out.c0, outs[0].c0) and torch.equal(out.c1, outs[0].c1)
     srv.close()
+
+
+def test_a_refused_launch_leaves_no_error_behind(fides):
+    """A launch that the CUDA runtime refuses (here: on the legacy stream, while another stream that
+    synchronises with it is being captured) is reported by its own call alone: neither the runtime's last
+    error nor the library's next call shows it again."""
+    import ctypes
+
+    from fides_b200 import params
+    prm = params.chain(12, 60, 50, 3, 2)
+    ctx = fides.Context(prm.logN, prm.q, prm.p, prm.dnum)
+    a, out = fides.to_device(np.ones((3, prm.N), dtype=np.uint64)), ctx.empty(3)
+    z = torch.ones(1, 4, dtype=torch.complex128, device="cuda")
+    ctx.add_poly(a, a, out=out)
+    ctx.encode(z, 2.0 ** 40, 2)
+    torch.cuda.synchronize()
+    rt = ctypes.CDLL("libcudart.so.12")
+    s, g = ctypes.c_void_p(), ctypes.c_void_p()
+    assert rt.cudaStreamCreate(ctypes.byref(s)) == 0
+    assert rt.cudaStreamBeginCapture(s, 0) == 0
+    try:
+        with pytest.raises(fides.FidesError) as e:
+            ctx.add_poly(a, a, out=out)
+        left = rt.cudaPeekAtLastError()
+    finally:
+        rt.cudaStreamEndCapture(s, ctypes.byref(g))
+        rt.cudaGetLastError()
+        rt.cudaStreamDestroy(s)
+    assert e.value.code == -2 and left == 0
+    ctx.encode(z, 2.0 ** 40, 2)
+    torch.cuda.synchronize()
