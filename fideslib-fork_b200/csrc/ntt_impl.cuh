@@ -385,9 +385,9 @@ struct PassThreads {
   static constexpr int MINB = NT >= TPS ? 1 : (TPS / NT > 32 ? 32 : TPS / NT);
 };
 
-template <int LOGN, int PASS, bool FWD, int IN, int OUT, int G, int LE>
+template <int LOGN, int PASS, bool FWD, int IN, int OUT, int G, int LE, typename List>
 __global__ void __launch_bounds__(PassThreads<LOGN, PASS, G, LE>::NT, PassThreads<LOGN, PASS, G, LE>::MINB)
-    ntt_pass(const PassArgs a, const __grid_constant__ NttLimbList L) {
+    ntt_pass(const PassArgs a, const __grid_constant__ List L) {
   constexpr int LOGP = PassShape<LOGN, PASS>::LOGP;
   constexpr int P = 1 << LOGP, E = 1 << LE, T = P / E, NT = T * G;
   constexpr int NCH = (LOGP + LE - 1) / LE;
@@ -676,36 +676,36 @@ __global__ void __launch_bounds__(PassThreads<LOGN, PASS, G, LE>::NT, PassThread
 }
 
 
-template <int LOGN, int PASS, bool FWD, int IN, int OUT, int G, int LE>
-void launch_pass_g(Context* c, const PassArgs& a, const NttLimbList& L, cudaStream_t s) {
+template <int LOGN, int PASS, bool FWD, int IN, int OUT, int G, int LE, typename List>
+void launch_pass_g(Context* c, const PassArgs& a, const List& L, cudaStream_t s) {
   constexpr int LOGP = PassShape<LOGN, PASS>::LOGP;
   constexpr int P = 1 << LOGP, T = P / (1 << LE);
   constexpr int smem = G * (P + P / (1 << LE)) * (int)sizeof(uint64_t) +
                        (EpStage<PASS, FWD, OUT>::on ? G * P * (int)sizeof(uint64_t) : 0);
   static bool attr_set = false;  // per instantiation; set before first launch
   if (!attr_set) {
-    FIDES_CUDA(cudaFuncSetAttribute(ntt_pass<LOGN, PASS, FWD, IN, OUT, G, LE>,
+    FIDES_CUDA(cudaFuncSetAttribute(ntt_pass<LOGN, PASS, FWD, IN, OUT, G, LE, List>,
                                     cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     attr_set = true;
   }
   dim3 grid(((1 << LOGN) >> LOGP) / G, L.n);
   // algorithmic bytes: half of a transform's read + write of each limb (two passes)
   LaunchScope ls(c, s, KK_NTT, 8.0 * (1 << LOGN) * L.n);
-  launch_pdl(ntt_pass<LOGN, PASS, FWD, IN, OUT, G, LE>, grid, T * G, smem, s, a, L);
+  launch_pdl(ntt_pass<LOGN, PASS, FWD, IN, OUT, G, LE, List>, grid, T * G, smem, s, a, L);
 }
 
 // The pass with the sub-transforms-per-CTA and residues per thread the context's tables pick
 // for this launch.
-template <int LOGN, int PASS, bool FWD, int IN, int OUT, int LE>
-void launch_pass_le(Context* c, const PassArgs& a, const NttLimbList& L, cudaStream_t s) {
+template <int LOGN, int PASS, bool FWD, int IN, int OUT, int LE, typename List>
+void launch_pass_le(Context* c, const PassArgs& a, const List& L, cudaStream_t s) {
   switch (c->ntt_shape(!FWD, PASS, L.n)) {
     case 4: launch_pass_g<LOGN, PASS, FWD, IN, OUT, 4, LE>(c, a, L, s); break;
     case 8: launch_pass_g<LOGN, PASS, FWD, IN, OUT, 8, LE>(c, a, L, s); break;
     default: launch_pass_g<LOGN, PASS, FWD, IN, OUT, 16, LE>(c, a, L, s);
   }
 }
-template <int LOGN, int PASS, bool FWD, int IN, int OUT>
-void launch_pass(Context* c, const PassArgs& a, const NttLimbList& L, cudaStream_t s) {
+template <int LOGN, int PASS, bool FWD, int IN, int OUT, typename List>
+void launch_pass(Context* c, const PassArgs& a, const List& L, cudaStream_t s) {
   if constexpr (ntt_has_le3(LOGN)) {
     if (LOGN >= 15 ? c->ntt_residues(!FWD, PASS, L.n) == 8 : L.n <= NTT_LE3_SMALL) {
       launch_pass_le<LOGN, PASS, FWD, IN, OUT, 3>(c, a, L, s);
@@ -716,8 +716,8 @@ void launch_pass(Context* c, const PassArgs& a, const NttLimbList& L, cudaStream
 }
 
 // The pass sequence of one transform for a given ring dimension.
-template <int LOGN>
-void run_transform(Context* c, const PassArgs& a, const NttLimbList& L, bool inverse, NttIn in, NttOut out,
+template <int LOGN, typename List>
+void run_transform(Context* c, const PassArgs& a, const List& L, bool inverse, NttIn in, NttOut out,
                    cudaStream_t s) {
   if (!inverse) {
     if (in == IN_SWITCH)
@@ -750,6 +750,8 @@ void run_transform(Context* c, const PassArgs& a, const NttLimbList& L, bool inv
 // Defined in ntt_inst_<logN>.cu.
 #define FIDES_NTT_DECL(LN)                                                                                  \
   void ntt_transform_##LN(Context* c, const nttk::PassArgs& a, const NttLimbList& L, bool inverse, NttIn in, \
+                          NttOut out, cudaStream_t s);                                                       \
+  void ntt_transform_##LN(Context* c, const nttk::PassArgs& a, const NttLongList& L, bool inverse, NttIn in, \
                           NttOut out, cudaStream_t s);
 FIDES_NTT_DECL(10)
 FIDES_NTT_DECL(11)

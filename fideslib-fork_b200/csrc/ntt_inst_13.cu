@@ -6,4 +6,8 @@ void ntt_transform_13(Context* c, const nttk::PassArgs& a, const NttLimbList& L,
                        cudaStream_t s) {
   nttk::run_transform<13>(c, a, L, inverse, in, out, s);
 }
+void ntt_transform_13(Context* c, const nttk::PassArgs& a, const NttLongList& L, bool inverse, NttIn in, NttOut out,
+                       cudaStream_t s) {
+  nttk::run_transform<13>(c, a, L, inverse, in, out, s);
+}
 }  // namespace fides

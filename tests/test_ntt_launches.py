@@ -68,3 +68,56 @@ def test_small_ring_products_alone_and_in_a_batch(fides, logN, bits):
     for c, p in zip(cts, rotated):
         s = ctx.rotate(dev(c), rot_d, 3)
         assert eq(p.c0, fides.to_host(s.c0)) and eq(p.c1, fides.to_host(s.c1))
+
+
+@pytest.fixture(scope="module")
+def small(fides):
+    from fides_b200 import params
+    prm = params.chain(12, 60, 50, 3, 2)
+    return prm, fides.Context(prm.logN, prm.q, prm.p, 2)
+
+
+@pytest.mark.parametrize("n", [96, 97, 230, 448, 449])
+def test_limbs_apart_take_one_launch_pair_per_448(fides, small, n):
+    prm, ctx = small
+    x = uniform_limbs(xrng(n), [prm.q[1]] * 2 * n, prm.N)
+    d = fides.to_device(x)
+    before = ctx.launch_count
+    ctx.ntt_limbs([d[2 * i] for i in range(n)], [1] * n)
+    assert ctx.launch_count - before == 2 * -(-n // 448)
+    ctx.ntt_limbs([d[2 * i] for i in range(n)], [1] * n, inverse=True)
+    assert eq(d, x)
+
+
+@pytest.mark.parametrize("call", ["decode", "encode", "rescale", "rotate", "mult"])
+def test_batches_of_more_polynomials_than_96(fides, small, call):
+    """Every prologue and epilogue on a list of more than 96 runs: one item's launches, its results."""
+    import torch
+    prm, ctx = small
+    n, rng = 100, np.random.default_rng(8)
+    ct = lambda l: fides.Ciphertext(*(fides.to_device(uniform_limbs(rng, prm.q[:l], prm.N)) for _ in range(2)))  # noqa: E731
+    key = fides.to_device(np.stack([np.stack([uniform_limbs(rng, prm.q + prm.p, prm.N) for _ in range(2)])
+                                    for _ in range(2)]))
+    polys = lambda cts: [p for c in cts for p in (c.c0, c.c1)]  # noqa: E731
+    cts = [ct(2) for _ in range(n)]
+    z = torch.from_numpy(rng.uniform(-1, 1, (n, 64, 2))).cuda()
+    z = torch.view_as_complex(z)
+    do = {"decode": lambda c, s: list(ctx.decode(torch.stack([x.c0.view(torch.int64) for x in c]).view(torch.uint64),
+                                                 2.0 ** 30)),
+          "encode": lambda c, s: list(ctx.encode(s, 2.0 ** 30, 2)),
+          "rescale": lambda c, s: ctx.rescale_many(polys(c)),
+          "rotate": lambda c, s: polys(ctx.rotate_batch([(x, key, 3) for x in c])),
+          "mult": lambda c, s: polys(ctx.mult_batch([(x, x) for x in c], key))}[call]
+    alone = [p for i in range(n) for p in do(cts[i:i + 1], z[i:i + 1])]
+    before = ctx.launch_count
+    together = do(cts, z)
+    launches = ctx.launch_count - before
+    assert len(alone) == len(together)
+    bits = lambda t: fides.to_host(t) if t.dtype == torch.uint64 else t.cpu().numpy()  # noqa: E731
+    for a, b in zip(alone, together):
+        assert np.array_equal(bits(a), bits(b))
+    before = ctx.launch_count
+    do(cts[:1], z[:1])
+    single = ctx.launch_count - before
+    if call in ("decode", "encode", "rescale"):  # at most 448 limbs in each of their transforms
+        assert launches == single
