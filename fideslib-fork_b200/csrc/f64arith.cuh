@@ -58,17 +58,18 @@ struct F64AccT {
 using F64Acc = F64AccT<false>;
 using F64AccPos = F64AccT<true>;
 
-// A sum of any number of products of two residues: folded after every eight.
+// A sum of any number of products of two residues, eight at first and at most seven after each fold: a
+// fold leaves its residue, below 2^49 + 1 in magnitude, in l, which is exact up to 2^53.  (A third
+// double for the folded part cost eight registers where four sums run, and a CTA an SM.)
 struct F64Sum {
   F64AccPos acc;
-  double done = 0.0;  // within q for each eight terms folded
   __device__ __forceinline__ void mac(double a, double b) { acc.mac(a, b); }
   __device__ __forceinline__ void flush(double w51, double q, double qinv) {
-    done = __dadd_rn(done, f_reduce(acc.fold(w51, q, qinv), q, qinv));
-    acc = F64AccPos{};
+    acc.l = f_reduce(acc.fold(w51, q, qinv), q, qinv);
+    acc.h = F64AccPos::H0;
   }
   __device__ __forceinline__ uint64_t residue(double w51, double q, double qinv) const {
-    return f_canon(__dadd_rn(done, acc.fold(w51, q, qinv)), q, qinv);
+    return f_canon(acc.fold(w51, q, qinv), q, qinv);
   }
 };
 

@@ -527,11 +527,13 @@ __global__ void __launch_bounds__(EW_THREADS) scalar_kernel(const __grid_constan
 // 2^128 before a reduction.
 constexpr int LC_BLOCK = 4;  // terms per block of loads (lincomb_kernel, dot_plain_kernel)
 
-__global__ void __launch_bounds__(EW_THREADS) dot_plain_kernel(const __grid_constant__ DotJob J,
-                                                               const DevPrime* primes, const F64Prime* f64, int logN) {
+// Memory bounds it, so warps in flight decide: with 114 registers (two CTAs an SM) 11 terms of 24 limbs at
+// N = 2^16 took 54.8 us on 50-bit primes and 62 on 55-bit ones, with 80 (three) 39.2 and 51.
+__global__ void __launch_bounds__(EW_THREADS, 3)
+    dot_plain_kernel(const __grid_constant__ DotJob J, const DevPrime* primes, const F64Prime* f64, int logN) {
   const int lane = blockIdx.x, j = blockIdx.z;
   const int pid = ext_prime(j, J.lq, J.nq);
-  const DevPrime p = primes[pid];
+  const uint64_t q = primes[pid].q;
   const size_t off = ((size_t)j << logN) + 2 * (blockIdx.y * blockDim.x + threadIdx.x);
   pdl_wait();
   auto ld2 = [](const uint64_t* q) { return *reinterpret_cast<const ulonglong2*>(q); };
@@ -545,15 +547,16 @@ __global__ void __launch_bounds__(EW_THREADS) dot_plain_kernel(const __grid_cons
         y[u] = ld2(J.c1[lane][t0 + u] + off);
       }
   };
+  load(0);  // before the form is known: the prime's load would hold these up
   ulonglong2 r0, r1;
-  if (p.q < NTT_F64_MAX) {
+  if (q < NTT_F64_MAX) {
     const F64Prime fp = f64[pid];
     F64Sum a0, a1, b0, b1;
     for (int t0 = 0; t0 < J.n; t0 += LC_BLOCK) {
-      if (t0 && t0 % 8 == 0)
+      if (t0) load(t0);
+      if (t0 >= 8)  // F64Sum: eight terms, then a block a fold
         a0.flush(fp.w51, fp.q, fp.qinv), a1.flush(fp.w51, fp.q, fp.qinv), b0.flush(fp.w51, fp.q, fp.qinv),
             b1.flush(fp.w51, fp.q, fp.qinv);
-      load(t0);
 #pragma unroll
       for (int u = 0; u < LC_BLOCK; ++u)
         if (t0 + u < J.n) {
@@ -567,6 +570,7 @@ __global__ void __launch_bounds__(EW_THREADS) dot_plain_kernel(const __grid_cons
     r0 = make_ulonglong2(a0.residue(fp.w51, fp.q, fp.qinv), a1.residue(fp.w51, fp.q, fp.qinv));
     r1 = make_ulonglong2(b0.residue(fp.w51, fp.q, fp.qinv), b1.residue(fp.w51, fp.q, fp.qinv));
   } else {
+    const DevPrime p = primes[pid];
     U128 a0{0, 0}, a1{0, 0}, b0{0, 0}, b1{0, 0};
     for (int t0 = 0; t0 < J.n; t0 += LC_BLOCK) {
       if (t0 && t0 % 12 == 0) {
@@ -575,7 +579,7 @@ __global__ void __launch_bounds__(EW_THREADS) dot_plain_kernel(const __grid_cons
         b0 = U128{reduce128(b0, p), 0};
         b1 = U128{reduce128(b1, p), 0};
       }
-      load(t0);
+      if (t0) load(t0);
 #pragma unroll
       for (int u = 0; u < LC_BLOCK; ++u)
         if (t0 + u < J.n) {
@@ -620,7 +624,7 @@ __global__ void __launch_bounds__(EW_THREADS) bsgs_dot_kernel(const __grid_const
     F64Sum s0, s1;
 #pragma unroll
     for (int k = 0; k < NB; ++k) {
-      if (k == 8) {
+      if (k == 8 || (k == 15 && k < J.nb)) {
         s0.flush(fp.w51, fp.q, fp.qinv);
         s1.flush(fp.w51, fp.q, fp.qinv);
       }
@@ -703,11 +707,13 @@ __global__ void __launch_bounds__(EW_THREADS) bsgs_dot2_kernel(const __grid_cons
   *reinterpret_cast<ulonglong2*>(J.out1[lane][i] + off) = ulonglong2{reduce128(s1x, p), reduce128(s1y, p)};
 }
 
-__global__ void __launch_bounds__(EW_THREADS) lincomb_kernel(const __grid_constant__ LinCombJob J,
-                                                             const DevPrime* primes, const F64Prime* f64, int logN) {
+// As dot_plain_kernel: 78 registers (three CTAs an SM) 41.3 us on 50-bit primes and 50.2 on 55-bit ones for
+// 11 terms of 24 limbs, 64 (four) 36.9 and 46.5.
+__global__ void __launch_bounds__(EW_THREADS, 4)
+    lincomb_kernel(const __grid_constant__ LinCombJob J, const DevPrime* primes, const F64Prime* f64, int logN) {
   const int j = blockIdx.y, lane = blockIdx.z;
   const int pid = ext_prime(j, J.lq, J.nq);
-  const DevPrime p = primes[pid];
+  const uint64_t q = primes[pid].q;
   const size_t off = ((size_t)j << logN) + 2 * (blockIdx.x * blockDim.x + threadIdx.x);
   pdl_wait();
   auto ld2 = [](const uint64_t* q) { return *reinterpret_cast<const ulonglong2*>(q); };
@@ -723,15 +729,20 @@ __global__ void __launch_bounds__(EW_THREADS) lincomb_kernel(const __grid_consta
         y[u] = ld2(J.x1[lane][t0 + u] + off);
       }
   };
-  ulonglong2 r0, r1;
-  if (p.q < NTT_F64_MAX) {
+  auto store = [&](ulonglong2 r0, ulonglong2 r1) {
+    const uint64_t ad = J.add0[j];
+    *reinterpret_cast<ulonglong2*>(J.out0[lane] + off) = make_ulonglong2(addmod(r0.x, ad, q), addmod(r0.y, ad, q));
+    *reinterpret_cast<ulonglong2*>(J.out1[lane] + off) = r1;
+  };
+  load(0);  // before the form is known: the prime's load would hold these up
+  if (q < NTT_F64_MAX) {
     const F64Prime fp = f64[pid];
     F64Sum a0, a1, b0, b1;
     for (int t0 = 0; t0 < J.n; t0 += LC_BLOCK) {
-      if (t0 && t0 % 8 == 0)
+      if (t0) load(t0);
+      if (t0 >= 8)  // F64Sum: eight terms, then a block a fold
         a0.flush(fp.w51, fp.q, fp.qinv), a1.flush(fp.w51, fp.q, fp.qinv), b0.flush(fp.w51, fp.q, fp.qinv),
             b1.flush(fp.w51, fp.q, fp.qinv);
-      load(t0);
 #pragma unroll
       for (int u = 0; u < LC_BLOCK; ++u)
         if (t0 + u < J.n) {
@@ -742,9 +753,10 @@ __global__ void __launch_bounds__(EW_THREADS) lincomb_kernel(const __grid_consta
           b1.mac(w, f_from_u64(y[u].y));
         }
     }
-    r0 = make_ulonglong2(a0.residue(fp.w51, fp.q, fp.qinv), a1.residue(fp.w51, fp.q, fp.qinv));
-    r1 = make_ulonglong2(b0.residue(fp.w51, fp.q, fp.qinv), b1.residue(fp.w51, fp.q, fp.qinv));
+    store(make_ulonglong2(a0.residue(fp.w51, fp.q, fp.qinv), a1.residue(fp.w51, fp.q, fp.qinv)),
+          make_ulonglong2(b0.residue(fp.w51, fp.q, fp.qinv), b1.residue(fp.w51, fp.q, fp.qinv)));
   } else {
+    const DevPrime p = primes[pid];
     U128 a0{0, 0}, a1{0, 0}, b0{0, 0}, b1{0, 0};
     for (int t0 = 0; t0 < J.n; t0 += LC_BLOCK) {
       if (t0 && t0 % 12 == 0) {
@@ -753,7 +765,7 @@ __global__ void __launch_bounds__(EW_THREADS) lincomb_kernel(const __grid_consta
         b0 = U128{reduce128(b0, p), 0};
         b1 = U128{reduce128(b1, p), 0};
       }
-      load(t0);
+      if (t0) load(t0);
 #pragma unroll
       for (int u = 0; u < LC_BLOCK; ++u)
         if (t0 + u < J.n) {
@@ -764,13 +776,8 @@ __global__ void __launch_bounds__(EW_THREADS) lincomb_kernel(const __grid_consta
           mac128(b1, w, y[u].y);
         }
     }
-    r0 = make_ulonglong2(reduce128(a0, p), reduce128(a1, p));
-    r1 = make_ulonglong2(reduce128(b0, p), reduce128(b1, p));
+    store(make_ulonglong2(reduce128(a0, p), reduce128(a1, p)), make_ulonglong2(reduce128(b0, p), reduce128(b1, p)));
   }
-  const uint64_t ad = J.add0[j];
-  *reinterpret_cast<ulonglong2*>(J.out0[lane] + off) =
-      make_ulonglong2(addmod(r0.x, ad, p.q), addmod(r0.y, ad, p.q));
-  *reinterpret_cast<ulonglong2*>(J.out1[lane] + off) = r1;
 }
 
 template <typename List, typename Job>

@@ -162,3 +162,48 @@ def test_inner_product_is_exact():
                 want += a * int(p)
             s = acc.fold(q, qinv)
             assert abs(s) < 2.0 ** 53 and canon(s, qd, qinv) == want % q
+
+
+class Sum(Acc):
+    """F64Sum over F64AccPos (csrc/f64arith.cuh)."""
+    H0 = 2.0 ** 103
+
+    def fold(self, q, qinv):
+        l, self.l = self.l, 0.0
+        r = super().fold(q, qinv) + f_reduce(l, float(q), qinv)
+        self.l = l
+        return r
+
+    def flush(self, q, qinv):
+        self.l, self.h = f_reduce(self.fold(q, qinv), float(q), qinv), self.H0
+
+
+def f_reduce(x, q, qinv):
+    return fma(-(fma(x, qinv, RND) - RND), q, x)
+
+
+@pytest.mark.parametrize("block", [4, 7])
+def test_long_sums_are_exact(block):
+    """Sums of residue products folded after the first eight terms and then after every `block` (4 in
+    dot_plain and lincomb, 7 in the BSGS sums), at the largest residues and at products whose low parts
+    lie half an ulp of h from it, all on one side."""
+    rng = random.Random(block)
+    for q in primes()[:6] + [(1 << 50) - 27]:
+        qd, qinv = float(q), 1.0 / q
+        for it in range(60):
+            acc, want, rest = Sum(), 0, 8
+            for t in range(40):
+                if not rest:
+                    acc.flush(q, qinv)
+                    assert abs(acc.l) <= 2.0 ** 49 + 1
+                    rest = block
+                a, b = rng.choice([(q - 1, q - 1), (rng.randrange(q), rng.randrange(q)), (0, q - 1)])
+                if it % 2 and q > 1 << 49:  # ab = 2^50 - r modulo 2^51, r small
+                    a = rng.randrange(q // 2, q - 1) | 1
+                    b = min(((1 << 50) - rng.randrange(3)) * pow(a, -1, 1 << 51) % (1 << 51), q - 1)
+                acc.mac(float(a), float(b))
+                assert abs(acc.l) <= 2.0 ** 53
+                want += a * b
+                rest -= 1
+            s = acc.fold(q, qinv)
+            assert abs(s) < 2.0 ** 53 and canon(s, qd, qinv) == want % q
