@@ -142,7 +142,8 @@ struct Context {
   int ntt_chunk = 0;
   int ntt_shape(bool inverse, int pass, int limbs) const { return ntt_g[inverse][pass][ntt_size_class(limbs)]; }
   // Residues per thread (16 or 8) of each pass, indexed like ntt_g.  The table
-  // decides at N >= 2^15 only (below, NTT_LE3_SMALL does); 16 by default, fides_ctx_autotune times both.
+  // decides at N >= 2^15 only (below, NTT_LE3_SMALL does), and not for rescales above 2^50 (ntt.cuh); 16 by
+  // default, fides_ctx_autotune times both.
   uint8_t ntt_r[2][2][4] = {{{16, 16, 16, 16}, {16, 16, 16, 16}}, {{16, 16, 16, 16}, {16, 16, 16, 16}}};
   int ntt_residues(bool inverse, int pass, int limbs) const { return ntt_r[inverse][pass][ntt_size_class(limbs)]; }
   uint32_t* d_status = nullptr;  // device word: bit 0 = a bounded device wait gave up,

@@ -63,6 +63,7 @@ void ntt_limbs(Context* c, const LimbRef* limbs, int n, bool inverse, cudaStream
     for (int i = 0; i < n; ++i) nf += c->primes[limbs[i].prime] < NTT_F64_MAX;
     c->ntt_limbs_by_form[0] += nf;
     c->ntt_limbs_by_form[1] += (uint64_t)n - nf;
+    a.wide = 2 * nf < (uint64_t)n;
   }
   auto launch = [&](const auto& list) {
     switch (c->logN) {

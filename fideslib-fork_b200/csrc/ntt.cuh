@@ -88,6 +88,10 @@ constexpr bool ntt_has_le3(int logN) { return logN >= 12; }
 // take 8: their time is that of one CTA, and its threads then run half the butterflies one after another
 // (one rotation at N = 2^13, level 3: 48 -> 41 us; one product at N = 2^14, level 9: 63 -> 49).
 constexpr int NTT_LE3_SMALL = 32;
+// A row pass with the rescale epilogue takes 8 at N >= 2^15 whatever the tables say where most limbs are of
+// primes above 2^50: its two integer products a residue are a chain that only more warps hide (16 rescales of
+// 24 limbs at N = 2^16 414-418 us with 16, 380 with 8; a plain transform 292 and 296, FP64 limbs 220 and 240,
+// so the tables, timed on plain transforms, would choose 16).
 // Start of the table of (direction, le) in a prime's block, and the block's size, in entries.
 constexpr size_t tw_start(int logN, bool fwd, int le) {
   size_t o = 0;

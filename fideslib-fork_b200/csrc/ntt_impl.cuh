@@ -141,6 +141,7 @@ struct PassArgs {
   int logN;
   int log1;  // size of the column sub-transform
   int n_q;
+  bool wide;  // most of the limbs are of primes above 2^50
 };
 
 // Element index u of register r for thread t, when the register index spans bits
@@ -552,7 +553,7 @@ __global__ void __launch_bounds__(PassThreads<LOGN, PASS, G, LE>::NT, PassThread
     if (OUT == OUT_MODDOWN || OUT == OUT_MDRS) {
       v = shoup(submod(e0, v, pr.q), pinv.w, pinv.ws, pr.q);
       if (OUT == OUT_MODDOWN && lr.ep1) v = addmod(v, lr.ep1[i], pr.q);
-    } else if (OUT == OUT_RESCALE) {
+    } else if (OUT == OUT_RESCALE) {  // v: any 64 bits, not reduced yet
       v = addmod(shoup(e0, rsc.qinv, rsc.qinv_s, pr.q), shoup(v, rsc.m, rsc.m_s, pr.q), pr.q);
     }
     data[i] = v;
@@ -662,8 +663,8 @@ __global__ void __launch_bounds__(PassThreads<LOGN, PASS, G, LE>::NT, PassThread
   else
     chunks<LE, LOGP, PASS, FWD, false, WARP>(x, sm, sidx, g, t, tw, pr, fin, B, direct_load && !STAGE_PRO, pol);
 
-  // ---- final reduction of the completed transform
-  if (FWD && PASS == ROW) {
+  // ---- final reduction of the completed transform (the rescale's products take its place)
+  if (FWD && PASS == ROW && OUT != OUT_RESCALE) {
     if (lazy4) {
 #pragma unroll
       for (int r = 0; r < E; ++r) x[r] = shoup(x[r], 1, pr.one_s, pr.q);  // any 64-bit x
@@ -707,7 +708,8 @@ void launch_pass_le(Context* c, const PassArgs& a, const List& L, cudaStream_t s
 template <int LOGN, int PASS, bool FWD, int IN, int OUT, typename List>
 void launch_pass(Context* c, const PassArgs& a, const List& L, cudaStream_t s) {
   if constexpr (ntt_has_le3(LOGN)) {
-    if (LOGN >= 15 ? c->ntt_residues(!FWD, PASS, L.n) == 8 : L.n <= NTT_LE3_SMALL) {
+    const bool wide_rescale = OUT == OUT_RESCALE && a.wide;
+    if (LOGN >= 15 ? wide_rescale || c->ntt_residues(!FWD, PASS, L.n) == 8 : L.n <= NTT_LE3_SMALL) {
       launch_pass_le<LOGN, PASS, FWD, IN, OUT, 3>(c, a, L, s);
       return;
     }

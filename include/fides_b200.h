@@ -104,8 +104,9 @@ int fides_ctx_ntt_chunk(fides_ctx* ctx, int set_limbs);
 int fides_ctx_ntt_shapes(fides_ctx* ctx, uint8_t* shapes);
 int fides_ctx_set_ntt_shape(fides_ctx* ctx, int inverse, int pass, int size_class, int subs_per_cta);
 /* Residues per thread of each pass (16, or 8 = three butterfly stages per register chunk and
- * twice the threads; settable for N >= 2^15, smaller rings choose by the launch's size), in the
- * same [inverse][pass][size class] layout;
+ * twice the threads; settable for N >= 2^15, smaller rings choose by the launch's size, and the
+ * row pass of a rescale takes 8 where most of its primes are above 2^50), in the same
+ * [inverse][pass][size class] layout;
  * fides_ctx_autotune times both with every shape.  Results never depend on them.  The
  * reference's counterpart is its fixed per-thread radix (src/NTT.cu:331-756). */
 int fides_ctx_ntt_residues(fides_ctx* ctx, uint8_t* residues);
