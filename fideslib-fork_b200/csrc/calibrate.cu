@@ -11,7 +11,8 @@ constexpr int CAL_E = 16;  // values per thread, as in the NTT passes
 
 // Every thread runs `rounds` x 4 stages x 8 butterflies on 16 register values, each
 // stage with its own twiddle (held in registers), and writes one checksum word so the
-// work cannot be elided.  Values wrap modulo 2^64: only the instruction stream matters.
+// work cannot be elided.  One stage of four brings x back below 16q first, as a pass's chunk does
+// for primes below 2^59 (Lazy4Red; larger primes do so at every second stage or at each).
 __global__ void __launch_bounds__(CAL_THREADS) bf_peak_kernel(uint64_t* out, uint64_t q, ShoupConst w0,
                                                              ShoupConst w1, ShoupConst w2, ShoupConst w3,
                                                              int rounds) {
@@ -25,7 +26,10 @@ __global__ void __launch_bounds__(CAL_THREADS) bf_peak_kernel(uint64_t* out, uin
       const ShoupConst w = b == 3 ? w0 : b == 2 ? w1 : b == 1 ? w2 : w3;
 #pragma unroll
       for (int r = 0; r < CAL_E; ++r)
-        if (!(r & (1 << b))) nttk::ct_bf4(x[r], x[r | (1 << b)], w, q, 4 * q);
+        if (!(r & (1 << b))) {
+          if (b == 3) x[r] = csub(x[r], 16 * q);
+          nttk::ct_bf4(x[r], x[r | (1 << b)], w, q, 4 * q);
+        }
     }
   }
   uint64_t s = 0;
@@ -104,7 +108,7 @@ double measure_bf_peak(int device) {
   int sms = 0;
   FIDES_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
   const int blocks = sms * 8;
-  const uint64_t q = (1ull << 50) - (1ull << 17) + 1;  // any odd modulus below 2^58
+  const uint64_t q = (1ull << 50) - (1ull << 17) + 1;  // any odd modulus below 2^59
   auto sc = [&](uint64_t w) { return h_shoup(w % q, q); };
   uint64_t* out = nullptr;
   cudaStream_t st = nullptr;

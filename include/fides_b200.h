@@ -112,8 +112,8 @@ int fides_ctx_set_ntt_shape(fides_ctx* ctx, int inverse, int pass, int size_clas
 int fides_ctx_ntt_residues(fides_ctx* ctx, uint8_t* residues);
 int fides_ctx_set_ntt_residues(fides_ctx* ctx, int inverse, int pass, int size_class, int residues_per_thread);
 /* Compute roofline of the NTT: butterflies per second that `device` sustains running the
- * forward NTT butterfly (one 64-bit Shoup product, two 64-bit additions) on register-resident
- * data, with no memory traffic.  Takes about 100 ms.  No reference counterpart. */
+ * forward NTT butterfly (one 64-bit Shoup product, two 64-bit additions, one conditional
+ * subtraction in four stages) on register-resident data, with no memory traffic.  Takes about 100 ms.  No reference counterpart. */
 int fides_int_peak(int device, double* butterflies_per_s);
 /* The same for the FP64 butterfly the NTT uses for primes below 2^50 (its FP64-pipe
  * roofline).  No reference counterpart. */
