@@ -5,11 +5,10 @@ bounds; these tests replay the same operation sequences in Python (IEEE doubles,
 fused multiply-add through rational arithmetic) on random and extreme operands, and compare
 with exact integer arithmetic:
 
-* the NTT butterfly product for primes below 2^50 (`f_mulmod`, `f_reduce`,
-  fideslib-fork_b200/csrc/ntt_impl.cuh), the row passes' twiddle w recovered from its stored
-  w / q, and the first stage of a transform on uncentred inputs in [0, q);
-* the key-switch inner product's data x data product and final reduction (`ksk_mul_f64`,
-  `ksk_canon_f64`, csrc/kernels.cu);
+* the NTT's prologues and epilogues on FP64 limbs (primes below 2^50, csrc/ntt_impl.cuh): products by
+  `f_mulmod`, `f_reduce` (csrc/f64arith.cuh), the signed coefficients of the encoder (`signed_f64`), the
+  canonical residue of a result (`f_to_canon`), and the first stage on uncentred inputs in [0, q).  The
+  butterflies' bounds and the sums of products are in test_ntt_fp64_bounds.py;
 * the tensor-core conversion's fold of eight s32 byte planes with a one-sided quotient
   correction (`tc_fold`, csrc/conv_tc.cu).
 """
@@ -37,10 +36,10 @@ def primes50():
     return [q for q in params.config_c(4).q if q < (1 << 50)]
 
 
-def f_mulmod(y, w, wq, q):
+def f_mulmod(y, w, q, qinv):
     p = y * w
     e = fma(y, w, -p)
-    k = fma(y, wq, RND) - RND
+    k = fma(p, qinv, RND) - RND
     return fma(-k, q, p) + e
 
 
@@ -48,100 +47,84 @@ def f_reduce(x, q, qinv):
     return fma(-(fma(x, qinv, RND) - RND), q, x)
 
 
-def test_ntt_fp64_butterfly_product_is_exact():
+def centred(w, q):
+    return float(w - q if w > q // 2 else w)
+
+
+def f_to_canon(v, q):
+    u = int(Fraction(v + (2.0 * q + TWO52))) & ((1 << 52) - 1)
+    u = u - 2 * q if u >= 2 * q else u
+    return u - q if u >= q else u
+
+
+def all_primes():
+    from fides_b200 import params
+    return primes50()[:5] + params.gen_primes(12, 34, 1) + params.gen_primes(12, 30, 1) + [(1 << 50) - 27, 12289]
+
+
+def exact(v, ref, q, bound):
+    """v is an integer congruent to ref within `bound`."""
+    assert v == int(v) and (int(v) - ref) % q == 0 and abs(v) <= bound + 1
+
+
+def test_prologues():
+    """Inputs of a transform's first stage: within 4q forward, within q inverse."""
     rng = random.Random(11)
-    qs = primes50()
-    for q in qs[:6] + qs[-3:]:
+    for q in all_primes():
         qd, qinv = float(q), 1.0 / q
-        for it in range(400):
-            w = rng.randrange(1, q)
-            wq = float(Fraction(w, q))
-            bound = int(1.9 * q) if it % 4 else q
-            y = rng.randrange(-bound, bound + 1)
-            if it % 50 == 0:
-                y = bound
-            r = f_mulmod(float(y), float(w), wq, qd)
-            assert r == int(r)
-            r = int(r)
-            assert (r - y * w) % q == 0
-            assert abs(r) <= q * (0.5 + abs(y) * 2.0 ** -53) + 1
-            # alternate-stage reduction of the other operand
-            x = rng.randrange(-2 * q + 1, 2 * q)
-            xr = f_reduce(float(x), qd, qinv)
-            assert (int(xr) - x) % q == 0 and abs(xr) <= q / 2 + 1
+        pick = lambda: rng.choice([rng.randrange(q), q - 1, 0, q // 2])  # noqa: E731
+        for it in range(200):
+            a, b = pick(), pick()  # the tensor term a1 b1
+            exact(f_mulmod(float(a), float(b), qd, qinv), a * b, q, 0.75 * q)
+            # the centred lift of a residue of any other prime below 2^50, and P times it beside the
+            # conversion's value
+            c = rng.choice([rng.randrange(-(1 << 49), (1 << 49) + 1), 1 << 49, -(1 << 49)])
+            exact(f_reduce(float(c), qd, qinv), c, q, q / 2)
+            P, x = rng.randrange(q), pick()
+            exact(float(x) + f_mulmod(float(c), centred(P, q), qd, qinv), x + c * P, q, 2 * q)
+            exact(float(x) + f_mulmod(float(a), centred(P, q), qd, qinv), x + a * P, q, 2 * q)
+            if q >= 1 << 33:  # signed_f64: the upper word's part reduced, the lower word as it is
+                m = rng.choice([rng.randrange(-(1 << 63), 1 << 63), (1 << 63) - 1, -(1 << 63), -1,
+                                rng.randrange(-(1 << 45), 1 << 45)])
+                hi = f_reduce(float((m >> 32) << 32), qd, qinv)
+                exact(hi + float(m & 0xffffffff), m, q, q)
 
 
-def test_row_twiddle_recovered_from_quotient():
-    """Row passes store the correctly rounded w / q and recover w = fma(w / q, q, RND) - RND."""
+def test_epilogues():
+    """Results of a transform, within 2q, through the epilogues to canonical residues."""
     rng = random.Random(12)
-    for q in primes50() + [(1 << 50) - 27, 12289]:
-        qd = float(q)
-        ws = [rng.randrange(1, q) for _ in range(300)] + [1, 2, q - 1, q - 2, q // 2]
-        for w in ws:
-            wq = w / q  # correctly rounded, as the host builds the table
-            assert wq == float(Fraction(w, q))
-            assert fma(wq, qd, RND) - RND == float(w)
+    for q in all_primes():
+        qd, qinv = float(q), 1.0 / q
+        pick = lambda: rng.choice([rng.randrange(q), q - 1, 0])  # noqa: E731
+        for it in range(200):
+            v = rng.choice([rng.randrange(-2 * q + 1, 2 * q), 2 * q - 1, -2 * q + 1, 0])
+            assert f_to_canon(float(v), qd) == v % q
+            e0, e1, w, m = pick(), pick(), pick(), pick()
+            down = f_mulmod(float(e0) - float(v), centred(w, q), qd, qinv)  # ModDown, and with a rescale
+            exact(down, (e0 - v) * w, q, 0.875 * q)
+            assert f_to_canon(down, qd) == (e0 - v) * w % q
+            assert f_to_canon(down + float(e1), qd) == ((e0 - v) * w + e1) % q
+            scaled = f_mulmod(float(e0), centred(w, q), qd, qinv) + f_mulmod(float(v), centred(m, q), qd, qinv)
+            exact(scaled, e0 * w + v * m, q, 1.5 * q)
+            assert f_to_canon(scaled, qd) == (e0 * w + v * m) % q
 
 
 def test_first_stage_on_uncentred_inputs():
-    """The first pass converts canonical residues in [0, q) without centring them: the
-    forward first stage reduces its x operand and multiplies y < q; the inverse first stage
-    reduces the sum (< 2q) and multiplies the difference (|d| < q).  Both stay exact and leave
-    the bounds the later stages assume (forward: |x +- r| <= 1.125 q + 1; inverse: q / 2 + 1)."""
+    """The first pass converts canonical residues in [0, q) without centring them: the forward first stage
+    reduces its x operand and multiplies y < q; the inverse first stage adds (< 2q) and multiplies the
+    difference (|d| < q).  Both stay exact within the bounds the later stages assume."""
     rng = random.Random(13)
-    for q in primes50()[:4] + [(1 << 50) - 27]:
+    for q in all_primes():
         qd, qinv = float(q), 1.0 / q
         for it in range(300):
-            w = rng.randrange(1, q)
-            wq = w / q
+            w = rng.randrange(-(q // 2), q // 2 + 1)
             x, y = rng.randrange(0, q), rng.randrange(0, q)
             if it % 50 == 0:
                 x, y = q - 1, q - 1
-            # forward butterfly
-            a = f_reduce(float(x), qd, qinv)
-            r = f_mulmod(float(y), float(w), wq, qd)
-            for v, ref in ((a + r, x + y * w), (a - r, x - y * w)):
-                assert v == int(v) and (int(v) - ref) % q == 0 and abs(v) <= 1.125 * q + 1
-            # inverse butterfly
-            s0 = f_reduce(float(x) + float(y), qd, qinv)
-            s1 = f_mulmod(float(x) - float(y), float(w), wq, qd)
-            assert (int(s0) - (x + y)) % q == 0 and abs(s0) <= q / 2 + 1
-            assert (int(s1) - (x - y) * w) % q == 0 and abs(s1) <= q * (0.5 + q * 2.0 ** -53) + 1
-
-
-def ksk_mul_f64(a, b, q, qinv):
-    x, y = float(a), float(b)
-    p = x * y
-    e = fma(x, y, -p)
-    k = fma(p, qinv, RND) - RND
-    return fma(-k, q, p) + e
-
-
-def ksk_canon_f64(s, q, qinv):
-    k = fma(s, qinv, RND) - RND
-    r = fma(-k, q, s)
-    if r < 0:
-        r = r + q
-    bits = Fraction(r + TWO52) - Fraction(TWO52)  # the low 52 bits of r + 2^52
-    return int(bits)
-
-
-def test_ksk_fp64_products_and_reduction():
-    rng = random.Random(13)
-    for q in primes50():
-        qd, qinv = float(q), 1.0 / q
-        for it in range(200):
-            terms = []
-            s = 0.0
-            for _ in range(6):  # four digits and two tensor terms at most
-                a = rng.randrange(q) if it % 7 else q - 1
-                b = rng.randrange(q) if it % 5 else q - 1
-                r = ksk_mul_f64(a, b, qd, qinv)
-                assert r == int(r) and abs(r) <= q and (int(r) - a * b) % q == 0
-                terms.append(a * b)
-                s = s + r
-            assert s == int(s)
-            assert ksk_canon_f64(s, qd, qinv) == sum(terms) % q
+            a, r = f_reduce(float(x), qd, qinv), f_mulmod(float(y), float(w), qd, qinv)
+            exact(a + r, x + y * w, q, 1.125 * q)
+            exact(a - r, x - y * w, q, 1.125 * q)
+            exact(f_mulmod(float(x) - float(y), float(w), qd, qinv), (x - y) * w, q, 0.625 * q)
 
 
 def tc_fold(d, q, qinv):
