@@ -834,7 +834,7 @@ void launch_conv(Context* c, const ConvJob* jobs, int n, cudaStream_t s) {
       FIDES_CUDA(cudaFuncSetAttribute(conv_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024)); \
       attr = true;                                                                                            \
     }                                                                                                         \
-    launch_pdl(conv_kernel<K>, grid, EW_THREADS, smem, s, L, c->d_prime, c->logN);                                    \
+    launch_pdl(conv_kernel<K>, grid, EW_THREADS, smem, s, L, c->d_prime, c->logN);                            \
     break;                                                                                                    \
   }
         FIDES_CONV_CASE(1) FIDES_CONV_CASE(2) FIDES_CONV_CASE(3) FIDES_CONV_CASE(4) FIDES_CONV_CASE(5)
@@ -851,7 +851,7 @@ void launch_conv(Context* c, const ConvJob* jobs, int n, cudaStream_t s) {
           launch_pdl(conv_kernel<0>, grid, EW_THREADS, smem, s, L, c->d_prime, c->logN);
         }
       }
-        }
+    }
   }
 }
 
@@ -979,12 +979,12 @@ void launch_ksk(Context* c, const KskJob* jobs, int n, cudaStream_t s) {
     }
     auto go = [&](auto kern) { go_list(kern, L); };
     switch (maxb * 16 + jg + (share_digits ? 128 : 0)) {
-#define FIDES_KSK_CASE(B, G)                    \
-  case B * 16 + G:                              \
-    go(ksk_kernel<B, G, 2, MAX_KSK_JOBS>);                    \
-    break;                                      \
-  case 128 + B * 16 + G:                        \
-    go(ksk_kernel<B, G, 2, MAX_KSK_JOBS, true>);              \
+#define FIDES_KSK_CASE(B, G)                     \
+  case B * 16 + G:                               \
+    go(ksk_kernel<B, G, 2, MAX_KSK_JOBS>);       \
+    break;                                       \
+  case 128 + B * 16 + G:                         \
+    go(ksk_kernel<B, G, 2, MAX_KSK_JOBS, true>); \
     break;
       FIDES_KSK_CASE(1, 1) FIDES_KSK_CASE(1, 2) FIDES_KSK_CASE(1, 4)
       FIDES_KSK_CASE(2, 1) FIDES_KSK_CASE(2, 2) FIDES_KSK_CASE(2, 4)
@@ -994,7 +994,7 @@ void launch_ksk(Context* c, const KskJob* jobs, int n, cudaStream_t s) {
       default:
         go(ksk_kernel<0, 1, 2, MAX_KSK_JOBS>);
     }
-    }
+  }
 }
 
 void launch_moddown_finish(Context* c, const FinJob* jobs, int n, cudaStream_t s) {
@@ -1009,7 +1009,7 @@ void launch_moddown_finish(Context* c, const FinJob* jobs, int n, cudaStream_t s
     for (int i = 0; i < m; ++i) bytes += 8.0 * c->N * ((L.j[i].add ? 4.0 : 3.0) * L.j[i].l);
     LaunchScope ls(c, s, KK_ELEM, bytes);
     launch_pdl(moddown_finish_kernel, grid, EW_THREADS, 0, s, L, c->d_prime, c->d_pinv, c->logN);
-    }
+  }
 }
 
 void launch_tensor(Context* c, const TensorJob* jobs, int n, cudaStream_t s) {
@@ -1024,7 +1024,7 @@ void launch_tensor(Context* c, const TensorJob* jobs, int n, cudaStream_t s) {
     for (int i = 0; i < m; ++i) bytes += 8.0 * c->N * ((L.j[i].d2 ? 7.0 : 6.0) * L.j[i].l);
     LaunchScope ls(c, s, KK_ELEM, bytes);
     launch_pdl(tensor_kernel, grid, EW_THREADS, 0, s, L, c->d_prime, c->logN);
-    }
+  }
 }
 
 void launch_switch_modulus(Context* c, const SwitchJob* jobs, int n, cudaStream_t s) {
@@ -1039,7 +1039,7 @@ void launch_switch_modulus(Context* c, const SwitchJob* jobs, int n, cudaStream_
     for (int i = 0; i < m; ++i) bytes += 8.0 * c->N * (1.0 + (L.j[i].l - 1));
     LaunchScope ls(c, s, KK_ELEM, bytes);
     launch_pdl(switch_kernel, grid, EW_THREADS, 0, s, L, c->d_prime, c->logN);
-    }
+  }
 }
 
 void launch_rescale_finish(Context* c, const RescaleJob* jobs, int n, cudaStream_t s) {
@@ -1054,7 +1054,7 @@ void launch_rescale_finish(Context* c, const RescaleJob* jobs, int n, cudaStream
     for (int i = 0; i < m; ++i) bytes += 8.0 * c->N * (3.0 * (L.j[i].l - 1));
     LaunchScope ls(c, s, KK_ELEM, bytes);
     launch_pdl(rescale_finish_kernel, grid, EW_THREADS, 0, s, L, c->d_prime, c->d_rescale, c->logN, c->n_q);
-    }
+  }
 }
 
 void launch_addsub(Context* c, const AddSubJob* jobs, int n, cudaStream_t s) {
@@ -1071,7 +1071,7 @@ void launch_addsub(Context* c, const AddSubJob* jobs, int n, cudaStream_t s) {
     dim3 grid(c->N / (2 * EW_THREADS), mx, m);
     LaunchScope ls(c, s, KK_ELEM, bytes);
     launch_pdl(addsub_kernel, grid, EW_THREADS, 0, s, L, c->d_prime, c->logN);
-    }
+  }
 }
 
 void launch_scalar(Context* c, const ScalarJob* jobs, int n, cudaStream_t s) {
@@ -1089,7 +1089,7 @@ void launch_scalar(Context* c, const ScalarJob* jobs, int n, cudaStream_t s) {
     dim3 grid(c->N / (2 * EW_THREADS), mx, m);
     LaunchScope ls(c, s, KK_ELEM, bytes);
     launch_pdl(scalar_kernel, grid, EW_THREADS, 0, s, L, c->d_prime, c->logN);
-    }
+  }
 }
 
 }  // namespace fides

@@ -8,9 +8,9 @@
 //   * N = 2^LOG1 x 2^LOG2.  Pass COL runs global stages [0, LOG1) on strided columns,
 //     pass ROW runs stages [LOG1, logN) on contiguous rows.  Forward = COL then ROW,
 //     inverse = ROW then COL; each pass reads and writes every limb once.
-//   * each thread keeps 2^LE elements in registers (16, or 8 at N >= 2^15 where the
-//     autotuner picks it) and runs LE stages per chunk; chunks exchange through padded
-//     shared memory;
+//   * each thread keeps 2^LE elements in registers (16, or 8: where the autotuner picks it at
+//     N >= 2^15, for small launches at N = 2^12 to 2^14, and for rescales above 2^50, below) and
+//     runs LE stages per chunk; chunks exchange through padded shared memory;
 //   * primes below 2^50 run FP64 butterflies (exact integers in doubles, ntt_impl.cuh), larger ones lazy
 //     butterflies with one 64-bit Shoup product each (primes < 2^62): below 2^61 the forward transform
 //     lets values grow by 4q a stage and subtracts once a chunk, at every second or at every stage, by

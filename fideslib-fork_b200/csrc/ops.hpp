@@ -91,7 +91,8 @@ void op_moddown_batch(Context* c, uint64_t* const* exts, const int* ls, uint64_t
 void op_accumulate(Context* c, const uint64_t* c0, const uint64_t* c1, int l, int radix, int stride, int size,
                    const std::vector<std::pair<int, const uint64_t*>>& keys, uint64_t* out0, uint64_t* out1,
                    cudaStream_t s);
-// ModDown followed by the rescale by q_(l_i - 1), fused (outs[i]: l_i - 1 limbs).
+// ModDown followed by the rescale by q_(l_i - 1), fused (outs[i]: l_i - 1 limbs).  The special limbs of
+// exts[i] and its limb l_i - 1, the one that goes, are transformed in place.
 void op_moddown_rescale_batch(Context* c, uint64_t* const* exts, const int* ls, uint64_t* const* outs, int n,
                               cudaStream_t s);
 // Hoisted rotations from ModUp digits computed earlier (op_modup of c1, own-digit limbs included):

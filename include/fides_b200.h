@@ -6,6 +6,7 @@
  * key pointer is DEVICE memory on the context's GPU.  Data are in EVALUATION format
  * (negacyclic NTT, bit-reversed order) unless stated otherwise -- the same layout as the
  * reference's RawCipherText limbs (src/CKKS/openfhe-interface/RawCiphertext.cuh:21-37).
+ * Every word of a limb is a residue, at least 0 and below the limb's prime, in operands and results.
  *
  * "level" l = number of active Q limbs of a ciphertext (1 <= l <= n_q).  An extended
  * polynomial at level l has l Q limbs followed by the K special limbs.
