@@ -978,7 +978,8 @@ void launch_ksk(Context* c, const KskJob* jobs, int n, cudaStream_t s) {
       continue;
     }
     auto go = [&](auto kern) { go_list(kern, L); };
-    switch (maxb * 16 + jg + (share_digits ? 128 : 0)) {
+    // more than four digits: the general kernel (9 to 12 of them would name a shared-digit form of 1 to 4)
+    switch (maxb > 4 ? 0 : maxb * 16 + jg + (share_digits ? 128 : 0)) {
 #define FIDES_KSK_CASE(B, G)                     \
   case B * 16 + G:                               \
     go(ksk_kernel<B, G, 2, MAX_KSK_JOBS>);       \
