@@ -35,9 +35,9 @@ void launch_pdl(void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, 
   cfg.attrs = &at;
   cfg.numAttrs = 1;
   void* p[] = {const_cast<void*>(static_cast<const void*>(&args))...};
-  const cudaError_t e = cudaLaunchKernelExC(&cfg, reinterpret_cast<const void*>(kernel), p);
-  if (e != cudaSuccess) cudaGetLastError();  // reported here, not by the thread's next check as well
-  FIDES_CUDA(e);
+  const cudaError_t kernel_launch = cudaLaunchKernelExC(&cfg, reinterpret_cast<const void*>(kernel), p);
+  if (kernel_launch != cudaSuccess) cudaGetLastError();  // reported here, not by the thread's next check as well
+  FIDES_CUDA(kernel_launch);
 }
 
 }  // namespace fides
